@@ -437,18 +437,85 @@ __global__ void batch_labels(const T *__restrict__ H, int p, const int *__restri
     lab[(size_t)j * nsel + s] = (unsigned char)best;
 }
 
-// consensus[j1][j2] = (1 / nsel) * #{s : label_s(j1) == label_s(j2)};
-// labels are stored column-major over solves (lab[j * nsel + s]).
-__global__ void batch_consensus(const unsigned char *__restrict__ lab, int p, int nsel,
-                                float *__restrict__ out) {
-    const int j1 = blockIdx.y * 16 + (threadIdx.x >> 4);
-    const int j2 = blockIdx.x * 16 + (threadIdx.x & 15);
-    if (j1 >= p || j2 >= p) return;
-    const unsigned char *a = lab + (size_t)j1 * nsel;
-    const unsigned char *b = lab + (size_t)j2 * nsel;
-    int same = 0;
-    for (int s = 0; s < nsel; s++) same += (a[s] == b[s]);
-    out[(size_t)j1 * p + j2] = (float)same / (float)nsel;
+// Bit planes of the labels: bit s of planes[(w * NB + b) * p + j] is bit b of
+// column j's label in solve 32 w + s (0 past nsel).  One warp a (column, word).
+template <int NB>
+__global__ void __launch_bounds__(256)
+    label_planes(const unsigned char *__restrict__ lab, int p, int nsel, int words,
+                 unsigned *__restrict__ planes) {
+    const int64_t t = ((int64_t)blockIdx.x * 256 + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (t >= (int64_t)p * words) return;
+    const int w = (int)(t / p), j = (int)(t - (int64_t)w * p);
+    const int s = 32 * w + lane;
+    const unsigned l = s < nsel ? lab[(size_t)j * nsel + s] : 0u;
+#pragma unroll
+    for (int b = 0; b < NB; b++) {
+        const unsigned bits = __ballot_sync(0xffffffffu, (l >> b) & 1u);
+        if (lane == b) planes[((size_t)w * NB + b) * p + j] = bits;
+    }
+}
+
+// consensus[j1][j2] = (1 / nsel) * #{s : label_s(j1) == label_s(j2)}: 32
+// solves at a time, the labels differ where any plane's bits differ.  Block
+// tile 64 x 64, a thread 8 rows x 2 columns.  NB covers the largest selected
+// rank - 1.  Bound: the p x p f32 store and the popcounts (16 a clock and SM)
+// of 25 M pairs x 2 words at p = 5000 and 64 solves; comparing the labels
+// byte by byte took 1576 us there, this 51-76 us (1 to 4 planes).
+template <int NB>
+__global__ void __launch_bounds__(256)
+    consensus_planes(const unsigned *__restrict__ planes, int p, int nsel, int words,
+                     float *__restrict__ out) {
+    __shared__ unsigned sa[NB][64], sb[NB][64];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int r0 = blockIdx.y * 64, c0 = blockIdx.x * 64;
+    int diff[8][2] = {};
+    for (int w = 0; w < words; w++) {
+        __syncthreads();
+        for (int e = threadIdx.x; e < 2 * NB * 64; e += 256) {
+            const int b = (e >> 6) % NB, q = e & 63;
+            const bool rows = e < NB * 64;
+            const int j = (rows ? r0 : c0) + q;
+            const unsigned v = j < p ? planes[((size_t)w * NB + b) * p + j] : 0u;
+            if (rows) sa[b][q] = v; else sb[b][q] = v;
+        }
+        __syncthreads();
+        unsigned cb[2][NB];
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+#pragma unroll
+            for (int b = 0; b < NB; b++) cb[h][b] = sb[b][tx + 32 * h];
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            unsigned x0 = 0u, x1 = 0u;
+#pragma unroll
+            for (int b = 0; b < NB; b++) {
+                const unsigned r = sa[b][ty + 8 * q];
+                x0 |= r ^ cb[0][b];
+                x1 |= r ^ cb[1][b];
+            }
+            diff[q][0] += __popc(x0);
+            diff[q][1] += __popc(x1);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int j1 = r0 + ty + 8 * q, j2 = c0 + tx + 32 * h;
+            if (j1 < p && j2 < p)
+                out[(size_t)j1 * p + j2] = (float)(nsel - diff[q][h]) / (float)nsel;
+        }
+}
+
+template <int NB>
+void launch_consensus(const unsigned char *lab, int p, int nsel, unsigned *planes, float *out,
+                      cudaStream_t s) {
+    const int words = (nsel + 31) / 32;
+    const int64_t warps = (int64_t)p * words;
+    label_planes<NB><<<(unsigned)((warps + 7) / 8), 256, 0, s>>>(lab, p, nsel, words, planes);
+    const unsigned g = (unsigned)((p + 63) / 64);
+    consensus_planes<NB><<<dim3(g, g), 256, 0, s>>>(planes, p, nsel, words, out);
 }
 
 // ---------------------------------------------------------------------------
@@ -1003,19 +1070,32 @@ nmfcu_status nmfcu_consensus_device(nmfcu_context *ctx, int64_t p, int32_t nsolv
     std::lock_guard<std::mutex> lk(nmfcu_internal::context_mutex(ctx));
     nmfcu_internal::DeviceScope dg(nmfcu_internal::context_device(ctx));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    void *pso = nullptr, *psr = nullptr, *plab = nullptr;
+    void *pso = nullptr, *psr = nullptr, *plab = nullptr, *ppl = nullptr;
     NMFCU_TRY(nmfcu_internal::context_buffer(ctx, 9, sizeof(int) * nsel, &pso));
     NMFCU_TRY(nmfcu_internal::context_buffer(ctx, 10, sizeof(int) * nsel, &psr));
     NMFCU_TRY(nmfcu_internal::context_buffer(ctx, 11, (size_t)p * nsel, &plab));
+    int bits = 1;  // of the largest selected label
+    for (int i = 0; i < nsel; i++)
+        while ((sr[i] - 1) >> bits) bits++;
+    const int nb = bits <= 4 ? bits : 8;
+    NMFCU_TRY(nmfcu_internal::context_buffer(
+        ctx, 12, sizeof(unsigned) * nb * (size_t)p * ((nsel + 31) / 32), &ppl));
     NMFCU_CUDA_TRY(cudaMemcpyAsync(pso, so.data(), sizeof(int) * nsel, cudaMemcpyHostToDevice, s));
     NMFCU_CUDA_TRY(cudaMemcpyAsync(psr, sr.data(), sizeof(int) * nsel, cudaMemcpyHostToDevice, s));
     const dim3 lg((unsigned)((p + 255) / 256), (unsigned)nsel);
     batch_labels<double><<<lg, 256, 0, s>>>(dH, (int)p, (const int *)pso, (const int *)psr, nsel,
                                             (unsigned char *)plab);
-    const dim3 cg((unsigned)((p + 15) / 16), (unsigned)((p + 15) / 16));
-    batch_consensus<<<cg, 256, 0, s>>>((const unsigned char *)plab, (int)p, nsel, d_out);
+    const auto planes = (unsigned *)ppl;
+    const auto lab = (const unsigned char *)plab;
+    switch (nb) {
+        case 1: launch_consensus<1>(lab, (int)p, nsel, planes, d_out, s); break;
+        case 2: launch_consensus<2>(lab, (int)p, nsel, planes, d_out, s); break;
+        case 3: launch_consensus<3>(lab, (int)p, nsel, planes, d_out, s); break;
+        case 4: launch_consensus<4>(lab, (int)p, nsel, planes, d_out, s); break;
+        default: launch_consensus<8>(lab, (int)p, nsel, planes, d_out, s); break;
+    }
     NMFCU_CUDA_TRY(cudaGetLastError());
-    nmfcu_internal::count_launches(ctx, 2);
+    nmfcu_internal::count_launches(ctx, 3);
     NMFCU_CUDA_TRY(cudaStreamSynchronize(s));
     return NMFCU_OK;
 }
