@@ -43,7 +43,9 @@ struct RunState {
     int stopped;       // 1 once the loop has stopped
     int error;         // 1: `iter % check_interval` with check_interval == 0
     int timeout;       // a bounded mbarrier wait gave up (stream.cuh codes)
-    unsigned gram_ticket;  // blocks of the running Gram launch that are done
+    // Tickets of the running epilogue or Gram launch: [0] the blocks (or
+    // groups of blocks) whose Gram partials are out, [1 + g] group g's blocks.
+    unsigned gram_ticket[1 + 32];
 };
 
 // Fixed constants of the streaming kernels.
@@ -638,12 +640,13 @@ __device__ __forceinline__ bool w_update_by_column(int method) {
            method == M_NSNMF || method == M_LSNMF || method == M_PRODUCT;
 }
 // Column j (< e.r) of w_update for those methods, with the same operations
-// in the same order (so the same bits).  numj = num[j], wrj = wr[j].
+// in the same order (so the same bits).  numj = num[j]; wr: the row's old
+// values.
 template <int RP>
-__device__ __forceinline__ double w_update_column(const EpiParams &e, double numj, double wrj,
-                                                  const double (&wr)[RP], int j,
-                                                  double ro = 0.0,
-                                                  const double *ax = nullptr) {
+__device__ __forceinline__ double w_update_column(const EpiParams &e, double numj,
+                                                  const double *wr, int j, double ro,
+                                                  const double *ax) {
+    const double wrj = wr[j];
     if (e.method == M_LSNMF) {
         const double temp = mul(wrj, ax[j]);
         return (temp > e.eps ? temp : e.eps) / add(numj, e.eps);
@@ -660,179 +663,367 @@ __device__ __forceinline__ double w_update_column(const EpiParams &e, double num
     }
     return mul(wrj, numj) / e.sums[j];  // M_BRUNET, M_NSNMF
 }
-
-// H epilogue: one thread per column; sums the S split partials in order.
-template <int RP>
-__global__ void __launch_bounds__(kThreads)
-    h_epilogue(double *__restrict__ H, int p, const double *__restrict__ part, int S,
-               EpiParams e, const RunState *st) {
-    if (run_stopped(st)) return;
-    const int j = blockIdx.x * kThreads + threadIdx.x;
-    if (j >= p) return;
-    double num[RP], hc[RP];
-#pragma unroll
-    for (int k = 0; k < RP; k++) {
-        double s = 0.0;
-        for (int sp = 0; sp < S; sp++) s += part[((int64_t)sp * RP + k) * p + j];
-        num[k] = s;
-        hc[k] = H[(int64_t)k * p + j];
+// Row i (< e.r) of h_update for the same methods.  hc(l): the column's old
+// values; ax: lsNMF's numerator of this row and column.
+template <int RP, typename Col>
+__device__ __forceinline__ double h_update_row(const EpiParams &e, double numi, Col &&hc, int i,
+                                               double ax) {
+    if (e.method == M_LSNMF) {
+        const double temp = mul(hc(i), ax);
+        return (temp > e.eps ? temp : e.eps) / add(numi, e.eps);
     }
-    h_update<RP>(e, num, hc);
+    if (e.method == M_PRODUCT) return numi;
+    if (e.method == M_LEE || e.method == M_OFFSET) {
+        double den = 0.0;
 #pragma unroll
-    for (int k = 0; k < RP; k++)
-        if (k < e.r) H[(int64_t)k * p + j] = hc[k];
-}
-
-// W epilogue: one thread per row.
-template <int RP>
-__global__ void __launch_bounds__(kThreads)
-    w_epilogue(double *__restrict__ W, int n, const double *__restrict__ part, int S,
-               EpiParams e, const RunState *st) {
-    if (run_stopped(st)) return;
-    const int i = blockIdx.x * kThreads + threadIdx.x;
-    if (i >= n) return;
-    double num[RP], wr[RP];
-#pragma unroll
-    for (int k = 0; k < RP; k++) {
-        double s = 0.0;
-        for (int sp = 0; sp < S; sp++) s += part[((int64_t)sp * n + i) * RP + k];
-        num[k] = s;
-        wr[k] = W[(int64_t)i * RP + k];
+        for (int l = RP - 1; l >= 0; l--)
+            if (l < e.r) den = add(den, mul(e.G[i * RP + l], hc(l)));
+        if (e.addon) den = add(den, e.addon[i]);
+        const double temp = mul(hc(i), numi);
+        return (temp > e.eps ? temp : e.eps) / add(den, e.eps);
     }
-    w_update<RP>(e, num, wr, e.roff ? e.roff[i] : 0.0);
-#pragma unroll
-    for (int k = 0; k < RP; k++)
-        if (k < e.r) W[(int64_t)i * RP + k] = wr[k];
+    return mul(hc(i), numi) / e.sums[i];  // M_BRUNET, M_NSNMF
 }
 
 // ---------------------------------------------------------------------------
-// Gram matrices and sums (two-stage, fixed order).
+// Gram matrices and sums.
 // ---------------------------------------------------------------------------
+// X^T X and the column sums of X (W, or H^T).  A launch runs in one of two
+// ways (GramPlan):
+//   few tiles   a block a tile of kTileRows rows of W / kTileCols columns of
+//               H, its warps sharing the tile;
+//   many tiles  a warp a tile of 32 rows / columns, a block's warps each
+//               every (warps of the launch)-th tile.
+// A warp adds four rows (columns) of its tile at a time on the FP64 tensor
+// cores (mma.sync.m8n8k4: a fragment of X is both operands), a block adds its
+// warps in a fixed tree, publishes its entries and takes a ticket; the last
+// block of each group of 16 sums the group's partials, the last group the
+// groups'.  No block waits on another.  The update epilogues (stream.cuh)
+// form the same sums over the same tiles from the values they have just
+// written, so a Gram has the same bits wherever it is formed.
+//
+// For brunet, which needs the sums alone, only those are formed.
+//
+// (One thread an entry walking all rows of a block, and the last block alone
+// summing 148 partials, took 31 us for H at 20 x 40000 and 9.1 us at 8 x 3000.)
+constexpr int kEpiThreads = 512;   // threads of a block, few tiles
+constexpr int kWideThreads = 256;  // threads of a block, many tiles
+constexpr int kTileCols = 32;      // columns of H a tile
+constexpr int kTileRows = 16;      // rows of W a tile (few tiles)
+constexpr int kGramGroup = 16;     // blocks of a group
+enum : int { GRAM_NONE = 0, GRAM_SUMS = 1, GRAM_FULL = 2 };
 
-// The second stage inside the first stage's launch: each block publishes
-// its partials and takes a ticket; the block that takes the last ticket sums
-// the B = gridDim.x partials in block order (the sums gram_finalize forms,
-// bit for bit) and resets the ticket for the next launch.  No block waits
-// on another.  G == nullptr leaves the partials for the caller (lee's and
-// nsNMF's col_rescale read them).
-template <int RP>
-__device__ __forceinline__ void gram_finish_last(const double *pg, const double *ps, double *G,
-                                                 double *sums, unsigned *ticket) {
-    if (G == nullptr) return;
-    __shared__ bool last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = (atomicAdd(ticket, 1u) == gridDim.x - 1);
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    const int tid = threadIdx.x;
-    const int B = (int)gridDim.x;
-    double g = 0.0;
-    for (int b = 0; b < B; b++) g += __ldcg(&pg[(int64_t)b * RP * RP + tid]);
-    G[tid] = g;
-    if (tid < RP) {
-        double t = 0.0;
-        for (int b = 0; b < B; b++) t += __ldcg(&ps[(int64_t)b * RP + tid]);
-        sums[tid] = t;
+// How an epilogue or Gram launch over `len` rows of W / columns of H runs: a
+// block a tile up to two blocks a multiprocessor, beyond that a warp a tile.
+// At 296 tiles the first still fits the chip at once; the second has every
+// warp at work, which the sequential HALS sweeps need.
+struct GramPlan {
+    bool few;
+    int blocks;
+};
+inline GramPlan gram_plan(int64_t len, int tile, int sms) {
+    GramPlan g;
+    const int64_t tiles = (len + tile - 1) / tile, cap = 2 * (int64_t)sms;
+    g.few = tiles <= cap;
+    if (g.few) {
+        g.blocks = (int)(tiles < 1 ? 1 : tiles);
+    } else {
+        const int64_t b = (len + kWideThreads - 1) / kWideThreads;
+        g.blocks = (int)(b < cap ? b : cap);
     }
-    if (tid == 0) *ticket = 0u;
+    // the tickets count at most 32 groups
+    const int most = 32 * kGramGroup;
+    if (g.blocks > most) {
+        g.few = false;
+        g.blocks = most;
+    }
+    return g;
 }
 
-// W^T W and colsum(W) partials over a row range, and with G given the
-// finished Gram and sums (gram_finish_last).  block RP*RP threads.
+struct GramOut {
+    int want = GRAM_NONE;
+    // lee, whose W columns are divided by their sums right after: write the
+    // Gram of the divided columns (sums stay those of W itself).
+    int rescaled = 0;
+    double *part = nullptr;  // (blocks + 32) x gram_entries(RP)
+    double *G = nullptr;     // RP x RP
+    double *sums = nullptr;  // RP
+    unsigned *ticket = nullptr;  // RunState::gram_ticket
+};
+
+__host__ __device__ constexpr int gram_entries(int RP) { return RP * (RP + 1) / 2 + RP; }
+
+// Entry e of the list [column sums | pairs k <= l]: k, and l (-1: a sum).
 template <int RP>
-__global__ void gram_w_partial(const double *__restrict__ W, int n, int rows_per_block,
-                               double *__restrict__ pg, double *__restrict__ ps,
-                               const RunState *st, double *G = nullptr, double *sums = nullptr,
-                               unsigned *ticket = nullptr) {
-    if (run_stopped(st)) return;
-    constexpr int CH = 64;
-    __shared__ double sW[CH][RP];
-    const int tid = threadIdx.x;
-    const int k = tid / RP, l = tid % RP;
-    const int u0 = blockIdx.x * rows_per_block;
-    const int u1 = min(n, u0 + rows_per_block);
-    double g = 0.0, s = 0.0;
-    for (int base = u0; base < u1; base += CH) {
-        const int rows = min(CH, u1 - base);
-        __syncthreads();
-        for (int t = tid; t < CH * RP; t += RP * RP)
-            (&sW[0][0])[t] = (t < rows * RP) ? W[(int64_t)base * RP + t] : 0.0;
-        __syncthreads();
-        for (int u = 0; u < rows; u++) {
-            g = fma(sW[u][k], sW[u][l], g);
-            if (tid < RP) s += sW[u][tid];
+__device__ __forceinline__ void gram_entry(int e, int &k, int &l) {
+    if (e < RP) {
+        k = e;
+        l = -1;
+        return;
+    }
+    e -= RP;
+    k = 0;
+    while (e >= RP - k) {
+        e -= RP - k;
+        k++;
+    }
+    l = k + e;
+}
+
+// mma.sync.m8n8k4 with f64 operands: D (8 x 8) += A (8 x 4) B (4 x 8), one
+// A and one B element and two D elements a thread (A[g][q], B[q][g],
+// D[g][2q + e] with g = lane / 4, q = lane % 4).  The asm has no side effects
+// beyond its operands (not volatile), so independent MMAs may be scheduled
+// across one another; each accumulator's chain keeps its order.
+__device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+        : "+d"(d[0]), "+d"(d[1])
+        : "d"(a), "d"(b));
+}
+
+template <int RP, int THREADS>
+struct GramAcc {
+    static constexpr int E = gram_entries(RP);
+    static constexpr int MT = (RP + 7) / 8;
+    static constexpr int NP = MT * (MT + 1) / 2;  // tiles mt <= nt
+    static constexpr int RAW = 2 * NP + MT;       // a lane's values
+    static constexpr int WARPS = THREADS / 32;
+    // Shared memory of finish(), in doubles.
+    static constexpr int SCRATCH_TREE = WARPS / 2 * RAW * 32;
+    static constexpr int SCRATCH = SCRATCH_TREE > 2 * THREADS + RP ? SCRATCH_TREE : 2 * THREADS + RP;
+    double d[NP][2], sm[MT];
+    __device__ __forceinline__ void init() {
+#pragma unroll
+        for (int i = 0; i < NP; i++) d[i][0] = d[i][1] = 0.0;
+#pragma unroll
+        for (int i = 0; i < MT; i++) sm[i] = 0.0;
+    }
+    // Adds four rows: at(k, q) is the value of row q (0..3) in column k < RP.
+    template <typename At>
+    __device__ __forceinline__ void add4(int want, At &&at) {
+        const int g = (threadIdx.x & 31) >> 2, q = threadIdx.x & 3;
+        double f[MT];
+#pragma unroll
+        for (int mt = 0; mt < MT; mt++) {
+            const int k = mt * 8 + g;
+            f[mt] = k < RP ? at(k, q) : 0.0;
+            sm[mt] += f[mt];
+        }
+        if (want != GRAM_FULL) return;
+        int i = 0;
+#pragma unroll
+        for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+            for (int nt = mt; nt < MT; nt++) dmma_8x8x4(d[i++], f[mt], f[nt]);
+    }
+    // Where entry (k, l) is in the warps' sum `raw`.
+    __device__ __forceinline__ static int raw_index(int k, int l) {
+        const int mt = k >> 3, g = k & 7;
+        if (l < 0) return (2 * NP + mt) * 32 + g * 4;
+        const int nt = l >> 3, c = l & 7;
+        const int pair = mt * MT - mt * (mt - 1) / 2 + (nt - mt);
+        return (2 * pair + (c & 1)) * 32 + g * 4 + (c >> 1);
+    }
+    // Sum of `count` partials of entry e (stride E from src) by the whole
+    // block: `split` threads an entry, each every split-th.  Valid in threads
+    // tid < cnt where split > 1, else in thread e - base.
+    __device__ __forceinline__ static double sum_parts(const double *src, int count, int e,
+                                                       bool on, int first, int step) {
+        double a = 0.0;
+        if (on)
+#pragma unroll 8
+            for (int b = first; b < count; b += step) a += __ldcg(src + (size_t)b * E + e);
+        return a;
+    }
+    // `count` partials at src into dst (E entries each), or, with the last
+    // group done, the finished Gram and sums.
+    __device__ __forceinline__ static void reduce(const double *src, int count, int limit,
+                                                  double *dst, const GramOut &g, double *scratch) {
+        const int tid = threadIdx.x;
+        double *red = scratch, *val = scratch + THREADS;  // val: THREADS + RP
+        const int split = limit < THREADS ? min(THREADS / limit, 16) : 1;
+        for (int base = 0; base < limit; base += THREADS) {
+            const int q = split > 1 ? tid / limit : 0;
+            const int e = split > 1 ? tid - q * limit : base + tid;
+            double a = sum_parts(src, count, e, e < limit && q < split, q, split);
+            if (split > 1) {
+                red[tid] = a;
+                __syncthreads();
+                if (tid < limit)
+                    for (int s = 1; s < split; s++) a += red[s * limit + tid];
+            }
+            const bool mine = split > 1 ? tid < limit : e < limit;
+            if (dst != nullptr) {
+                if (mine) dst[e] = a;
+                continue;
+            }
+            // The sums are the first entries, so the first round has them all.
+            if (base == 0) {
+                if (mine && e < RP) {
+                    val[e] = a;
+                    g.sums[e] = a;
+                }
+                __syncthreads();
+            }
+            if (!mine || e < RP) continue;
+            int k, l;
+            gram_entry<RP>(e, k, l);
+            if (g.rescaled) {
+                if (val[k] > 0.0) a /= val[k];
+                if (val[l] > 0.0) a /= val[l];
+            }
+            g.G[k * RP + l] = a;
+            g.G[l * RP + k] = a;
         }
     }
-    pg[(int64_t)blockIdx.x * RP * RP + tid] = g;
-    if (tid < RP) ps[(int64_t)blockIdx.x * RP + tid] = s;
-    gram_finish_last<RP>(pg, ps, G, sums, ticket);
-}
-
-// H H^T and rowsum(H) partials over a column range, and with G given the
-// finished Gram and sums.  block RP*RP threads.
-template <int RP>
-__global__ void gram_h_partial(const double *__restrict__ H, int p, int cols_per_block,
-                               double *__restrict__ pg, double *__restrict__ ps,
-                               const RunState *st, double *G = nullptr, double *sums = nullptr,
-                               unsigned *ticket = nullptr) {
-    if (run_stopped(st)) return;
-    constexpr int CC = 64;
-    __shared__ double sH[RP][CC + 1];
-    const int tid = threadIdx.x;
-    const int k = tid / RP, l = tid % RP;
-    const int c0 = blockIdx.x * cols_per_block;
-    const int c1 = min(p, c0 + cols_per_block);
-    double g = 0.0, s = 0.0;
-    for (int base = c0; base < c1; base += CC) {
-        const int cols = min(CC, c1 - base);
-        __syncthreads();
-        for (int t = tid; t < RP * CC; t += RP * RP) {
-            const int kk = t / CC, cc = t % CC;
-            sH[kk][cc] = (cc < cols) ? H[(int64_t)kk * p + base + cc] : 0.0;
+    // Adds up the block's warps, publishes, and finishes where this block is
+    // the last.  scratch: SCRATCH doubles of shared memory, free to overwrite
+    // once every thread of the block has called this.
+    __device__ __forceinline__ void finish(const GramOut &g, double *scratch) {
+        if (g.want == GRAM_NONE) return;
+        const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+        const int limit = g.want == GRAM_FULL ? E : RP;
+#pragma unroll
+        for (int mt = 0; mt < MT; mt++) {  // over the four rows of a step
+            sm[mt] += __shfl_xor_sync(0xffffffffu, sm[mt], 1);
+            sm[mt] += __shfl_xor_sync(0xffffffffu, sm[mt], 2);
+        }
+        for (int half = WARPS / 2; half >= 1; half >>= 1) {
+            __syncthreads();
+            if (warp >= half && warp < 2 * half) {
+                double *w = scratch + (size_t)(warp - half) * RAW * 32 + lane;
+#pragma unroll
+                for (int i = 0; i < NP; i++) {
+                    w[(2 * i) * 32] = d[i][0];
+                    w[(2 * i + 1) * 32] = d[i][1];
+                }
+#pragma unroll
+                for (int i = 0; i < MT; i++) w[(2 * NP + i) * 32] = sm[i];
+            }
+            __syncthreads();
+            if (warp < half) {
+                const double *w = scratch + (size_t)warp * RAW * 32 + lane;
+#pragma unroll
+                for (int i = 0; i < NP; i++) {
+                    d[i][0] += w[(2 * i) * 32];
+                    d[i][1] += w[(2 * i + 1) * 32];
+                }
+#pragma unroll
+                for (int i = 0; i < MT; i++) sm[i] += w[(2 * NP + i) * 32];
+            }
         }
         __syncthreads();
-        for (int c = 0; c < cols; c++) {
-            g = fma(sH[k][c], sH[l][c], g);
-            if (tid < RP) s += sH[tid][c];
+        if (warp == 0) {
+            double *w = scratch + lane;
+#pragma unroll
+            for (int i = 0; i < NP; i++) {
+                w[(2 * i) * 32] = d[i][0];
+                w[(2 * i + 1) * 32] = d[i][1];
+            }
+#pragma unroll
+            for (int i = 0; i < MT; i++) w[(2 * NP + i) * 32] = sm[i];
         }
+        __syncthreads();
+        const int B = (int)gridDim.x;
+        for (int e = tid; e < limit; e += THREADS) {
+            int k, l;
+            gram_entry<RP>(e, k, l);
+            g.part[(size_t)blockIdx.x * E + e] = scratch[raw_index(k, l)];
+        }
+        __shared__ bool last;
+        __threadfence();
+        __syncthreads();
+        const double *src = g.part;
+        int count = B;
+        if (B > 2 * kGramGroup) {
+            const int group = (int)blockIdx.x / kGramGroup;
+            const int groups = (B + kGramGroup - 1) / kGramGroup;
+            const int members = min(kGramGroup, B - group * kGramGroup);
+            if (tid == 0) last = (atomicAdd(g.ticket + 1 + group, 1u) == (unsigned)members - 1u);
+            __syncthreads();
+            if (!last) return;
+            __threadfence();
+            double *dst = g.part + (size_t)(B + group) * E;
+            reduce(g.part + (size_t)group * kGramGroup * E, members, limit, dst, g, scratch);
+            if (tid == 0) g.ticket[1 + group] = 0u;
+            __threadfence();
+            __syncthreads();
+            src = g.part + (size_t)B * E;
+            count = groups;
+        }
+        if (tid == 0) last = (atomicAdd(g.ticket, 1u) == (unsigned)count - 1u);
+        __syncthreads();
+        if (!last) return;
+        __threadfence();
+        reduce(src, count, limit, nullptr, g, scratch);
+        if (tid == 0) *g.ticket = 0u;
     }
-    pg[(int64_t)blockIdx.x * RP * RP + tid] = g;
-    if (tid < RP) ps[(int64_t)blockIdx.x * RP + tid] = s;
-    gram_finish_last<RP>(pg, ps, G, sums, ticket);
-}
+};
 
-// Sum B partial Grams / sums in block order.  block RP*RP threads.
-template <int RP>
-__global__ void gram_finalize(const double *__restrict__ pg, const double *__restrict__ ps,
-                              int B, double *__restrict__ G, double *__restrict__ sums,
-                              const RunState *st) {
+// W^T W and colsum(W) on their own (a W no epilogue has just written).
+template <int RP, int THREADS>
+__global__ void __launch_bounds__(THREADS)
+    gram_w_tiles(const double *__restrict__ W, int n, GramOut g, const RunState *st) {
     if (run_stopped(st)) return;
-    const int tid = threadIdx.x;
-    double g = 0.0;
-    for (int b = 0; b < B; b++) g += pg[(int64_t)b * RP * RP + tid];
-    G[tid] = g;
-    if (tid < RP) {
-        double s = 0.0;
-        for (int b = 0; b < B; b++) s += ps[(int64_t)b * RP + tid];
-        sums[tid] = s;
+    using GA = GramAcc<RP, THREADS>;
+    constexpr bool FEW = THREADS == kEpiThreads;
+    extern __shared__ double scratch[];
+    const int warp = threadIdx.x >> 5;
+    GA ga;
+    ga.init();
+    const auto steps = [&](int i0, int rows, int s0, int s1) {
+        for (int s = s0; s < s1; s++)
+            ga.add4(g.want, [&](int k, int q) {
+                const int u = 4 * s + q;
+                return u < rows ? W[(size_t)(i0 + u) * RP + k] : 0.0;
+            });
+    };
+    if (FEW) {
+        const int i0 = blockIdx.x * kTileRows;
+        if (warp < kTileRows / 4) steps(i0, min(kTileRows, n - i0), warp, warp + 1);
+    } else {
+        const int tiles = (n + 31) / 32;
+        for (int t = blockIdx.x * GA::WARPS + warp; t < tiles; t += gridDim.x * GA::WARPS)
+            steps(t * 32, min(32, n - t * 32), 0, 8);
     }
+    ga.finish(g, scratch);
 }
 
-// lee's col_rescale (lib.rs:1461-1470): every block re-sums the colsum
-// partials in the same order, then divides its rows.  W[:, k] /= s_k when
-// s_k > 0.
+// H H^T and rowsum(H) on their own.
+template <int RP, int THREADS>
+__global__ void __launch_bounds__(THREADS)
+    gram_h_tiles(const double *__restrict__ H, int p, GramOut g, const RunState *st) {
+    if (run_stopped(st)) return;
+    using GA = GramAcc<RP, THREADS>;
+    constexpr bool FEW = THREADS == kEpiThreads;
+    extern __shared__ double scratch[];
+    const int warp = threadIdx.x >> 5;
+    GA ga;
+    ga.init();
+    const auto steps = [&](int j0, int s0, int s1) {
+        for (int s = s0; s < s1; s++)
+            ga.add4(g.want, [&](int k, int q) {
+                const int j = j0 + 4 * s + q;
+                return j < p ? H[(size_t)k * p + j] : 0.0;
+            });
+    };
+    if (FEW) {
+        if (warp < kTileCols / 4) steps(blockIdx.x * kTileCols, warp, warp + 1);
+    } else {
+        const int tiles = (p + kTileCols - 1) / kTileCols;
+        for (int t = blockIdx.x * GA::WARPS + warp; t < tiles; t += gridDim.x * GA::WARPS)
+            steps(t * kTileCols, 0, kTileCols / 4);
+    }
+    ga.finish(g, scratch);
+}
+
+// lee's col_rescale (lib.rs:1461-1470): W[:, k] /= sums[k] when sums[k] > 0.
 template <int RP>
-__global__ void col_rescale(double *__restrict__ W, int n, int r, const double *__restrict__ ps,
-                            int B, const RunState *st) {
+__global__ void col_rescale(double *__restrict__ W, int n, int r, const double *__restrict__ sums,
+                            const RunState *st) {
     if (run_stopped(st)) return;
     __shared__ double s[RP];
-    if (threadIdx.x < RP) {
-        double a = 0.0;
-        for (int b = 0; b < B; b++) a += ps[(int64_t)b * RP + threadIdx.x];
-        s[threadIdx.x] = a;
-    }
+    if (threadIdx.x < RP) s[threadIdx.x] = sums[threadIdx.x];
     __syncthreads();
     const int64_t total = (int64_t)n * RP;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;

@@ -42,11 +42,13 @@ struct StreamOps {
                                        const double *W, int n, int p, const StreamK &sk,
                                        double *part, RunState *st, int grid,
                                        cudaStream_t s) const = 0;
+    // The updates, with the new factor's Gram and sums as `g` asks.
     virtual void h_epi(double *H, void *Ht, int p, const double *part, const StreamK &sk,
-                       int tcols, const EpiParams &e, const RunState *st,
-                       cudaStream_t s) const = 0;
+                       int tcols, const EpiParams &e, const GramOut &g, GramPlan gp,
+                       const RunState *st, cudaStream_t s) const = 0;
     virtual void w_epi(double *W, int n, const double *part, const StreamK &sk, int trows,
-                       const EpiParams &e, const RunState *st, cudaStream_t s) const = 0;
+                       const EpiParams &e, const GramOut &g, GramPlan gp, const RunState *st,
+                       cudaStream_t s) const = 0;
     // f32 only: W (n x RP f64) -> the f32 copy (n x rps()) that the H pass streams.
     virtual void w_copy(const double *W, void *Wc, int n, const RunState *st,
                         cudaStream_t s) const = 0;

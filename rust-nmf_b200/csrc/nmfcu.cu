@@ -122,19 +122,12 @@ struct Ops {
     virtual void off_update(const double *W, int n, int r, const double *rsh, const double *rsv,
                             int p, double eps, double *off, const RunState *st,
                             cudaStream_t s) const = 0;
-    virtual void gram_w(const double *W, int n, int B, int rows_per_block, double *pg,
-                        double *ps, const RunState *st, cudaStream_t s) const = 0;
-    virtual void gram_h(const double *H, int p, int B, int cols_per_block, double *pg,
-                        double *ps, const RunState *st, cudaStream_t s) const = 0;
-    // The same partials, and the finished Gram G and sums from the launch's
-    // last block (one launch; ticket zero before and after).
-    virtual void gram_w_fin(const double *W, int n, int B, int rows_per_block, double *pg,
-                            double *ps, double *G, double *sums, unsigned *ticket,
-                            const RunState *st, cudaStream_t s) const = 0;
-    virtual void gram_h_fin(const double *H, int p, int B, int cols_per_block, double *pg,
-                            double *ps, double *G, double *sums, unsigned *ticket,
-                            const RunState *st, cudaStream_t s) const = 0;
-    virtual void rescale(double *W, int n, int r, const double *ps, int B, const RunState *st,
+    // Gram and sums of W / H (kernels.cuh).
+    virtual void gram_w(const double *W, int n, const GramOut &g, GramPlan gp, const RunState *st,
+                        cudaStream_t s) const = 0;
+    virtual void gram_h(const double *H, int p, const GramOut &g, GramPlan gp, const RunState *st,
+                        cudaStream_t s) const = 0;
+    virtual void rescale(double *W, int n, int r, const double *sums, const RunState *st,
                          cudaStream_t s) const = 0;
     virtual void dnmf_scale(double *W, double *H, int n, int p, int r, const double *Gw,
                             const double *Gh, const RunState *st, cudaStream_t s) const = 0;
@@ -184,31 +177,19 @@ struct OpsT final : Ops {
         if (n > 0)
             nmfcu::off_update<RP><<<cdiv(n, kThreads), kThreads, 0, s>>>(W, n, r, rsh, rsv, p, eps, off, st);
     }
-    void gram_w(const double *W, int n, int B, int rows_per_block, double *pg, double *ps,
-                const RunState *st, cudaStream_t s) const override {
-        gram_w_partial<RP><<<B, RP * RP, 0, s>>>(W, n, rows_per_block, pg, ps, st);
+    void gram_w(const double *W, int n, const GramOut &g, GramPlan gp, const RunState *st,
+                cudaStream_t s) const override {
+        launch_gram_w<RP>(W, n, g, gp, st, s);
     }
-    void gram_h(const double *H, int p, int B, int cols_per_block, double *pg, double *ps,
-                const RunState *st, cudaStream_t s) const override {
-        gram_h_partial<RP><<<B, RP * RP, 0, s>>>(H, p, cols_per_block, pg, ps, st);
+    void gram_h(const double *H, int p, const GramOut &g, GramPlan gp, const RunState *st,
+                cudaStream_t s) const override {
+        launch_gram_h<RP>(H, p, g, gp, st, s);
     }
-    void gram_w_fin(const double *W, int n, int B, int rows_per_block, double *pg, double *ps,
-                    double *G, double *sums, unsigned *ticket, const RunState *st,
-                    cudaStream_t s) const override {
-        gram_w_partial<RP><<<B, RP * RP, 0, s>>>(W, n, rows_per_block, pg, ps, st, G, sums,
-                                                 ticket);
-    }
-    void gram_h_fin(const double *H, int p, int B, int cols_per_block, double *pg, double *ps,
-                    double *G, double *sums, unsigned *ticket, const RunState *st,
-                    cudaStream_t s) const override {
-        gram_h_partial<RP><<<B, RP * RP, 0, s>>>(H, p, cols_per_block, pg, ps, st, G, sums,
-                                                 ticket);
-    }
-    void rescale(double *W, int n, int r, const double *ps, int B, const RunState *st,
+    void rescale(double *W, int n, int r, const double *sums, const RunState *st,
                  cudaStream_t s) const override {
         if (n <= 0) return;
         const unsigned blocks = std::min<unsigned>(cdiv((int64_t)n * RP, kThreads), 1184u);
-        col_rescale<RP><<<blocks, kThreads, 0, s>>>(W, n, r, ps, B, st);
+        col_rescale<RP><<<blocks, kThreads, 0, s>>>(W, n, r, sums, st);
     }
     void dnmf_scale(double *W, double *H, int n, int p, int r, const double *Gw,
                     const double *Gh, const RunState *st, cudaStream_t s) const override {
@@ -354,8 +335,7 @@ struct DevBuf {
 struct Plan {
     int n = 0, p = 0, r = 0, RP = 0;
     int S2 = 1, cols_per_split = 1;    // objective pass column splits
-    int Bw = 1, rows_per_gram = 1;     // W Gram blocks
-    int Bh = 1, cols_per_gram = 1;     // H Gram blocks
+    GramPlan gw{true, 1}, gh{true, 1}; // the W / H epilogues and Grams
     int obj_blocks = 0;                // objective partial count
 };
 
@@ -373,10 +353,8 @@ Plan make_plan(int64_t n, int64_t p, int64_t r, int sms) {
     pl.cols_per_split = (int)cps;
     pl.S2 = (int)std::max<int64_t>(1, (p + cps - 1) / cps);
     pl.obj_blocks = (int)(((n + kThreads - 1) / kThreads) * pl.S2);
-    pl.Bw = (int)std::max<int64_t>(1, std::min<int64_t>((n + 63) / 64, sms));
-    pl.rows_per_gram = (int)std::max<int64_t>(1, (n + pl.Bw - 1) / pl.Bw);
-    pl.Bh = (int)std::max<int64_t>(1, std::min<int64_t>((p + 63) / 64, sms));
-    pl.cols_per_gram = (int)std::max<int64_t>(1, (p + pl.Bh - 1) / pl.Bh);
+    pl.gw = gram_plan(n, kTileRows, sms);
+    pl.gh = gram_plan(p, kTileCols, sms);
     return pl;
 }
 
@@ -434,7 +412,7 @@ struct nmfcu_context {
     std::mutex mu;
 
     // Workspace.
-    DevBuf V64, V32, W, H, part, pg, ps, Gw, sw, Gh, sh, Gw2, sw2, obj, dev, state;
+    DevBuf V64, V32, W, H, part, pg, Gw, sw, Gh, sh, Gw2, sw2, obj, dev, state;
     DevBuf Wf32, Ht64, Ht32;
     DevBuf Vs, Fs;     // split-bf16 form: V hi/lo, the factor's three terms
     DevBuf Xs;         // split-bf16 brunet: W and H in the tcr tile and unit layouts
@@ -789,26 +767,34 @@ nmfcu_status enqueue_objective(nmfcu_context *c, const RunArgs &a, long long ite
     return NMFCU_OK;
 }
 
-// The Grams and sums in one launch each; the ticket lives in the run state,
-// which every run zeroes before its first launch.
-void gram_w_full(nmfcu_context *c, const RunArgs &a, double *G, double *sums, cudaStream_t s) {
-    const Plan &pl = a.pl;
-    RunState *st = c->state.as<RunState>();
-    nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER);
-    a.ops->gram_w_fin(a.W, pl.n, pl.Bw, pl.rows_per_gram, c->pg.as<double>(), c->ps.as<double>(),
-                      G, sums, &st->gram_ticket, st, s);
+// Where an epilogue or Gram launch leaves the Gram and sums.  The ticket lives
+// in the run state, which every run zeroes before its first launch.
+GramOut gram_out(nmfcu_context *c, int want, double *G, double *sums, bool rescaled = false) {
+    GramOut g;
+    g.want = want;
+    g.rescaled = rescaled ? 1 : 0;
+    g.part = c->pg.as<double>();
+    g.G = G;
+    g.sums = sums;
+    g.ticket = c->state.as<RunState>()->gram_ticket;
+    return g;
 }
-void gram_h_full(nmfcu_context *c, const RunArgs &a, double *G, double *sums, cudaStream_t s) {
-    const Plan &pl = a.pl;
-    RunState *st = c->state.as<RunState>();
+void gram_w_full(nmfcu_context *c, const RunArgs &a, double *G, double *sums, cudaStream_t s,
+                 int want = GRAM_FULL, bool rescaled = false) {
     nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER);
-    a.ops->gram_h_fin(a.H, pl.p, pl.Bh, pl.cols_per_gram, c->pg.as<double>(), c->ps.as<double>(),
-                      G, sums, &st->gram_ticket, st, s);
+    a.ops->gram_w(a.W, a.pl.n, gram_out(c, want, G, sums, rescaled), a.pl.gw,
+                  c->state.as<RunState>(), s);
+}
+void gram_h_full(nmfcu_context *c, const RunArgs &a, double *G, double *sums, cudaStream_t s,
+                 int want = GRAM_FULL) {
+    nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER);
+    a.ops->gram_h(a.H, a.pl.p, gram_out(c, want, G, sums), a.pl.gh, c->state.as<RunState>(), s);
 }
 
-// H step: the streaming contraction over all rows, then the per-column update.
+// H step: the streaming contraction over all rows, then the per-column update
+// (and the new H's Gram and sums as `g` asks).
 nmfcu_status h_step(nmfcu_context *c, const RunArgs &a, const PassSet &ps, const EpiParams &e,
-                    bool ratio, cudaStream_t s) {
+                    bool ratio, cudaStream_t s, const GramOut &g = GramOut()) {
     const Plan &pl = a.pl;
     RunState *st = c->state.as<RunState>();
     if (ps.tcr) {
@@ -830,7 +816,8 @@ nmfcu_status h_step(nmfcu_context *c, const RunArgs &a, const PassSet &ps, const
                                      c->part.as<double>(), st, s));
         }
         nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER);
-        ps.so->h_epi(a.H, nullptr, pl.p, c->part.as<double>(), sk, kTcTile, e, st, s);
+        ps.so->h_epi(a.H, nullptr, pl.p, c->part.as<double>(), sk, kTcTile, e, g, pl.gh, st, s);
+        CUDA_TRY(cudaPeekAtLastError());
         return NMFCU_OK;
     }
     if (ps.tc) {
@@ -846,7 +833,8 @@ nmfcu_status h_step(nmfcu_context *c, const RunArgs &a, const PassSet &ps, const
                                     c->part.as<double>(), st, s));
         }
         nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER);
-        ps.so->h_epi(a.H, ps.Ht, pl.p, c->part.as<double>(), sk, kTcTile, e, st, s);
+        ps.so->h_epi(a.H, ps.Ht, pl.p, c->part.as<double>(), sk, kTcTile, e, g, pl.gh, st, s);
+        CUDA_TRY(cudaPeekAtLastError());
         return NMFCU_OK;
     }
     const int tcols = ps.so->h_tcols(ratio);
@@ -868,13 +856,15 @@ nmfcu_status h_step(nmfcu_context *c, const RunArgs &a, const PassSet &ps, const
                                   c->part.as<double>(), st, sk.G, s));
     }
     nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER);
-    ps.so->h_epi(a.H, ps.Ht, pl.p, c->part.as<double>(), sk, tcols, e, st, s);
+    ps.so->h_epi(a.H, ps.Ht, pl.p, c->part.as<double>(), sk, tcols, e, g, pl.gh, st, s);
+    CUDA_TRY(cudaPeekAtLastError());
     return NMFCU_OK;
 }
 
-// W step: the streaming contraction over all columns, then the per-row update.
+// W step: the streaming contraction over all columns, then the per-row update
+// (and the new W's Gram and sums as `g` asks).
 nmfcu_status w_step(nmfcu_context *c, const RunArgs &a, const PassSet &ps, const EpiParams &e,
-                    bool ratio, cudaStream_t s) {
+                    bool ratio, cudaStream_t s, const GramOut &g = GramOut()) {
     const Plan &pl = a.pl;
     RunState *st = c->state.as<RunState>();
     if (ps.tcr) {
@@ -896,7 +886,9 @@ nmfcu_status w_step(nmfcu_context *c, const RunArgs &a, const PassSet &ps, const
                                      c->part.as<double>(), st, s));
         }
         nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER);
-        ps.so->w_epi(a.Wout ? a.Wout : a.W, pl.n, c->part.as<double>(), sk, kTcTile, e, st, s);
+        ps.so->w_epi(a.Wout ? a.Wout : a.W, pl.n, c->part.as<double>(), sk, kTcTile, e, g, pl.gw, st,
+                     s);
+        CUDA_TRY(cudaPeekAtLastError());
         return NMFCU_OK;
     }
     if (ps.tc) {
@@ -912,7 +904,9 @@ nmfcu_status w_step(nmfcu_context *c, const RunArgs &a, const PassSet &ps, const
                                     c->part.as<double>(), st, s));
         }
         nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER);
-        ps.so->w_epi(a.Wout ? a.Wout : a.W, pl.n, c->part.as<double>(), sk, kTcTile, e, st, s);
+        ps.so->w_epi(a.Wout ? a.Wout : a.W, pl.n, c->part.as<double>(), sk, kTcTile, e, g, pl.gw, st,
+                     s);
+        CUDA_TRY(cudaPeekAtLastError());
         return NMFCU_OK;
     }
     const int trows = ps.so->w_trows(ratio);
@@ -929,7 +923,8 @@ nmfcu_status w_step(nmfcu_context *c, const RunArgs &a, const PassSet &ps, const
                                   c->part.as<double>(), st, sk.G, s));
     }
     nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER);
-    ps.so->w_epi(a.Wout ? a.Wout : a.W, pl.n, c->part.as<double>(), sk, trows, e, st, s);
+    ps.so->w_epi(a.Wout ? a.Wout : a.W, pl.n, c->part.as<double>(), sk, trows, e, g, pl.gw, st, s);
+    CUDA_TRY(cudaPeekAtLastError());
     return NMFCU_OK;
 }
 
@@ -958,7 +953,10 @@ EpiParams epi(const nmfcu_options *o, int r, const double *G, const double *sums
     return e;
 }
 
-// Enqueue one full iteration `it` (1-based).
+// Enqueue one full iteration `it` (1-based).  The Grams and sums the steps
+// divide by come with the epilogue that wrote the factor; a launch of their
+// own forms them where something else wrote it since: the start, a clamp, an
+// extrapolation, a scaling, a smoothing.
 nmfcu_status enqueue_iteration(nmfcu_context *c, const RunArgs &a, long long it, bool fp64,
                                cudaStream_t s) {
     const Plan &pl = a.pl;
@@ -971,10 +969,13 @@ nmfcu_status enqueue_iteration(nmfcu_context *c, const RunArgs &a, long long it,
     switch (o->method) {
         case NMFCU_BRUNET: {
             // nmf_run_brunet lib.rs:1558-1575.
-            gram_w_full(c, a, Gw, sw, s);  // sum_w (lib.rs:1563-1568)
-            NMF_TRY(h_step(c, a, ps, epi(o, pl.r, Gw, sw, true), true, s));
-            gram_h_full(c, a, Gh, sh, s);  // sum_h (lib.rs:161-169)
-            NMF_TRY(w_step(c, a, ps, epi(o, pl.r, Gh, sh, false), true, s));
+            // sum_w (lib.rs:1563-1568) and sum_h (lib.rs:161-169); the Grams
+            // themselves are not used.
+            if (it % 10 == 1) gram_w_full(c, a, Gw, sw, s, GRAM_SUMS);
+            NMF_TRY(h_step(c, a, ps, epi(o, pl.r, nullptr, sw, true), true, s,
+                           gram_out(c, GRAM_SUMS, Gh, sh)));
+            NMF_TRY(w_step(c, a, ps, epi(o, pl.r, nullptr, sh, false), true, s,
+                           gram_out(c, it % 10 == 0 ? GRAM_NONE : GRAM_SUMS, Gw, sw)));
             if (it % 10 == 0) {
                 nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER);
                 a.ops->clamp(a.W, a.H, pl.n, pl.p, pl.r, DBL_EPSILON, st, s);
@@ -983,15 +984,15 @@ nmfcu_status enqueue_iteration(nmfcu_context *c, const RunArgs &a, long long it,
         }
         case NMFCU_LEE: {
             // nmf_run_lee lib.rs:1618-1636.
-            gram_w_full(c, a, Gw, sw, s);  // W^T W (lib.rs:1622-1631)
-            NMF_TRY(h_step(c, a, ps, epi(o, pl.r, Gw, sw, true), false, s));
-            gram_h_full(c, a, Gh, sh, s);  // H H^T (lib.rs:293-302)
-            NMF_TRY(w_step(c, a, ps, epi(o, pl.r, Gh, sh, false), false, s));
+            // W^T W (lib.rs:1622-1631) and H H^T (lib.rs:293-302)
+            if (it == 1) gram_w_full(c, a, Gw, sw, s);
+            NMF_TRY(h_step(c, a, ps, epi(o, pl.r, Gw, sw, true), false, s,
+                           gram_out(c, GRAM_FULL, Gh, sh)));
+            NMF_TRY(w_step(c, a, ps, epi(o, pl.r, Gh, sh, false), false, s,
+                           gram_out(c, GRAM_FULL, Gw, sw, o->rescale != 0)));
             if (o->rescale) {
-                nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER, 2);
-                a.ops->gram_w(a.W, pl.n, pl.Bw, pl.rows_per_gram, c->pg.as<double>(),
-                              c->ps.as<double>(), st, s);
-                a.ops->rescale(a.W, pl.n, pl.r, c->ps.as<double>(), pl.Bw, st, s);
+                nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER);
+                a.ops->rescale(a.W, pl.n, pl.r, sw, st, s);
             }
             break;
         }
@@ -1004,8 +1005,8 @@ nmfcu_status enqueue_iteration(nmfcu_context *c, const RunArgs &a, long long it,
                 nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER);
                 a.ops->ns_right(a.W, pl.n, pl.r, o->theta, a.Wns, st, s);
             }
-            gram_w_full(c, aw, Gw, sw, s);  // colsum(W S)
-            NMF_TRY(h_step(c, aw, ps, epi(o, pl.r, Gw, sw, true), true, s));
+            gram_w_full(c, aw, Gw, sw, s, GRAM_SUMS);  // colsum(W S)
+            NMF_TRY(h_step(c, aw, ps, epi(o, pl.r, nullptr, sw, true), true, s));
             RunArgs ah = a;
             ah.H = a.Hns;
             {
@@ -1015,31 +1016,30 @@ nmfcu_status enqueue_iteration(nmfcu_context *c, const RunArgs &a, long long it,
             // The W pass streams (S H)^T (the tensor-core passes split S H
             // themselves).
             if (!ps.tcr) transpose_h(c, ah, ps, s);
-            gram_h_full(c, ah, Gh, sh, s);  // rowsum(S H)
-            NMF_TRY(w_step(c, ah, ps, epi(o, pl.r, Gh, sh, false), true, s));
+            gram_h_full(c, ah, Gh, sh, s, GRAM_SUMS);  // rowsum(S H)
+            NMF_TRY(w_step(c, ah, ps, epi(o, pl.r, nullptr, sh, false), true, s,
+                           gram_out(c, GRAM_SUMS, Gw, sw)));
             {
-                nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER, 2);
-                a.ops->gram_w(a.W, pl.n, pl.Bw, pl.rows_per_gram, c->pg.as<double>(),
-                              c->ps.as<double>(), st, s);
-                a.ops->rescale(a.W, pl.n, pl.r, c->ps.as<double>(), pl.Bw, st, s);
+                nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER);
+                a.ops->rescale(a.W, pl.n, pl.r, sw, st, s);
             }
             break;
         }
         case NMFCU_OFFSET: {
             // nmf_run_offset lib.rs:1694-1742: lee updates with the offset
             // terms, then the offset update.
-            gram_w_full(c, a, Gw, sw, s);  // W^T W
+            if (it == 1) gram_w_full(c, a, Gw, sw, s);  // W^T W
             {
                 nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER);
                 a.ops->off_addon(a.W, pl.n, pl.r, a.off, a.addon, st, s);
             }
             EpiParams eh = epi(o, pl.r, Gw, sw, true);
             eh.addon = a.addon;
-            NMF_TRY(h_step(c, a, ps, eh, false, s));
-            gram_h_full(c, a, Gh, sh, s);  // H H^T, rowSums(H)
+            // H H^T, rowSums(H)
+            NMF_TRY(h_step(c, a, ps, eh, false, s, gram_out(c, GRAM_FULL, Gh, sh)));
             EpiParams ew = epi(o, pl.r, Gh, sh, false);
             ew.roff = a.off;
-            NMF_TRY(w_step(c, a, ps, ew, false, s));
+            NMF_TRY(w_step(c, a, ps, ew, false, s, gram_out(c, GRAM_FULL, Gw, sw)));
             {
                 nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER);
                 a.ops->off_update(a.W, pl.n, pl.r, sh, a.rsv, pl.p, o->eps, a.off, st, s);
@@ -1081,12 +1081,15 @@ nmfcu_status enqueue_iteration(nmfcu_context *c, const RunArgs &a, long long it,
             [[fallthrough]];
         default: {
             // nmf_run_hals lib.rs:667-676; nmf_run_dnmf lib.rs:862-884.
-            gram_w_full(c, a, Gw, sw, s);
-            NMF_TRY(h_step(c, a, ps, epi(o, pl.r, Gw, sw, true), false, s));
-            gram_h_full(c, a, Gh, sh, s);
-            NMF_TRY(w_step(c, a, ps, epi(o, pl.r, Gh, sh, false), false, s));
-            if (o->method == NMFCU_DNMF) {
-                gram_w_full(c, a, c->Gw2.as<double>(), c->sw2.as<double>(), s);
+            const bool dnmf = o->method == NMFCU_DNMF;
+            if (it == 1 || o->method != NMFCU_HALS) gram_w_full(c, a, Gw, sw, s);
+            NMF_TRY(h_step(c, a, ps, epi(o, pl.r, Gw, sw, true), false, s,
+                           gram_out(c, GRAM_FULL, Gh, sh)));
+            NMF_TRY(w_step(c, a, ps, epi(o, pl.r, Gh, sh, false), false, s,
+                           o->method == NMFCU_EHALS ? GramOut()
+                           : dnmf ? gram_out(c, GRAM_FULL, c->Gw2.as<double>(), c->sw2.as<double>())
+                                  : gram_out(c, GRAM_FULL, Gw, sw)));
+            if (dnmf) {
                 nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER);
                 a.ops->dnmf_scale(a.W, a.H, pl.n, pl.p, pl.r, c->Gw2.as<double>(), Gh, st, s);
             }
@@ -1133,9 +1136,8 @@ std::vector<WsNeed> workspace_needs(nmfcu_context *c, const Plan &pl, bool need_
         v.push_back({&c->Ht32, sizeof(float) * (size_t)pl.p * rps});
         v.push_back({&c->Wf32, sizeof(float) * (size_t)pl.n * rps});
     }
-    const size_t B = (size_t)std::max(pl.Bw, pl.Bh);
-    v.push_back({&c->pg, sizeof(double) * B * RP * RP});
-    v.push_back({&c->ps, sizeof(double) * B * RP});
+    v.push_back({&c->pg, sizeof(double) * (size_t)(std::max(pl.gw.blocks, pl.gh.blocks) + 32) *
+                             gram_entries(pl.RP)});
     v.push_back({&c->Gw, sizeof(double) * RP * RP});
     v.push_back({&c->Gh, sizeof(double) * RP * RP});
     v.push_back({&c->Gw2, sizeof(double) * RP * RP});
@@ -1761,7 +1763,7 @@ void drain_timing(nmfcu_context *c) {
 
 size_t context_bytes(nmfcu_context *c) {
     size_t t = 0;
-    for (const DevBuf *b : {&c->V64, &c->V32, &c->W, &c->H, &c->part, &c->pg, &c->ps, &c->Gw,
+    for (const DevBuf *b : {&c->V64, &c->V32, &c->W, &c->H, &c->part, &c->pg, &c->Gw,
                             &c->sw, &c->Gh, &c->sh, &c->Gw2, &c->sw2, &c->obj, &c->dev, &c->state,
                             &c->Wf32, &c->Ht64, &c->Ht32, &c->Vs, &c->Fs, &c->Xs, &c->Wns, &c->Hns,
                             &c->off, &c->rsv, &c->addon, &c->Wprev, &c->Hprev,
@@ -1795,7 +1797,7 @@ size_t slot_growth(nmfcu_context *c, int slot, size_t bytes) {
 
 void context_release(nmfcu_context *c) {
     DeviceGuard dg(c->device);
-    for (DevBuf *b : {&c->V64, &c->V32, &c->W, &c->H, &c->part, &c->pg, &c->ps, &c->Gw, &c->sw,
+    for (DevBuf *b : {&c->V64, &c->V32, &c->W, &c->H, &c->part, &c->pg, &c->Gw, &c->sw,
                       &c->Gh, &c->sh, &c->Gw2, &c->sw2, &c->obj, &c->dev, &c->state, &c->Wf32,
                       &c->Ht64, &c->Ht32, &c->Vs, &c->Fs, &c->Xs, &c->Wns, &c->Hns,
                             &c->off, &c->rsv, &c->addon, &c->Wprev, &c->Hprev,
@@ -2414,9 +2416,11 @@ nmfcu_status nmfcu_shard_step(nmfcu_shard *sh, int32_t phase, void *stream) {
             const PassSet &ps = fp64 ? a.p64 : a.main;
             const bool ratio = (o->method == NMFCU_BRUNET);
             double *Gw = c->Gw.as<double>(), *sw = c->sw.as<double>();
-            gram_w_full(c, a, Gw, sw, s);
-            NMF_TRY(h_step(c, a, ps, epi(o, pl.r, Gw, sw, true), ratio, s));
-            gram_h_full(c, a, RG, Rs, s);
+            // (lee's rescaled W has its Gram from the W update)
+            if (itn == 1 || !(o->method == NMFCU_LEE && o->rescale))
+                gram_w_full(c, a, Gw, sw, s);
+            NMF_TRY(h_step(c, a, ps, epi(o, pl.r, Gw, sw, true), ratio, s,
+                           gram_out(c, GRAM_FULL, RG, Rs)));
             RunArgs aw = a;
             aw.Wout = Rnum;
             EpiParams ep = epi(o, pl.r, nullptr, nullptr, false);
@@ -2436,10 +2440,10 @@ nmfcu_status nmfcu_shard_step(nmfcu_shard *sh, int32_t phase, void *stream) {
                 nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER);
                 a.ops->clamp(a.W, a.H, pl.n, pl.p, pl.r, DBL_EPSILON, st, s);
             } else if (o->method == NMFCU_LEE && o->rescale) {
-                nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER, 2);
-                a.ops->gram_w(a.W, pl.n, pl.Bw, pl.rows_per_gram, c->pg.as<double>(),
-                              c->ps.as<double>(), st, s);
-                a.ops->rescale(a.W, pl.n, pl.r, c->ps.as<double>(), pl.Bw, st, s);
+                double *Gw = c->Gw.as<double>(), *sw = c->sw.as<double>();
+                gram_w_full(c, a, Gw, sw, s, GRAM_FULL, true);
+                nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER);
+                a.ops->rescale(a.W, pl.n, pl.r, sw, st, s);
             } else if (o->method == NMFCU_DNMF) {
                 gram_w_full(c, a, c->Gw2.as<double>(), c->sw2.as<double>(), s);
                 nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER);

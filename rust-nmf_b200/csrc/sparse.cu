@@ -39,6 +39,8 @@
 #include "../../include/nmfcu.h"
 #include "internal.h"
 #include "kernels.cuh"
+#include "launch.h"
+#include "stream.cuh"
 
 using nmfcu_internal::fail;
 
@@ -317,10 +319,11 @@ struct SparseV {
 
 struct Work {
     double *W, *H, *Ht, *numW, *numH;          // padded factors, contractions
-    double *pg, *ps, *Gw, *sw, *Gh, *sh, *Gw2, *sw2;
+    double *pg, *Gw, *sw, *Gh, *sh, *Gw2, *sw2;
     double *opart, *obj, *dev;
     RunState *st;
-    int Bw, rows_per_gram, Bh, cols_per_gram, Bo;
+    nmfcu::GramPlan gw, gh;
+    int Bo;
 };
 
 // Carves `sizes` (bytes) out of one context slot, 256-byte aligned.
@@ -393,6 +396,7 @@ struct Loop {
     cudaStream_t s;
     int sms;
 
+    // H^T of an H the last epilogue did not write.
     void transpose_h() {
         if (p <= 0) return;
         nmfcu_internal::TimedScope sc(c, s, NMFCU_KCLASS_OTHER);
@@ -400,15 +404,30 @@ struct Loop {
             std::max(1u, std::min<unsigned>(cdiv((int64_t)p * RP, kT), 4096u));
         nmfcu::h_transpose<double><<<blocks, kT, 0, s>>>(w.H, w.Ht, p, r, RP);
     }
+    nmfcu::GramOut gram_out(int want, double *G, double *sums, bool rescaled = false) const {
+        nmfcu::GramOut g;
+        g.want = want;
+        g.rescaled = rescaled ? 1 : 0;
+        g.part = w.pg;
+        g.G = G;
+        g.sums = sums;
+        g.ticket = w.st->gram_ticket;
+        return g;
+    }
     void gram_w(double *G, double *sums) {
-        nmfcu_internal::TimedScope sc(c, s, NMFCU_KCLASS_OTHER, 2);
-        nmfcu::gram_w_partial<RP><<<w.Bw, RP * RP, 0, s>>>(w.W, n, w.rows_per_gram, w.pg, w.ps, w.st);
-        nmfcu::gram_finalize<RP><<<1, RP * RP, 0, s>>>(w.pg, w.ps, w.Bw, G, sums, w.st);
+        nmfcu_internal::TimedScope sc(c, s, NMFCU_KCLASS_OTHER);
+        nmfcu::launch_gram_w<RP>(w.W, n, gram_out(nmfcu::GRAM_FULL, G, sums), w.gw, w.st, s);
     }
     void gram_h(double *G, double *sums) {
-        nmfcu_internal::TimedScope sc(c, s, NMFCU_KCLASS_OTHER, 2);
-        nmfcu::gram_h_partial<RP><<<w.Bh, RP * RP, 0, s>>>(w.H, p, w.cols_per_gram, w.pg, w.ps, w.st);
-        nmfcu::gram_finalize<RP><<<1, RP * RP, 0, s>>>(w.pg, w.ps, w.Bh, G, sums, w.st);
+        nmfcu_internal::TimedScope sc(c, s, NMFCU_KCLASS_OTHER);
+        nmfcu::launch_gram_h<RP>(w.H, p, gram_out(nmfcu::GRAM_FULL, G, sums), w.gh, w.st, s);
+    }
+    // The contractions as partials of one CTA's one slot.
+    static nmfcu::StreamK one_slot() {
+        nmfcu::StreamK sk;
+        sk.U = 1;
+        sk.G = sk.UPT = sk.slots = sk.nseg = sk.fold = sk.valid = 1;
+        return sk;
     }
     EpiParams epi(const double *G, const double *sums, bool hside) const {
         EpiParams e;
@@ -421,41 +440,40 @@ struct Loop {
         e.sums = sums;
         return e;
     }
-    void h_step(bool ratio, const EpiParams &e) {
-        if (ratio) transpose_h();
+    void h_step(bool ratio, const EpiParams &e, const nmfcu::GramOut &g) {
         {
             nmfcu_internal::TimedScope sc(c, s, NMFCU_KCLASS_HSTEP);
-            const unsigned g = line_grid(p, sms);
+            const unsigned grid = line_grid(p, sms);
             if (ratio)
-                sparse_pass<RP, true, true><<<g, kT, 0, s>>>(sv.cptr, sv.cidx, sv.cval, p, p, w.Ht,
+                sparse_pass<RP, true, true><<<grid, kT, 0, s>>>(sv.cptr, sv.cidx, sv.cval, p, p, w.Ht,
                                                              w.W, w.numH, w.st);
             else
-                sparse_pass<RP, false, true><<<g, kT, 0, s>>>(sv.cptr, sv.cidx, sv.cval, p, p,
+                sparse_pass<RP, false, true><<<grid, kT, 0, s>>>(sv.cptr, sv.cidx, sv.cval, p, p,
                                                               nullptr, w.W, w.numH, w.st);
         }
         nmfcu_internal::TimedScope sc(c, s, NMFCU_KCLASS_OTHER);
-        nmfcu::h_epilogue<RP><<<std::max(1u, cdiv(p, kT)), kT, 0, s>>>(w.H, p, w.numH, 1, e, w.st);
+        nmfcu::launch_h_epilogue<RP, double, RP>(w.H, w.Ht, p, w.numH, one_slot(), std::max(p, 1),
+                                                 e, g, w.gh, w.st, s);
     }
-    void w_step(bool ratio, const EpiParams &e) {
-        transpose_h();
+    void w_step(bool ratio, const EpiParams &e, const nmfcu::GramOut &g) {
         {
             nmfcu_internal::TimedScope sc(c, s, NMFCU_KCLASS_WSTEP);
-            const unsigned g = line_grid(n, sms);
+            const unsigned grid = line_grid(n, sms);
             if (ratio)
-                sparse_pass<RP, true, false><<<g, kT, 0, s>>>(sv.rptr, sv.ridx, sv.rval, n, 0, w.W,
+                sparse_pass<RP, true, false><<<grid, kT, 0, s>>>(sv.rptr, sv.ridx, sv.rval, n, 0, w.W,
                                                               w.Ht, w.numW, w.st);
             else
-                sparse_pass<RP, false, false><<<g, kT, 0, s>>>(sv.rptr, sv.ridx, sv.rval, n, 0,
+                sparse_pass<RP, false, false><<<grid, kT, 0, s>>>(sv.rptr, sv.ridx, sv.rval, n, 0,
                                                                nullptr, w.Ht, w.numW, w.st);
         }
         nmfcu_internal::TimedScope sc(c, s, NMFCU_KCLASS_OTHER);
-        nmfcu::w_epilogue<RP><<<std::max(1u, cdiv(n, kT)), kT, 0, s>>>(w.W, n, w.numW, 1, e, w.st);
+        nmfcu::launch_w_epilogue<RP>(w.W, n, w.numW, one_slot(), std::max(n, 1), e, g, w.gw, w.st,
+                                     s);
     }
     void objective(long long iter) {
         const bool kl = (o->method == NMFCU_BRUNET);
         gram_w(w.Gw2, w.sw2);
         gram_h(w.Gh, w.sh);
-        transpose_h();
         {
             nmfcu_internal::TimedScope sc(c, s, NMFCU_KCLASS_OBJECTIVE, 2);
             if (kl) {
@@ -484,45 +502,51 @@ struct Loop {
         switch (o->method) {
             case NMFCU_BRUNET:
                 // nmf_run_brunet lib.rs:1558-1575
-                gram_w(w.Gw, w.sw);
-                h_step(true, epi(w.Gw, w.sw, true));
-                gram_h(w.Gh, w.sh);
-                w_step(true, epi(w.Gh, w.sh, false));
+                if (it % 10 == 1) gram_w(w.Gw, w.sw);
+                h_step(true, epi(nullptr, w.sw, true), gram_out(nmfcu::GRAM_SUMS, w.Gh, w.sh));
+                w_step(true, epi(nullptr, w.sh, false),
+                       gram_out(it % 10 == 0 ? nmfcu::GRAM_NONE : nmfcu::GRAM_SUMS, w.Gw, w.sw));
                 if (it % 10 == 0) {
-                    nmfcu_internal::TimedScope sc(c, s, NMFCU_KCLASS_OTHER);
-                    const int64_t m = std::max<int64_t>((int64_t)n * RP, (int64_t)r * p);
-                    nmfcu::clamp_wh<RP><<<std::max(1u, std::min<unsigned>(cdiv(m, kT), 1184u)), kT, 0, s>>>(
-                        w.W, w.H, n, p, r, DBL_EPSILON, w.st);
+                    {
+                        nmfcu_internal::TimedScope sc(c, s, NMFCU_KCLASS_OTHER);
+                        const int64_t m = std::max<int64_t>((int64_t)n * RP, (int64_t)r * p);
+                        nmfcu::clamp_wh<RP><<<std::max(1u, std::min<unsigned>(cdiv(m, kT), 1184u)), kT, 0, s>>>(
+                            w.W, w.H, n, p, r, DBL_EPSILON, w.st);
+                    }
+                    transpose_h();
                 }
                 break;
             case NMFCU_LEE:
                 // nmf_run_lee lib.rs:1618-1636
-                gram_w(w.Gw, w.sw);
-                h_step(false, epi(w.Gw, w.sw, true));
-                gram_h(w.Gh, w.sh);
-                w_step(false, epi(w.Gh, w.sh, false));
+                if (it == 1) gram_w(w.Gw, w.sw);
+                h_step(false, epi(w.Gw, w.sw, true), gram_out(nmfcu::GRAM_FULL, w.Gh, w.sh));
+                w_step(false, epi(w.Gh, w.sh, false),
+                       gram_out(nmfcu::GRAM_FULL, w.Gw, w.sw, o->rescale != 0));
                 if (o->rescale && n > 0) {
-                    nmfcu_internal::TimedScope sc(c, s, NMFCU_KCLASS_OTHER, 2);
-                    nmfcu::gram_w_partial<RP><<<w.Bw, RP * RP, 0, s>>>(w.W, n, w.rows_per_gram,
-                                                                       w.pg, w.ps, w.st);
-                    nmfcu::col_rescale<RP><<<std::min<unsigned>(cdiv((int64_t)n * RP, kT), 1184u), kT, 0, s>>>(
-                        w.W, n, r, w.ps, w.Bw, w.st);
-                }
-                break;
-            default:
-                // nmf_run_hals lib.rs:667-676; nmf_run_dnmf lib.rs:862-884
-                gram_w(w.Gw, w.sw);
-                h_step(false, epi(w.Gw, w.sw, true));
-                gram_h(w.Gh, w.sh);
-                w_step(false, epi(w.Gh, w.sh, false));
-                if (o->method == NMFCU_DNMF) {
-                    gram_w(w.Gw2, w.sw2);
                     nmfcu_internal::TimedScope sc(c, s, NMFCU_KCLASS_OTHER);
-                    const int64_t m = std::max<int64_t>((int64_t)n * RP, (int64_t)r * p);
-                    nmfcu::dnmf_rescale<RP><<<std::max(1u, std::min<unsigned>(cdiv(m, kT), 1184u)), kT, 0, s>>>(
-                        w.W, w.H, n, p, r, w.Gw2, w.Gh, w.st);
+                    nmfcu::col_rescale<RP><<<std::min<unsigned>(cdiv((int64_t)n * RP, kT), 1184u), kT, 0, s>>>(
+                        w.W, n, r, w.sw, w.st);
                 }
                 break;
+            default: {
+                // nmf_run_hals lib.rs:667-676; nmf_run_dnmf lib.rs:862-884
+                const bool dnmf = o->method == NMFCU_DNMF;
+                if (it == 1 || dnmf) gram_w(w.Gw, w.sw);
+                h_step(false, epi(w.Gw, w.sw, true), gram_out(nmfcu::GRAM_FULL, w.Gh, w.sh));
+                w_step(false, epi(w.Gh, w.sh, false),
+                       dnmf ? gram_out(nmfcu::GRAM_FULL, w.Gw2, w.sw2)
+                            : gram_out(nmfcu::GRAM_FULL, w.Gw, w.sw));
+                if (dnmf) {
+                    {
+                        nmfcu_internal::TimedScope sc(c, s, NMFCU_KCLASS_OTHER);
+                        const int64_t m = std::max<int64_t>((int64_t)n * RP, (int64_t)r * p);
+                        nmfcu::dnmf_rescale<RP><<<std::max(1u, std::min<unsigned>(cdiv(m, kT), 1184u)), kT, 0, s>>>(
+                            w.W, w.H, n, p, r, w.Gw2, w.Gh, w.st);
+                    }
+                    transpose_h();
+                }
+                break;
+            }
         }
     }
 };
@@ -540,29 +564,26 @@ nmfcu_status make_work(nmfcu_context *c, int64_t n, int64_t p, int RP, int64_t m
     w.Ht = static_cast<double *>(b[2]);
     w.numW = static_cast<double *>(b[3]);
     w.numH = static_cast<double *>(b[4]);
-    w.Bw = (int)std::max<int64_t>(1, std::min<int64_t>((n + 63) / 64, sms));
-    w.rows_per_gram = (int)std::max<int64_t>(1, (n + w.Bw - 1) / w.Bw);
-    w.Bh = (int)std::max<int64_t>(1, std::min<int64_t>((p + 63) / 64, sms));
-    w.cols_per_gram = (int)std::max<int64_t>(1, (p + w.Bh - 1) / w.Bh);
+    w.gw = nmfcu::gram_plan(n, nmfcu::kTileRows, sms);
+    w.gh = nmfcu::gram_plan(p, nmfcu::kTileCols, sms);
     w.Bo = (int)line_grid(n, sms);
-    const int B = std::max(w.Bw, w.Bh);
+    const int B = std::max(w.gw.blocks, w.gh.blocks) + 32;
     const size_t g = d * RP * RP, v = d * RP;
     NMFCU_TRY(carve(c, kSlotSmall,
-                    {d * B * RP * RP, d * B * RP, g, v, g, v, g, v, d * 2 * w.Bo, d * 8,
+                    {d * B * nmfcu::gram_entries(RP), g, v, g, v, g, v, d * 2 * w.Bo, d * 8,
                      sizeof(RunState), d * (size_t)(max_iter + 1)},
                     b));
     w.pg = static_cast<double *>(b[0]);
-    w.ps = static_cast<double *>(b[1]);
-    w.Gw = static_cast<double *>(b[2]);
-    w.sw = static_cast<double *>(b[3]);
-    w.Gh = static_cast<double *>(b[4]);
-    w.sh = static_cast<double *>(b[5]);
-    w.Gw2 = static_cast<double *>(b[6]);
-    w.sw2 = static_cast<double *>(b[7]);
-    w.opart = static_cast<double *>(b[8]);
-    w.obj = static_cast<double *>(b[9]);
-    w.st = static_cast<RunState *>(b[10]);
-    w.dev = static_cast<double *>(b[11]);
+    w.Gw = static_cast<double *>(b[1]);
+    w.sw = static_cast<double *>(b[2]);
+    w.Gh = static_cast<double *>(b[3]);
+    w.sh = static_cast<double *>(b[4]);
+    w.Gw2 = static_cast<double *>(b[5]);
+    w.sw2 = static_cast<double *>(b[6]);
+    w.opart = static_cast<double *>(b[7]);
+    w.obj = static_cast<double *>(b[8]);
+    w.st = static_cast<RunState *>(b[9]);
+    w.dev = static_cast<double *>(b[10]);
     return NMFCU_OK;
 }
 
@@ -572,6 +593,7 @@ nmfcu_status run_loop_t(nmfcu_context *c, const nmfcu_options *o, int64_t n, int
                         int64_t *n_iter) {
     Loop<RP> L{c, o, (int)n, (int)p, (int)r, sv, w, s, nmfcu_internal::context_sms(c)};
     NMFCU_CUDA_TRY(cudaMemsetAsync(w.st, 0, sizeof(RunState), s));
+    L.transpose_h();
     if (stat) L.objective(0);
     for (long long it = 1; it <= o->max_iter; it++) {
         L.iteration(it);

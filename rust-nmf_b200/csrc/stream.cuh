@@ -730,19 +730,10 @@ __global__ void __launch_bounds__(WCfg<T, RP, RATIO>::kWarps * 32, 1)
 // FP64 plain passes on the FP64 tensor cores (lee / hals / dnmf / offset,
 // the lsNMF numerators and the NNDSVD products in the plain method)
 // ---------------------------------------------------------------------------
-// mma.sync.m8n8k4 with f64 operands: D (8 x 8) += A (8 x 4) B (4 x 8), one
-// A and one B element and two D elements a thread (A[g][q], B[q][g],
-// D[g][2q + e] with g = lane / 4, q = lane % 4).  One instruction does 256
-// FMAs, where the CUDA-core passes issue one DFMA (and its operand loads)
-// per 32; the ring, stream-K split and partial layouts are the CUDA-core
-// passes' own, so the epilogues are shared.  The asm has no side effects
-// beyond its operands (not volatile), so independent MMAs may be scheduled
-// across one another; each accumulator's chain keeps its order.
-__device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {
-    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-        : "+d"(d[0]), "+d"(d[1])
-        : "d"(a), "d"(b));
-}
+// mma.sync.m8n8k4 (dmma_8x8x4, kernels.cuh): one instruction does 256 FMAs,
+// where the CUDA-core passes issue one DFMA (and its operand loads) per 32;
+// the ring, stream-K split and partial layouts are the CUDA-core passes' own,
+// so the epilogues are shared.
 
 // H pass: A[k][j] = sum_u W[u][k] V[u][j] with M = k (rank tiles of 8), N = j
 // (4 column tiles of 8 a warp), K = u (4 rows a k-step, 4 k-steps a unit of
@@ -1445,145 +1436,390 @@ __global__ void __launch_bounds__(DWRCfg<RP>::kWarps * 32, 1)
 // Epilogues for the stream-K partials
 // ---------------------------------------------------------------------------
 
-// Sum of the partials of output `c` of major tile `mt`, over its segments and
-// their CTAs, in that order.  `stride_k` / `stride_row` describe the partial
-// layout: element (slot base) + k * stride_k + c * stride_c.
-template <int RP>
-__device__ __forceinline__ void gather_partials(const double *__restrict__ part,
-                                                const StreamK &sk, int mt, size_t slot_elems,
-                                                size_t off, size_t stride_k, double (&num)[RP]) {
-#pragma unroll
-    for (int k = 0; k < RP; k++) num[k] = 0.0;
-    if (sk.G <= 0) return;  // no units at all: every sum is empty
-    if (sk.fold) {
-        int lo, hi;
-        sk_range_major(sk, mt, &lo, &hi);
-        for (int b = lo; b <= hi; b++) {
-            const double *src =
-                part + ((size_t)b * sk.slots + fold_slot(sk, b, mt)) * slot_elems + off;
-#pragma unroll
-            for (int k = 0; k < RP; k++) num[k] += src[(size_t)k * stride_k];
-        }
-        return;
+// The partials of a major tile: CTAs lo..hi.  A CTA after the first begins
+// inside the tile, so its slot is 0; the first's is slot_lo.
+struct TilePartials {
+    int lo, hi, slot_lo;
+    template <typename U>
+    __device__ __forceinline__ void find_as(const StreamK &sk, int mt) {
+        const U G = (U)sk.G, units = (U)sk.U, mu = (U)sk.major_units();
+        const U a = (U)mt * mu;
+        const U e = min(a + (U)sk.valid, units);
+        // start(b) = floor(b U / G) <= x  <=>  b <= ((x + 1) G - 1) / U
+        lo = (int)(((a + 1) * G - 1) / units);
+        hi = (int)((e * G - 1) / units);
+        slot_lo = mt - (int)(((U)lo * units / G) / mu);
     }
-    for (int seg = 0; seg < sk.nseg; seg++) {
-        const int t = mt * sk.nseg + seg;
-        int lo, hi;
-        sk_range(sk, t, &lo, &hi);
-        for (int b = lo; b <= hi; b++) {
-            const int slot = t - (int)(sk.start(b) / sk.UPT);
-            const double *src = part + ((size_t)b * sk.slots + slot) * slot_elems + off;
-#pragma unroll
-            for (int k = 0; k < RP; k++) num[k] += src[(size_t)k * stride_k];
-        }
+    __device__ __forceinline__ void find(const StreamK &sk, int mt) {
+        lo = 0;
+        hi = -1;  // no units at all: every sum is empty
+        slot_lo = 0;
+        if (sk.G <= 0) return;
+        if (sk.U < (1ll << 31) / sk.G)  // 32-bit divisions
+            find_as<unsigned>(sk, mt);
+        else
+            find_as<unsigned long long>(sk, mt);
     }
-}
+    __device__ __forceinline__ size_t slot(const StreamK &sk, int b) const {
+        return (size_t)b * sk.slots + (b == lo ? slot_lo : 0);
+    }
+};
 
-// One thread per column: sum the partials, apply the H update, write H
-// (RP x p, f64) and the copy H^T (p x RPS_T, type TH) the next W pass streams.
-template <int RP, typename TH, int RPS_T>
-__global__ void __launch_bounds__(kThreads)
+// Doubles of shared memory of an epilogue launch.
+template <int RP, int THREADS>
+struct EpiSmem {
+    static constexpr bool FEW = THREADS == kEpiThreads;
+    static constexpr int WARPS = THREADS / 32;
+    // few tiles: shares of a row's (H) / an element's (W) partials
+    static constexpr int NSH = WARPS / RP > 1 ? WARPS / RP : 1;
+    static constexpr int NSW = THREADS / (kTileRows * RP) > 1 ? THREADS / (kTileRows * RP) : 1;
+    static constexpr int TILES_H =
+        FEW ? (NSH + 2) * RP * (kTileCols + 1) : WARPS * RP * (kTileCols + 1);
+    static constexpr int TILES_W =
+        FEW ? NSW * kTileRows * RP + 2 * kTileRows * (RP + 1) : WARPS * 32 * (RP + 1);
+    static constexpr int TREE = GramAcc<RP, THREADS>::SCRATCH;
+    static constexpr int G = RP * RP;
+    static constexpr int H = G + (TILES_H > TREE ? TILES_H : TREE);
+    static constexpr int W = G + (TILES_W > TREE ? TILES_W : TREE);
+};
+
+// H update: the sums of a column's partials, the update, H (RP x p, f64), the
+// copy H^T (p x RPS_T, type TH) the next W pass streams, and the new H's terms
+// of H H^T / rowsum(H).  Few tiles: latency counts, so a block's warps share
+// a tile (a warp a row k, split further where the rank leaves warps over).
+// Many: a thread a column.
+//
+// One thread a column throughout, searching its partials' CTAs by bisection,
+// took 22.7 us at 1500 x 3000 rank 8, and the Gram 9.1 us in a launch of its own.
+template <int RP, typename TH, int RPS_T, int THREADS>
+__global__ void __launch_bounds__(THREADS)
     h_epilogue_sk(double *__restrict__ H, TH *__restrict__ Ht, int p,
-                  const double *__restrict__ part, StreamK sk, int tcols, EpiParams e,
+                  const double *__restrict__ part, StreamK sk, int tcols, EpiParams e, GramOut g,
                   const RunState *st) {
     if (run_stopped(st)) return;
-    const int j = blockIdx.x * kThreads + threadIdx.x;
-    if (j >= p) return;
-    const int ct = j / tcols, c = j - ct * tcols;
-    double num[RP], hc[RP];
-    gather_partials<RP>(part, sk, ct, (size_t)RP * tcols, c, tcols, num);
+    using ES = EpiSmem<RP, THREADS>;
+    constexpr int TC = kTileCols, LD = kTileCols + 1, WARPS = THREADS / 32;
+    extern __shared__ double smem_epi[];
+    double *sG = smem_epi, *tile = smem_epi + ES::G;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (e.G != nullptr)
+        for (int x = threadIdx.x; x < RP * RP; x += THREADS) sG[x] = e.G[x];
+    EpiParams es = e;
+    es.G = sG;
+    GramAcc<RP, THREADS> ga;
+    ga.init();
+    TilePartials tp;
+    if constexpr (ES::FEW) {
+        constexpr int NS = ES::NSH;
+        double *sNum = tile, *sOld = tile + NS * RP * LD, *sNew = sOld + RP * LD;
+        const int j0 = blockIdx.x * TC, j = j0 + lane;
+        const int ct = j0 / tcols, c = j0 - ct * tcols + lane;
+        tp.find(sk, ct);
+        for (int k = warp; k < RP; k += WARPS)
+            sOld[k * LD + lane] = j < p ? H[(size_t)k * p + j] : 0.0;
+        for (int it = warp; it < RP * NS; it += WARPS) {
+            const int s = it / RP, k = it - s * RP;
+            double a = 0.0;
+            if (j < p) {
+                const double *src = part + (size_t)k * tcols + c;
+#pragma unroll 8
+                for (int b = tp.lo + s; b <= tp.hi; b += NS)
+                    a += src[tp.slot(sk, b) * RP * tcols];
+            }
+            sNum[(s * RP + k) * LD + lane] = a;
+        }
+        __syncthreads();
+        if (w_update_by_column(e.method)) {
+            for (int k = warp; k < RP; k += WARPS) {
+                double v = 0.0;
+                if (k < e.r && j < p) {
+                    double num = sNum[k * LD + lane];
 #pragma unroll
-    for (int k = 0; k < RP; k++) hc[k] = H[(size_t)k * p + j];
-    double ax[RP];
+                    for (int s = 1; s < NS; s++) num += sNum[(s * RP + k) * LD + lane];
+                    const double ax = e.aux != nullptr ? e.aux[(size_t)k * p + j] : 0.0;
+                    v = h_update_row<RP>(
+                        es, num, [&](int l) { return sOld[l * LD + lane]; }, k, ax);
+                    H[(size_t)k * p + j] = v;
+                }
+                sNew[k * LD + lane] = v;
+            }
+        } else if (warp == 0) {
+            // The HALS / dnmf sweeps run over a column's rows in order.
+            double num[RP], hc[RP];
 #pragma unroll
-    for (int k = 0; k < RP; k++) ax[k] = (e.aux != nullptr && k < e.r) ? e.aux[(size_t)k * p + j] : 0.0;
-    h_update<RP>(e, num, hc, ax);
+            for (int k = 0; k < RP; k++) {
+                num[k] = sNum[k * LD + lane];
 #pragma unroll
-    for (int k = 0; k < RP; k++)
-        if (k < e.r) H[(size_t)k * p + j] = hc[k];
-    if (Ht == nullptr) return;  // the tensor-core passes stream their own H terms
-    TH *ht = Ht + (size_t)j * RPS_T;
+                for (int s = 1; s < NS; s++) num[k] += sNum[(s * RP + k) * LD + lane];
+                hc[k] = sOld[k * LD + lane];
+            }
+            h_update<RP>(es, num, hc);
 #pragma unroll
-    for (int k = 0; k < RPS_T; k++) ht[k] = (k < e.r && k < RP) ? (TH)hc[k] : (TH)0;
+            for (int k = 0; k < RP; k++) {
+                const bool in = k < e.r && j < p;
+                sNew[k * LD + lane] = in ? hc[k] : 0.0;
+                if (in) H[(size_t)k * p + j] = hc[k];
+            }
+        }
+        __syncthreads();
+        if (Ht != nullptr) {  // (the tensor-core passes stream their own H terms)
+            TH *ht = Ht + (size_t)j0 * RPS_T;
+            const int cols = min(TC, p - j0);
+            for (int x = threadIdx.x; x < cols * RPS_T; x += THREADS) {
+                const int cc = x / RPS_T, k = x - cc * RPS_T;
+                ht[x] = k < RP ? (TH)sNew[k * LD + cc] : (TH)0;
+            }
+        }
+        if (g.want != GRAM_NONE && warp < TC / 4)
+            ga.add4(g.want, [&](int k, int q) { return sNew[k * LD + 4 * warp + q]; });
+    } else {
+        double *sNew = tile + warp * RP * LD;  // this warp's
+        __syncthreads();                       // sG
+        const int tiles = (p + TC - 1) / TC;
+        for (int t = blockIdx.x * WARPS + warp; t < tiles; t += gridDim.x * WARPS) {
+            const int j0 = t * TC, j = j0 + lane;
+            const int ct = j0 / tcols, c = j0 - ct * tcols + lane;
+            tp.find(sk, ct);
+            double num[RP], hc[RP];
+#pragma unroll
+            for (int k = 0; k < RP; k++) {
+                num[k] = 0.0;
+                hc[k] = j < p ? H[(size_t)k * p + j] : 0.0;
+            }
+            if (j < p)
+                for (int b = tp.lo; b <= tp.hi; b++) {
+                    const double *src = part + tp.slot(sk, b) * RP * tcols + c;
+#pragma unroll
+                    for (int k = 0; k < RP; k++) num[k] += src[(size_t)k * tcols];
+                }
+            double ax[RP];
+#pragma unroll
+            for (int k = 0; k < RP; k++)
+                ax[k] = (e.aux != nullptr && k < e.r && j < p) ? e.aux[(size_t)k * p + j] : 0.0;
+            h_update<RP>(es, num, hc, ax);
+            __syncwarp();  // the last tile's readers of sNew
+#pragma unroll
+            for (int k = 0; k < RP; k++) {
+                const bool in = k < e.r && j < p;
+                sNew[k * LD + lane] = in ? hc[k] : 0.0;
+                if (in) H[(size_t)k * p + j] = hc[k];
+            }
+            __syncwarp();
+            if (Ht != nullptr) {
+                TH *ht = Ht + (size_t)j0 * RPS_T;
+                const int cols = min(TC, p - j0);
+                for (int x = lane; x < cols * RPS_T; x += 32) {
+                    const int cc = x / RPS_T, k = x - cc * RPS_T;
+                    ht[x] = k < RP ? (TH)sNew[k * LD + cc] : (TH)0;
+                }
+            }
+            if (g.want != GRAM_NONE)
+                for (int s = 0; s < TC / 4; s++)
+                    ga.add4(g.want, [&](int k, int q) { return sNew[k * LD + 4 * s + q]; });
+        }
+    }
+    ga.finish(g, tile);
 }
 
-// One warp per row: lane l adds the partials of segments l, l + 32, ...
-// (each over its CTAs in order; with folded partials, of CTAs l, l + 32, ...
-// of the row tile), a fixed xor butterfly adds the lanes, and
-// lane 0 applies the W update -- a long row (many column segments) is
-// gathered 32 segments at a time.  Deterministic.
-template <int RP>
-__global__ void __launch_bounds__(kThreads)
+// W update: a row's partials lie contiguous in each CTA's slot.  Few tiles: a
+// thread an element of the block's tile (split further where that leaves
+// threads over); many: a thread a row, its sums and values by way of the
+// warp's shared memory so that the loads and stores are contiguous.  (A warp a
+// row took 9.0 us at 1500 x 3000 rank 8, the Gram 6.3 us in a launch of its own.)
+template <int RP, int THREADS>
+__global__ void __launch_bounds__(THREADS)
     w_epilogue_sk(double *__restrict__ W, int n, const double *__restrict__ part, StreamK sk,
-                  int trows, EpiParams e, const RunState *st) {
+                  int trows, EpiParams e, GramOut g, const RunState *st) {
     if (run_stopped(st)) return;
-    const int i = (int)(((size_t)blockIdx.x * kThreads + threadIdx.x) >> 5);
-    const int lane = threadIdx.x & 31;
-    if (i >= n) return;  // uniform across the warp
-    const int rt = i / trows, rl = i - rt * trows;
-    double num[RP];
-#pragma unroll
-    for (int k = 0; k < RP; k++) num[k] = 0.0;
-    if (sk.G > 0 && sk.fold) {
-        // Folded partials: lane l adds CTAs lo + l, lo + l + 32, ...
-        const size_t slot_elems = (size_t)trows * RP;
-        int lo, hi;
-        sk_range_major(sk, rt, &lo, &hi);
-        for (int b = lo + lane; b <= hi; b += 32) {
-            const double *src = part + ((size_t)b * sk.slots + fold_slot(sk, b, rt)) * slot_elems +
-                                (size_t)rl * RP;
-#pragma unroll
-            for (int k = 0; k < RP; k++) num[k] += src[k];
+    using ES = EpiSmem<RP, THREADS>;
+    constexpr int WARPS = THREADS / 32, LD = RP + 1;
+    extern __shared__ double smem_epi[];
+    double *sG = smem_epi, *tile = smem_epi + ES::G;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (e.G != nullptr)
+        for (int x = threadIdx.x; x < RP * RP; x += THREADS) sG[x] = e.G[x];
+    EpiParams es = e;
+    es.G = sG;
+    GramAcc<RP, THREADS> ga;
+    ga.init();
+    TilePartials tp;
+    if constexpr (ES::FEW) {
+        constexpr int TR = kTileRows, EL = TR * RP, NS = ES::NSW;
+        double *sNum = tile, *sOld = tile + NS * EL, *sNew = sOld + TR * LD;
+        const int i0 = blockIdx.x * TR;
+        const int rt = i0 / trows, rl = i0 - rt * trows;
+        const int elems = min(TR, n - i0) * RP;
+        tp.find(sk, rt);
+        for (int x = threadIdx.x; x < EL; x += THREADS)
+            sOld[(x / RP) * LD + x % RP] = x < elems ? W[(size_t)i0 * RP + x] : 0.0;
+        for (int it = threadIdx.x; it < EL * NS; it += THREADS) {
+            const int s = it / EL, x = it - s * EL;
+            double a = 0.0;
+            if (x < elems) {
+                const double *src = part + (size_t)rl * RP + x;
+#pragma unroll 8
+                for (int b = tp.lo + s; b <= tp.hi; b += NS)
+                    a += src[tp.slot(sk, b) * trows * RP];
+            }
+            sNum[it] = a;
         }
-    } else if (sk.G > 0) {
-        const size_t slot_elems = (size_t)trows * RP;
-        for (int seg = lane; seg < sk.nseg; seg += 32) {
-            const int t = rt * sk.nseg + seg;
-            int lo, hi;
-            sk_range(sk, t, &lo, &hi);
-            for (int b = lo; b <= hi; b++) {
-                const int slot = t - (int)(sk.start(b) / sk.UPT);
-                const double *src = part + ((size_t)b * sk.slots + slot) * slot_elems + (size_t)rl * RP;
+        __syncthreads();
+        if (w_update_by_column(e.method)) {
+            for (int x = threadIdx.x; x < EL; x += THREADS) {
+                const int u = x / RP, k = x - u * RP;
+                double v = 0.0;
+                if (x < elems && k < e.r) {
+                    double num = sNum[x];
 #pragma unroll
-                for (int k = 0; k < RP; k++) num[k] += src[k];
+                    for (int s = 1; s < NS; s++) num += sNum[s * EL + x];
+                    const int i = i0 + u;
+                    v = w_update_column<RP>(es, num, sOld + u * LD, k,
+                                            e.roff != nullptr ? e.roff[i] : 0.0,
+                                            e.aux != nullptr ? e.aux + (size_t)i * RP : nullptr);
+                    W[(size_t)i0 * RP + x] = v;
+                }
+                sNew[u * LD + k] = v;
+            }
+        } else if (threadIdx.x < TR) {
+            // The HALS / dnmf sweeps run over a row's columns in order.
+            const int u = threadIdx.x;
+            double num[RP], wr[RP];
+#pragma unroll
+            for (int k = 0; k < RP; k++) {
+                num[k] = sNum[u * RP + k];
+#pragma unroll
+                for (int s = 1; s < NS; s++) num[k] += sNum[s * EL + u * RP + k];
+                wr[k] = sOld[u * LD + k];
+            }
+            w_update<RP>(es, num, wr);
+#pragma unroll
+            for (int k = 0; k < RP; k++) {
+                const bool in = k < e.r && u * RP < elems;
+                sNew[u * LD + k] = in ? wr[k] : 0.0;
+                if (in) W[(size_t)(i0 + u) * RP + k] = wr[k];
             }
         }
-    }
-#pragma unroll
-    for (int k = 0; k < RP; k++)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) num[k] += __shfl_xor_sync(0xffffffffu, num[k], o);
-    // Every lane now holds the row's sums.  Methods whose columns update
-    // independently take one lane a column; the HALS / dnmf sweeps, which
-    // run over the columns in order, lane 0.
-    double wr[RP];
-#pragma unroll
-    for (int k = 0; k < RP; k++) wr[k] = W[(size_t)i * RP + k];
-    const double ro = e.roff ? e.roff[i] : 0.0;
-    if (w_update_by_column(e.method)) {
-        if (lane >= e.r || lane >= RP) return;
-        double numj = 0.0, wrj = 0.0;
-#pragma unroll
-        for (int k = 0; k < RP; k++)
-            if (k == lane) {
-                numj = num[k];
-                wrj = wr[k];
+        __syncthreads();
+        if (g.want != GRAM_NONE && warp < TR / 4)
+            ga.add4(g.want, [&](int k, int q) { return sNew[(4 * warp + q) * LD + k]; });
+    } else {
+        double *sRow = tile + warp * 32 * LD;  // this warp's 32 rows
+        __syncthreads();                       // sG
+        const int tiles = (n + 31) / 32;
+        for (int t = blockIdx.x * WARPS + warp; t < tiles; t += gridDim.x * WARPS) {
+            const int i0 = t * 32, i = i0 + lane;
+            const int rt = i0 / trows, rl = i0 - rt * trows;
+            const int elems = min(32, n - i0) * RP;
+            tp.find(sk, rt);
+            double num[RP], wr[RP];
+            __syncwarp();  // the last tile's readers of sRow
+#pragma unroll 4
+            for (int x = lane; x < 32 * RP; x += 32) {
+                double a = 0.0;
+                if (x < elems) {
+                    const double *src = part + (size_t)rl * RP + x;
+                    for (int b = tp.lo; b <= tp.hi; b++) a += src[tp.slot(sk, b) * trows * RP];
+                }
+                sRow[(x / RP) * LD + x % RP] = a;
             }
-        const double *ax = e.aux != nullptr ? e.aux + (size_t)i * RP : nullptr;
-        const double out = w_update_column<RP>(e, numj, wrj, wr, lane, ro, ax);
-        // All lanes have read the row before any writes it.
-        __syncwarp(__activemask());
-        W[(size_t)i * RP + lane] = out;
-        return;
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < RP; k++) num[k] = sRow[lane * LD + k];
+            __syncwarp();
+#pragma unroll 4
+            for (int x = lane; x < 32 * RP; x += 32)
+                sRow[(x / RP) * LD + x % RP] = x < elems ? W[(size_t)i0 * RP + x] : 0.0;
+            __syncwarp();
+            double ax[RP];
+#pragma unroll
+            for (int k = 0; k < RP; k++) {
+                wr[k] = sRow[lane * LD + k];
+                ax[k] = (e.aux != nullptr && i < n) ? e.aux[(size_t)i * RP + k] : 0.0;
+            }
+            w_update<RP>(es, num, wr, (e.roff != nullptr && i < n) ? e.roff[i] : 0.0, ax);
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < RP; k++) {
+                // ranks past r keep what they hold
+                if (k < e.r) sRow[lane * LD + k] = i < n ? wr[k] : 0.0;
+            }
+            __syncwarp();
+#pragma unroll 4
+            for (int x = lane; x < elems; x += 32)
+                W[(size_t)i0 * RP + x] = sRow[(x / RP) * LD + x % RP];
+            if (g.want != GRAM_NONE)
+                for (int s = 0; s < 8; s++)
+                    ga.add4(g.want, [&](int k, int q) { return sRow[(4 * s + q) * LD + k]; });
+        }
     }
-    if (lane != 0) return;
-    double ax[RP];
-#pragma unroll
-    for (int k = 0; k < RP; k++) ax[k] = e.aux != nullptr ? e.aux[(size_t)i * RP + k] : 0.0;
-    w_update<RP>(e, num, wr, ro, ax);
-#pragma unroll
-    for (int k = 0; k < RP; k++)
-        if (k < e.r) W[(size_t)i * RP + k] = wr[k];
+    ga.finish(g, tile);
+}
+
+// Launchers; a kernel has to be allowed more than 48 KB of shared memory.
+template <typename Kernel>
+inline void allow_smem(Kernel *k, size_t bytes) {
+    if (bytes > 40 * 1024)  // (static shared memory counts too)
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+template <int RP, typename TH, int RPS_T>
+void launch_h_epilogue(double *H, TH *Ht, int p, const double *part, const StreamK &sk, int tcols,
+                       const EpiParams &e, const GramOut &g, GramPlan gp, const RunState *st,
+                       cudaStream_t s) {
+    if (p <= 0 && g.want == GRAM_NONE) return;
+    const auto go = [&](auto *k, int threads, size_t bytes) {
+        allow_smem(k, bytes);
+        k<<<gp.blocks, threads, bytes, s>>>(H, Ht, p, part, sk, tcols, e, g, st);
+    };
+    if (gp.few)
+        go(h_epilogue_sk<RP, TH, RPS_T, kEpiThreads>, kEpiThreads,
+           sizeof(double) * EpiSmem<RP, kEpiThreads>::H);
+    else
+        go(h_epilogue_sk<RP, TH, RPS_T, kWideThreads>, kWideThreads,
+           sizeof(double) * EpiSmem<RP, kWideThreads>::H);
+}
+template <int RP>
+void launch_w_epilogue(double *W, int n, const double *part, const StreamK &sk, int trows,
+                       const EpiParams &e, const GramOut &g, GramPlan gp, const RunState *st,
+                       cudaStream_t s) {
+    if (n <= 0 && g.want == GRAM_NONE) return;
+    const auto go = [&](auto *k, int threads, size_t bytes) {
+        allow_smem(k, bytes);
+        k<<<gp.blocks, threads, bytes, s>>>(W, n, part, sk, trows, e, g, st);
+    };
+    if (gp.few)
+        go(w_epilogue_sk<RP, kEpiThreads>, kEpiThreads,
+           sizeof(double) * EpiSmem<RP, kEpiThreads>::W);
+    else
+        go(w_epilogue_sk<RP, kWideThreads>, kWideThreads,
+           sizeof(double) * EpiSmem<RP, kWideThreads>::W);
+}
+template <int RP>
+void launch_gram_w(const double *W, int n, const GramOut &g, GramPlan gp, const RunState *st,
+                   cudaStream_t s) {
+    const auto go = [&](auto *k, int threads, size_t bytes) {
+        allow_smem(k, bytes);
+        k<<<gp.blocks, threads, bytes, s>>>(W, n, g, st);
+    };
+    if (gp.few)
+        go(gram_w_tiles<RP, kEpiThreads>, kEpiThreads,
+           sizeof(double) * GramAcc<RP, kEpiThreads>::SCRATCH);
+    else
+        go(gram_w_tiles<RP, kWideThreads>, kWideThreads,
+           sizeof(double) * GramAcc<RP, kWideThreads>::SCRATCH);
+}
+template <int RP>
+void launch_gram_h(const double *H, int p, const GramOut &g, GramPlan gp, const RunState *st,
+                   cudaStream_t s) {
+    const auto go = [&](auto *k, int threads, size_t bytes) {
+        allow_smem(k, bytes);
+        k<<<gp.blocks, threads, bytes, s>>>(H, p, g, st);
+    };
+    if (gp.few)
+        go(gram_h_tiles<RP, kEpiThreads>, kEpiThreads,
+           sizeof(double) * GramAcc<RP, kEpiThreads>::SCRATCH);
+    else
+        go(gram_h_tiles<RP, kWideThreads>, kWideThreads,
+           sizeof(double) * GramAcc<RP, kWideThreads>::SCRATCH);
 }
 
 // f32 copy of W (n x RP f64 -> n x RPS f32, zero pad) for the f32 H pass.

@@ -166,16 +166,14 @@ struct StreamOpsT final : StreamOps {
             return cudaErrorNotSupported;
     }
     void h_epi(double *H, void *Ht, int p, const double *part, const StreamK &sk, int tcols,
-               const EpiParams &e, const RunState *st, cudaStream_t s) const override {
-        if (p <= 0) return;
-        h_epilogue_sk<RP, T, RPS><<<(p + kThreads - 1) / kThreads, kThreads, 0, s>>>(
-            H, static_cast<T *>(Ht), p, part, sk, tcols, e, st);
+               const EpiParams &e, const GramOut &g, GramPlan gp, const RunState *st,
+               cudaStream_t s) const override {
+        launch_h_epilogue<RP, T, RPS>(H, static_cast<T *>(Ht), p, part, sk, tcols, e, g, gp, st, s);
     }
     void w_epi(double *W, int n, const double *part, const StreamK &sk, int trows,
-               const EpiParams &e, const RunState *st, cudaStream_t s) const override {
-        if (n <= 0) return;
-        w_epilogue_sk<RP><<<(unsigned)(((size_t)n * 32 + kThreads - 1) / kThreads), kThreads, 0, s>>>(W, n, part, sk,
-                                                                            trows, e, st);
+               const EpiParams &e, const GramOut &g, GramPlan gp, const RunState *st,
+               cudaStream_t s) const override {
+        launch_w_epilogue<RP>(W, n, part, sk, trows, e, g, gp, st, s);
     }
     void w_copy(const double *W, void *Wc, int n, const RunState *st,
                 cudaStream_t s) const override {
