@@ -52,6 +52,7 @@ struct RunState {
 constexpr int kThreads = 256;
 constexpr int kWarps = 8;
 
+// (A kernel bound by latency reads it first and acts on it after its loads.)
 __device__ __forceinline__ bool run_stopped(const RunState *st) {
     return st != nullptr && st->stopped != 0;
 }
@@ -697,8 +698,10 @@ __device__ __forceinline__ double h_update_row(const EpiParams &e, double numi, 
 // A warp adds four rows (columns) of its tile at a time on the FP64 tensor
 // cores (mma.sync.m8n8k4: a fragment of X is both operands), a block adds its
 // warps in a fixed tree, publishes its entries and takes a ticket; the last
-// block of each group of 16 sums the group's partials, the last group the
-// groups'.  No block waits on another.  The update epilogues (stream.cuh)
+// block sums the blocks' partials.  Where that is more than 32 loads a thread
+// (a round trip to L2 per eight, and a second ticket costs two), the last
+// block of each group of 16 sums the group's and the last group the groups'.
+// No block waits on another.  The update epilogues (stream.cuh)
 // form the same sums over the same tiles from the values they have just
 // written, so a Gram has the same bits wherever it is formed.
 //
@@ -781,7 +784,43 @@ __device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {
         : "d"(a), "d"(b));
 }
 
-template <int RP, int THREADS>
+// a + src[0] + src[step] + ... (count of them, in order), up to eight loads in
+// flight at a time: left to itself the remainder of an unrolled loop waits for
+// its loads in ever smaller groups.
+template <int N, bool ALL, typename Load>
+__device__ __forceinline__ double sum_batch(double a, const double *&src, size_t step, int count,
+                                            Load &&load) {
+    double v[N];
+#pragma unroll
+    for (int u = 0; u < N; u++) {
+        v[u] = ALL || u < count ? load(src) : 0.0;
+        src += step;
+    }
+#pragma unroll
+    for (int u = 0; u < N; u++) a += v[u];
+    return a;
+}
+template <typename Load>
+__device__ __forceinline__ double sum_strided(double a, const double *src, size_t step, int count,
+                                              Load &&load) {
+    for (; count >= 8; count -= 8) a = sum_batch<8, true>(a, src, step, 8, load);
+    if (count > 4)
+        a = sum_batch<7, false>(a, src, step, count, load);
+    else if (count > 0)
+        a = sum_batch<4, false>(a, src, step, count, load);
+    return a;
+}
+
+// One more block's partials are out: its ticket.  Orders the block's earlier
+// writes before it and the other blocks' before what follows.
+__device__ __forceinline__ unsigned take_ticket(unsigned *t) {
+    unsigned old;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(t) : "memory");
+    return old;
+}
+
+// ACTIVE: the block's warps that add rows (the first ones).
+template <int RP, int THREADS, int ACTIVE>
 struct GramAcc {
     static constexpr int E = gram_entries(RP);
     static constexpr int MT = (RP + 7) / 8;
@@ -789,7 +828,7 @@ struct GramAcc {
     static constexpr int RAW = 2 * NP + MT;       // a lane's values
     static constexpr int WARPS = THREADS / 32;
     // Shared memory of finish(), in doubles.
-    static constexpr int SCRATCH_TREE = WARPS / 2 * RAW * 32;
+    static constexpr int SCRATCH_TREE = ACTIVE / 2 * RAW * 32;
     static constexpr int SCRATCH = SCRATCH_TREE > 2 * THREADS + RP ? SCRATCH_TREE : 2 * THREADS + RP;
     double d[NP][2], sm[MT];
     __device__ __forceinline__ void init() {
@@ -829,11 +868,10 @@ struct GramAcc {
     // tid < cnt where split > 1, else in thread e - base.
     __device__ __forceinline__ static double sum_parts(const double *src, int count, int e,
                                                        bool on, int first, int step) {
-        double a = 0.0;
-        if (on)
-#pragma unroll 8
-            for (int b = first; b < count; b += step) a += __ldcg(src + (size_t)b * E + e);
-        return a;
+        if (!on || first >= count) return 0.0;
+        return sum_strided(0.0, src + (size_t)first * E + e, (size_t)step * E,
+                           (count - first + step - 1) / step,
+                           [](const double *q) { return __ldcg(q); });
     }
     // `count` partials at src into dst (E entries each), or, with the last
     // group done, the finished Gram and sums.
@@ -888,7 +926,7 @@ struct GramAcc {
             sm[mt] += __shfl_xor_sync(0xffffffffu, sm[mt], 1);
             sm[mt] += __shfl_xor_sync(0xffffffffu, sm[mt], 2);
         }
-        for (int half = WARPS / 2; half >= 1; half >>= 1) {
+        for (int half = ACTIVE / 2; half >= 1; half >>= 1) {
             __syncthreads();
             if (warp >= half && warp < 2 * half) {
                 double *w = scratch + (size_t)(warp - half) * RAW * 32 + lane;
@@ -931,30 +969,26 @@ struct GramAcc {
             g.part[(size_t)blockIdx.x * E + e] = scratch[raw_index(k, l)];
         }
         __shared__ bool last;
-        __threadfence();
         __syncthreads();
         const double *src = g.part;
         int count = B;
-        if (B > 2 * kGramGroup) {
+        if (B > 2 * kGramGroup && (int64_t)B * limit > 32 * THREADS) {
             const int group = (int)blockIdx.x / kGramGroup;
             const int groups = (B + kGramGroup - 1) / kGramGroup;
             const int members = min(kGramGroup, B - group * kGramGroup);
-            if (tid == 0) last = (atomicAdd(g.ticket + 1 + group, 1u) == (unsigned)members - 1u);
+            if (tid == 0) last = (take_ticket(g.ticket + 1 + group) == (unsigned)members - 1u);
             __syncthreads();
             if (!last) return;
-            __threadfence();
             double *dst = g.part + (size_t)(B + group) * E;
             reduce(g.part + (size_t)group * kGramGroup * E, members, limit, dst, g, scratch);
             if (tid == 0) g.ticket[1 + group] = 0u;
-            __threadfence();
             __syncthreads();
             src = g.part + (size_t)B * E;
             count = groups;
         }
-        if (tid == 0) last = (atomicAdd(g.ticket, 1u) == (unsigned)count - 1u);
+        if (tid == 0) last = (take_ticket(g.ticket) == (unsigned)count - 1u);
         __syncthreads();
         if (!last) return;
-        __threadfence();
         reduce(src, count, limit, nullptr, g, scratch);
         if (tid == 0) *g.ticket = 0u;
     }
@@ -965,8 +999,8 @@ template <int RP, int THREADS>
 __global__ void __launch_bounds__(THREADS)
     gram_w_tiles(const double *__restrict__ W, int n, GramOut g, const RunState *st) {
     if (run_stopped(st)) return;
-    using GA = GramAcc<RP, THREADS>;
     constexpr bool FEW = THREADS == kEpiThreads;
+    using GA = GramAcc<RP, THREADS, FEW ? kTileRows / 4 : THREADS / 32>;
     extern __shared__ double scratch[];
     const int warp = threadIdx.x >> 5;
     GA ga;
@@ -994,8 +1028,8 @@ template <int RP, int THREADS>
 __global__ void __launch_bounds__(THREADS)
     gram_h_tiles(const double *__restrict__ H, int p, GramOut g, const RunState *st) {
     if (run_stopped(st)) return;
-    using GA = GramAcc<RP, THREADS>;
     constexpr bool FEW = THREADS == kEpiThreads;
+    using GA = GramAcc<RP, THREADS, FEW ? kTileCols / 4 : THREADS / 32>;
     extern __shared__ double scratch[];
     const int warp = threadIdx.x >> 5;
     GA ga;

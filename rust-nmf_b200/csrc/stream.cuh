@@ -1470,6 +1470,9 @@ template <int RP, int THREADS>
 struct EpiSmem {
     static constexpr bool FEW = THREADS == kEpiThreads;
     static constexpr int WARPS = THREADS / 32;
+    // Blocks of a multiprocessor at once: two for few tiles (up to 296 of
+    // them on 148 multiprocessors) where 64 registers hold a rank-12 sweep.
+    static constexpr int BLOCKS = FEW && RP <= 12 ? 2 : 1;
     // few tiles: shares of a row's (H) / an element's (W) partials
     static constexpr int NSH = WARPS / RP > 1 ? WARPS / RP : 1;
     static constexpr int NSW = THREADS / (kTileRows * RP) > 1 ? THREADS / (kTileRows * RP) : 1;
@@ -1477,10 +1480,11 @@ struct EpiSmem {
         FEW ? (NSH + 2) * RP * (kTileCols + 1) : WARPS * RP * (kTileCols + 1);
     static constexpr int TILES_W =
         FEW ? NSW * kTileRows * RP + 2 * kTileRows * (RP + 1) : WARPS * 32 * (RP + 1);
-    static constexpr int TREE = GramAcc<RP, THREADS>::SCRATCH;
+    using GH = GramAcc<RP, THREADS, FEW ? kTileCols / 4 : WARPS>;
+    using GW = GramAcc<RP, THREADS, FEW ? kTileRows / 4 : WARPS>;
     static constexpr int G = RP * RP;
-    static constexpr int H = G + (TILES_H > TREE ? TILES_H : TREE);
-    static constexpr int W = G + (TILES_W > TREE ? TILES_W : TREE);
+    static constexpr int H = G + (TILES_H > GH::SCRATCH ? TILES_H : GH::SCRATCH);
+    static constexpr int W = G + (TILES_W > GW::SCRATCH ? TILES_W : GW::SCRATCH);
 };
 
 // H update: the sums of a column's partials, the update, H (RP x p, f64), the
@@ -1492,42 +1496,67 @@ struct EpiSmem {
 // One thread a column throughout, searching its partials' CTAs by bisection,
 // took 22.7 us at 1500 x 3000 rank 8, and the Gram 9.1 us in a launch of its own.
 template <int RP, typename TH, int RPS_T, int THREADS>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, EpiSmem<RP, THREADS>::BLOCKS)
     h_epilogue_sk(double *__restrict__ H, TH *__restrict__ Ht, int p,
                   const double *__restrict__ part, StreamK sk, int tcols, EpiParams e, GramOut g,
                   const RunState *st) {
-    if (run_stopped(st)) return;
     using ES = EpiSmem<RP, THREADS>;
     constexpr int TC = kTileCols, LD = kTileCols + 1, WARPS = THREADS / 32;
     extern __shared__ double smem_epi[];
     double *sG = smem_epi, *tile = smem_epi + ES::G;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (e.G != nullptr)
-        for (int x = threadIdx.x; x < RP * RP; x += THREADS) sG[x] = e.G[x];
+    const bool stopped = run_stopped(st);
     EpiParams es = e;
     es.G = sG;
-    GramAcc<RP, THREADS> ga;
+    typename ES::GH ga;
     ga.init();
     TilePartials tp;
     if constexpr (ES::FEW) {
         constexpr int NS = ES::NSH;
+        constexpr int PG = (RP * RP + THREADS - 1) / THREADS, PK = (RP + WARPS - 1) / WARPS;
         double *sNum = tile, *sOld = tile + NS * RP * LD, *sNew = sOld + RP * LD;
         const int j0 = blockIdx.x * TC, j = j0 + lane;
         const int ct = j0 / tcols, c = j0 - ct * tcols + lane;
+        // All loads in flight before the first is used.
+        double gv[PG], ov[PK];
+#pragma unroll
+        for (int i = 0; i < PG; i++) {
+            const int x = threadIdx.x + i * THREADS;
+            gv[i] = e.G != nullptr && x < RP * RP ? e.G[x] : 0.0;
+        }
+#pragma unroll
+        for (int i = 0; i < PK; i++) {
+            const int k = warp + i * WARPS;
+            ov[i] = k < RP && j < p ? H[(size_t)k * p + j] : 0.0;
+        }
         tp.find(sk, ct);
-        for (int k = warp; k < RP; k += WARPS)
-            sOld[k * LD + lane] = j < p ? H[(size_t)k * p + j] : 0.0;
+        const size_t step = (size_t)sk.slots * RP * tcols;
         for (int it = warp; it < RP * NS; it += WARPS) {
             const int s = it / RP, k = it - s * RP;
             double a = 0.0;
             if (j < p) {
                 const double *src = part + (size_t)k * tcols + c;
-#pragma unroll 8
-                for (int b = tp.lo + s; b <= tp.hi; b += NS)
-                    a += src[tp.slot(sk, b) * RP * tcols];
+                int b = tp.lo + s;
+                if (s == 0 && b <= tp.hi) {  // the first CTA, whose slot may not be 0
+                    a = src[tp.slot(sk, b) * RP * tcols];
+                    b += NS;
+                }
+                a = sum_strided(a, src + b * step, NS * step, (tp.hi - b + NS) / NS,
+                                [](const double *q) { return *q; });
             }
             sNum[(s * RP + k) * LD + lane] = a;
         }
+#pragma unroll
+        for (int i = 0; i < PG; i++) {
+            const int x = threadIdx.x + i * THREADS;
+            if (x < RP * RP) sG[x] = gv[i];
+        }
+#pragma unroll
+        for (int i = 0; i < PK; i++) {
+            const int k = warp + i * WARPS;
+            if (k < RP) sOld[k * LD + lane] = ov[i];
+        }
+        if (stopped) return;
         __syncthreads();
         if (w_update_by_column(e.method)) {
             for (int k = warp; k < RP; k += WARPS) {
@@ -1574,7 +1603,10 @@ __global__ void __launch_bounds__(THREADS)
             ga.add4(g.want, [&](int k, int q) { return sNew[k * LD + 4 * warp + q]; });
     } else {
         double *sNew = tile + warp * RP * LD;  // this warp's
-        __syncthreads();                       // sG
+        if (e.G != nullptr)
+            for (int x = threadIdx.x; x < RP * RP; x += THREADS) sG[x] = e.G[x];
+        __syncthreads();
+        if (stopped) return;
         const int tiles = (p + TC - 1) / TC;
         for (int t = blockIdx.x * WARPS + warp; t < tiles; t += gridDim.x * WARPS) {
             const int j0 = t * TC, j = j0 + lane;
@@ -1627,42 +1659,68 @@ __global__ void __launch_bounds__(THREADS)
 // warp's shared memory so that the loads and stores are contiguous.  (A warp a
 // row took 9.0 us at 1500 x 3000 rank 8, the Gram 6.3 us in a launch of its own.)
 template <int RP, int THREADS>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, EpiSmem<RP, THREADS>::BLOCKS)
     w_epilogue_sk(double *__restrict__ W, int n, const double *__restrict__ part, StreamK sk,
                   int trows, EpiParams e, GramOut g, const RunState *st) {
-    if (run_stopped(st)) return;
     using ES = EpiSmem<RP, THREADS>;
     constexpr int WARPS = THREADS / 32, LD = RP + 1;
     extern __shared__ double smem_epi[];
     double *sG = smem_epi, *tile = smem_epi + ES::G;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (e.G != nullptr)
-        for (int x = threadIdx.x; x < RP * RP; x += THREADS) sG[x] = e.G[x];
+    const bool stopped = run_stopped(st);
     EpiParams es = e;
     es.G = sG;
-    GramAcc<RP, THREADS> ga;
+    typename ES::GW ga;
     ga.init();
     TilePartials tp;
     if constexpr (ES::FEW) {
         constexpr int TR = kTileRows, EL = TR * RP, NS = ES::NSW;
+        constexpr int PG = (RP * RP + THREADS - 1) / THREADS;
+        constexpr int PO = (EL + THREADS - 1) / THREADS;
         double *sNum = tile, *sOld = tile + NS * EL, *sNew = sOld + TR * LD;
         const int i0 = blockIdx.x * TR;
         const int rt = i0 / trows, rl = i0 - rt * trows;
         const int elems = min(TR, n - i0) * RP;
+        // All loads in flight before the first is used.
+        double gv[PG], ov[PO];
+#pragma unroll
+        for (int i = 0; i < PG; i++) {
+            const int x = threadIdx.x + i * THREADS;
+            gv[i] = e.G != nullptr && x < RP * RP ? e.G[x] : 0.0;
+        }
+#pragma unroll
+        for (int i = 0; i < PO; i++) {
+            const int x = threadIdx.x + i * THREADS;
+            ov[i] = x < elems ? W[(size_t)i0 * RP + x] : 0.0;
+        }
         tp.find(sk, rt);
-        for (int x = threadIdx.x; x < EL; x += THREADS)
-            sOld[(x / RP) * LD + x % RP] = x < elems ? W[(size_t)i0 * RP + x] : 0.0;
+        const size_t step = (size_t)sk.slots * trows * RP;
         for (int it = threadIdx.x; it < EL * NS; it += THREADS) {
             const int s = it / EL, x = it - s * EL;
             double a = 0.0;
             if (x < elems) {
                 const double *src = part + (size_t)rl * RP + x;
-#pragma unroll 8
-                for (int b = tp.lo + s; b <= tp.hi; b += NS)
-                    a += src[tp.slot(sk, b) * trows * RP];
+                int b = tp.lo + s;
+                if (s == 0 && b <= tp.hi) {  // the first CTA, whose slot may not be 0
+                    a = src[tp.slot(sk, b) * trows * RP];
+                    b += NS;
+                }
+                a = sum_strided(a, src + b * step, NS * step, (tp.hi - b + NS) / NS,
+                                [](const double *q) { return *q; });
             }
             sNum[it] = a;
         }
+#pragma unroll
+        for (int i = 0; i < PG; i++) {
+            const int x = threadIdx.x + i * THREADS;
+            if (x < RP * RP) sG[x] = gv[i];
+        }
+#pragma unroll
+        for (int i = 0; i < PO; i++) {
+            const int x = threadIdx.x + i * THREADS;
+            if (x < EL) sOld[(x / RP) * LD + x % RP] = ov[i];
+        }
+        if (stopped) return;
         __syncthreads();
         if (w_update_by_column(e.method)) {
             for (int x = threadIdx.x; x < EL; x += THREADS) {
@@ -1704,7 +1762,10 @@ __global__ void __launch_bounds__(THREADS)
             ga.add4(g.want, [&](int k, int q) { return sNew[(4 * warp + q) * LD + k]; });
     } else {
         double *sRow = tile + warp * 32 * LD;  // this warp's 32 rows
-        __syncthreads();                       // sG
+        if (e.G != nullptr)
+            for (int x = threadIdx.x; x < RP * RP; x += THREADS) sG[x] = e.G[x];
+        __syncthreads();
+        if (stopped) return;
         const int tiles = (n + 31) / 32;
         for (int t = blockIdx.x * WARPS + warp; t < tiles; t += gridDim.x * WARPS) {
             const int i0 = t * 32, i = i0 + lane;
@@ -1802,10 +1863,10 @@ void launch_gram_w(const double *W, int n, const GramOut &g, GramPlan gp, const 
     };
     if (gp.few)
         go(gram_w_tiles<RP, kEpiThreads>, kEpiThreads,
-           sizeof(double) * GramAcc<RP, kEpiThreads>::SCRATCH);
+           sizeof(double) * GramAcc<RP, kEpiThreads, kTileRows / 4>::SCRATCH);
     else
         go(gram_w_tiles<RP, kWideThreads>, kWideThreads,
-           sizeof(double) * GramAcc<RP, kWideThreads>::SCRATCH);
+           sizeof(double) * GramAcc<RP, kWideThreads, kWideThreads / 32>::SCRATCH);
 }
 template <int RP>
 void launch_gram_h(const double *H, int p, const GramOut &g, GramPlan gp, const RunState *st,
@@ -1816,10 +1877,10 @@ void launch_gram_h(const double *H, int p, const GramOut &g, GramPlan gp, const 
     };
     if (gp.few)
         go(gram_h_tiles<RP, kEpiThreads>, kEpiThreads,
-           sizeof(double) * GramAcc<RP, kEpiThreads>::SCRATCH);
+           sizeof(double) * GramAcc<RP, kEpiThreads, kTileCols / 4>::SCRATCH);
     else
         go(gram_h_tiles<RP, kWideThreads>, kWideThreads,
-           sizeof(double) * GramAcc<RP, kWideThreads>::SCRATCH);
+           sizeof(double) * GramAcc<RP, kWideThreads, kWideThreads / 32>::SCRATCH);
 }
 
 // f32 copy of W (n x RP f64 -> n x RPS f32, zero pad) for the f32 H pass.
