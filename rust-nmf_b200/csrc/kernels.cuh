@@ -88,239 +88,6 @@ __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, 
 __device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, b); }
 
 // ---------------------------------------------------------------------------
-// H-step contraction: reduce over rows [u0, u1) for 32 columns per CTA.
-// grid (ceil(p/32), S), block (32, 8).  part is [S][RP][p] f64.
-// ---------------------------------------------------------------------------
-template <typename TV, typename TA, int RP, bool RATIO>
-__global__ void __launch_bounds__(kThreads)
-    hstep_contract(const TV *__restrict__ V, int64_t ldv, int n, int p,
-                   const double *__restrict__ W, const double *__restrict__ H,
-                   int rows_per_split, double *__restrict__ part, const RunState *st) {
-    if (run_stopped(st)) return;
-    // Rows of W staged per chunk; in f32 the per-chunk f32 sums are flushed
-    // into f64 accumulators once per chunk.
-    constexpr int CH = (sizeof(TA) == 8) ? 64 : 256;
-    constexpr int SBUF = (CH * RP * (int)sizeof(TA) > 4 * RP * 32 * 8)
-                             ? CH * RP
-                             : (4 * RP * 32 * 8) / (int)sizeof(TA);
-    __shared__ __align__(16) TA sbuf[SBUF];
-
-    const int lane = threadIdx.x;
-    const int warp = threadIdx.y;
-    const int tid = warp * 32 + lane;
-    const int j = blockIdx.x * 32 + lane;
-    const bool colok = j < p;
-    const int u0 = blockIdx.y * rows_per_split;
-    const int u1 = min(n, u0 + rows_per_split);
-
-    double acc[RP];
-#pragma unroll
-    for (int k = 0; k < RP; k++) acc[k] = 0.0;
-    TA hcol[RATIO ? RP : 1];
-    if constexpr (RATIO) {
-#pragma unroll
-        for (int k = 0; k < RP; k++) hcol[k] = colok ? (TA)H[(int64_t)k * p + j] : (TA)0;
-    }
-
-    // f64: accf is the accumulator.  f32: accf holds one chunk's sums and is
-    // flushed into the f64 acc after every chunk.
-    TA accf[RP];
-#pragma unroll
-    for (int k = 0; k < RP; k++) accf[k] = (TA)0;
-
-    for (int base = u0; base < u1; base += CH) {
-        const int rows = min(CH, u1 - base);
-        __syncthreads();
-        const double *wsrc = W + (int64_t)base * RP;
-        for (int t = tid; t < CH * RP; t += kThreads)
-            sbuf[t] = (t < rows * RP) ? (TA)wsrc[t] : (TA)0;
-        __syncthreads();
-
-        // Each warp takes rows warp, warp + 8, ...; 4 rows per step so four
-        // independent V loads are in flight before the arithmetic.
-        for (int rr = warp; rr < rows; rr += 4 * kWarps) {
-            TA v[4];
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int row = rr + q * kWarps;
-                v[q] = (colok && row < rows) ? (TA)V[(int64_t)(base + row) * ldv + j] : (TA)0;
-            }
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int row = rr + q * kWarps;
-                if (row < rows) {
-                    const TA *wr = sbuf + row * RP;
-                    if constexpr (RATIO) {
-                        TA wh = (TA)0;
-#pragma unroll
-                        for (int k = 0; k < RP; k++) wh = fma(wr[k], hcol[k], wh);
-                        const TA qv = (wh != (TA)0) ? ratio_div(v[q], wh) : (TA)0;
-#pragma unroll
-                        for (int k = 0; k < RP; k++) accf[k] = fma(wr[k], qv, accf[k]);
-                    } else {
-#pragma unroll
-                        for (int k = 0; k < RP; k++) accf[k] = fma(wr[k], v[q], accf[k]);
-                    }
-                }
-            }
-        }
-        if constexpr (sizeof(TA) == 4) {
-#pragma unroll
-            for (int k = 0; k < RP; k++) {
-                acc[k] += (double)accf[k];
-                accf[k] = (TA)0;
-            }
-        }
-    }
-    if constexpr (sizeof(TA) == 8) {
-#pragma unroll
-        for (int k = 0; k < RP; k++) acc[k] = (double)accf[k];
-    }
-
-    // CTA reduction over the 8 warps in a fixed tree order (deterministic).
-    // sbuf holds CH * RP >= 4 * 32 * RP * 8 / sizeof(TA) elements, enough for
-    // 4 * 32 * RP doubles in both precisions.
-    double *red = reinterpret_cast<double *>(sbuf);
-#pragma unroll
-    for (int level = 4; level >= 1; level >>= 1) {
-        __syncthreads();
-        if (warp >= level && warp < 2 * level) {
-#pragma unroll
-            for (int k = 0; k < RP; k++) red[((warp - level) * RP + k) * 32 + lane] = acc[k];
-        }
-        __syncthreads();
-        if (warp < level) {
-#pragma unroll
-            for (int k = 0; k < RP; k++) acc[k] += red[(warp * RP + k) * 32 + lane];
-        }
-    }
-    if (warp == 0 && colok) {
-        double *dst = part + (int64_t)blockIdx.y * RP * p + j;
-#pragma unroll
-        for (int k = 0; k < RP; k++) dst[(int64_t)k * p] = acc[k];
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Row-owned V pass: one thread per row of V, V tiles staged through shared
-// memory so that a warp's global loads are row-contiguous.
-//   MODE 0 (plain)  : part[i][k] += V[i][j] H[k][j]
-//   MODE 1 (ratio)  : part[i][k] += H[k][j] V[i][j] / (W H)[i][j]
-//   MODE 2 (KL)     : obj += kl term of (V, W H)   (lib.rs:1418-1427)
-//   MODE 3 (Frob)   : obj += (V - W H)^2           (lib.rs:1440-1441)
-// grid (ceil(n/256), S2), block 256.  part is [S2][n][RP] (modes 0, 1);
-// obj is one f64 per CTA (modes 2, 3), indexed blockIdx.y * gridDim.x + x.
-// ---------------------------------------------------------------------------
-template <typename TV, typename TA, int RP, int MODE>
-__global__ void __launch_bounds__(kThreads)
-    rowpass(const TV *__restrict__ V, int64_t ldv, int n, int p, const double *__restrict__ W,
-            const double *__restrict__ H, int cols_per_split, double *__restrict__ part,
-            double *__restrict__ obj, const RunState *st, const double *__restrict__ roff = nullptr) {
-    if (run_stopped(st)) return;
-    constexpr int TC = (sizeof(TV) == 8) ? 16 : 32;  // 128 B of a V row per tile
-    __shared__ TV sV[kThreads][TC + 1];
-    __shared__ __align__(16) TA sH[TC][RP];
-
-    const int tid = threadIdx.x;
-    const int row0 = blockIdx.x * kThreads;
-    const int i = row0 + tid;
-    const bool rowok = i < n;
-    const int c0 = blockIdx.y * cols_per_split;
-    const int c1 = min(p, c0 + cols_per_split);
-
-    constexpr bool NEED_W = (MODE != 0);
-    TA wrow[NEED_W ? RP : 1];
-    if constexpr (NEED_W) {
-#pragma unroll
-        for (int k = 0; k < RP; k++) wrow[k] = rowok ? (TA)W[(int64_t)i * RP + k] : (TA)0;
-    }
-    double acc[MODE <= 1 ? RP : 1];
-#pragma unroll
-    for (int k = 0; k < (MODE <= 1 ? RP : 1); k++) acc[k] = 0.0;
-    double objacc = 0.0;
-    // offset method: the row's offset is part of the estimate (lib.rs:1746-1752)
-    const double ro = (MODE == 3 && roff != nullptr && rowok) ? roff[i] : 0.0;
-
-    constexpr int NA = (MODE <= 1) ? RP : 1;
-    TA accf[NA];  // f64: the accumulator; f32: one tile's sums
-#pragma unroll
-    for (int k = 0; k < NA; k++) accf[k] = (TA)0;
-
-    for (int c = c0; c < c1; c += TC) {
-        __syncthreads();
-        for (int e = tid; e < kThreads * TC; e += kThreads) {
-            const int rr = e / TC, cc = e - rr * TC;
-            const int gi = row0 + rr, gc = c + cc;
-            sV[rr][cc] = (gi < n && gc < c1) ? V[(int64_t)gi * ldv + gc] : (TV)0;
-        }
-        for (int e = tid; e < TC * RP; e += kThreads) {
-            const int k = e / TC, cc = e - k * TC;
-            const int gc = c + cc;
-            sH[cc][k] = (gc < c1) ? (TA)H[(int64_t)k * p + gc] : (TA)0;
-        }
-        __syncthreads();
-        const int ncols = min(TC, c1 - c);
-#pragma unroll 4
-        for (int cc = 0; cc < ncols; cc++) {
-            const TA v = (TA)sV[tid][cc];
-            const TA *hr = sH[cc];
-            if constexpr (MODE == 0) {
-#pragma unroll
-                for (int k = 0; k < RP; k++) accf[k] = fma(v, hr[k], accf[k]);
-            } else {
-                TA wh = (TA)0;
-#pragma unroll
-                for (int k = 0; k < RP; k++) wh = fma(wrow[k], hr[k], wh);
-                if constexpr (MODE == 1) {
-                    const TA q = (wh != (TA)0) ? ratio_div(v, wh) : (TA)0;
-#pragma unroll
-                    for (int k = 0; k < RP; k++) accf[k] = fma(hr[k], q, accf[k]);
-                } else if constexpr (MODE == 2) {
-                    const double vv = (double)v, ww = (double)wh;
-                    if (vv > 0.0) {
-                        if (ww > 0.0) objacc += vv * log(vv / ww) - vv + ww;
-                    } else {
-                        objacc += ww;
-                    }
-                } else {
-                    const double d = (double)v - ((double)wh + ro);
-                    objacc += d * d;
-                }
-            }
-        }
-        if constexpr (MODE <= 1 && sizeof(TA) == 4) {
-#pragma unroll
-            for (int k = 0; k < RP; k++) {
-                acc[k] += (double)accf[k];
-                accf[k] = (TA)0;
-            }
-        }
-    }
-
-    if constexpr (MODE <= 1) {
-        if constexpr (sizeof(TA) == 8) {
-#pragma unroll
-            for (int k = 0; k < RP; k++) acc[k] = (double)accf[k];
-        }
-        if (rowok) {
-            double *dst = part + ((int64_t)blockIdx.y * n + i) * RP;
-#pragma unroll
-            for (int k = 0; k < RP; k++) dst[k] = acc[k];
-        }
-    } else {
-        // Block reduction of the objective in a fixed order.
-        __shared__ double red[kThreads];
-        red[tid] = rowok ? objacc : 0.0;
-        __syncthreads();
-        for (int s = kThreads / 2; s > 0; s >>= 1) {
-            if (tid < s) red[tid] += red[tid + s];
-            __syncthreads();
-        }
-        if (tid == 0) obj[(int64_t)blockIdx.y * gridDim.x + blockIdx.x] = red[0];
-    }
-}
-
-// ---------------------------------------------------------------------------
 // nsNMF and offset helpers
 // ---------------------------------------------------------------------------
 // Smoothing matrix entry S[k][j] = (1 - theta) I + (theta / r) (lib.rs:458-466).

@@ -42,6 +42,13 @@ struct StreamOps {
                                        const double *W, int n, int p, const StreamK &sk,
                                        double *part, RunState *st, int grid,
                                        cudaStream_t s) const = 0;
+    // Objective terms of the f64 V, one partial a CTA (sk.G of them), on the
+    // ratio passes' H split (the map of V with their H box): KL, or squared
+    // residuals with row offsets roff (or null).  f64 only.
+    virtual cudaError_t objective(bool kl, const CUtensorMap &tmV, const CUtensorMap &tmW,
+                                  const double *H, int n, int p, const StreamK &sk,
+                                  const double *roff, double *part, RunState *st,
+                                  cudaStream_t s) const = 0;
     // The updates, with the new factor's Gram and sums as `g` asks.
     virtual void h_epi(double *H, void *Ht, int p, const double *part, const StreamK &sk,
                        int tcols, const EpiParams &e, const GramOut &g, GramPlan gp,

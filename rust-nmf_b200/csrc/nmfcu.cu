@@ -94,16 +94,9 @@ inline unsigned grid_for(int64_t total) {
 }
 inline int64_t round_up(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
 
-// Grams, rescaling, clamps and the objective pass: O(r^2 (n + p)) work plus
-// the objective's one read of V.
+// Grams, rescaling, clamps and the like: O(r^2 (n + p)) work.
 struct Ops {
     virtual ~Ops() = default;
-    // mode 2 KL objective, 3 Frobenius objective (f64 V); roff: row offsets
-    // added to W H (offset method) or nullptr
-    virtual void objective(const double *V, int64_t ldv, int n, int p, const double *W,
-                           const double *H, int mode, int S2, int cols_per_split, double *obj,
-                           const RunState *st, cudaStream_t s,
-                           const double *roff = nullptr) const = 0;
     // W update from a dense (summed) contraction num (n x RP)
     virtual void w_apply(double *W, int n, const double *num, const EpiParams &e,
                          const RunState *st, cudaStream_t s) const = 0;
@@ -137,18 +130,6 @@ struct Ops {
 
 template <int RP>
 struct OpsT final : Ops {
-    void objective(const double *V, int64_t ldv, int n, int p, const double *W, const double *H,
-                   int mode, int S2, int cols_per_split, double *obj, const RunState *st,
-                   cudaStream_t s, const double *roff) const override {
-        if (n <= 0 || S2 <= 0) return;
-        dim3 grid(cdiv(n, kThreads), S2), block(kThreads);
-        if (mode == 2)
-            nmfcu::rowpass<double, double, RP, 2><<<grid, block, 0, s>>>(
-                V, ldv, n, p, W, H, cols_per_split, nullptr, obj, st);
-        else
-            nmfcu::rowpass<double, double, RP, 3><<<grid, block, 0, s>>>(
-                V, ldv, n, p, W, H, cols_per_split, nullptr, obj, st, roff);
-    }
     void w_apply(double *W, int n, const double *num, const EpiParams &e, const RunState *st,
                  cudaStream_t s) const override {
         if (n > 0) nmfcu::w_apply_dense<RP><<<cdiv(n, kThreads), kThreads, 0, s>>>(W, n, num, e, st);
@@ -334,9 +315,8 @@ struct DevBuf {
 // Launch geometry of the small kernels of one problem shape.
 struct Plan {
     int n = 0, p = 0, r = 0, RP = 0;
-    int S2 = 1, cols_per_split = 1;    // objective pass column splits
     GramPlan gw{true, 1}, gh{true, 1}; // the W / H epilogues and Grams
-    int obj_blocks = 0;                // objective partial count
+    int obj_blocks = 0;                // lsNMF: objective partial count
 };
 
 Plan make_plan(int64_t n, int64_t p, int64_t r, int sms) {
@@ -350,9 +330,8 @@ Plan make_plan(int64_t n, int64_t p, int64_t r, int sms) {
     int64_t S2 = std::max<int64_t>(1, (target + rb - 1) / rb);
     S2 = std::min<int64_t>(S2, std::max<int64_t>(1, p / 256));
     int64_t cps = std::max<int64_t>(32, ((p + S2 - 1) / S2 + 31) / 32 * 32);
-    pl.cols_per_split = (int)cps;
-    pl.S2 = (int)std::max<int64_t>(1, (p + cps - 1) / cps);
-    pl.obj_blocks = (int)(((n + kThreads - 1) / kThreads) * pl.S2);
+    pl.obj_blocks =
+        (int)(((n + kThreads - 1) / kThreads) * std::max<int64_t>(1, (p + cps - 1) / cps));
     pl.gw = gram_plan(n, kTileRows, sms);
     pl.gh = gram_plan(p, kTileCols, sms);
     return pl;
@@ -511,6 +490,7 @@ struct PassSet {
     const StreamOps *so = nullptr;
     bool f32 = false;
     CUtensorMap tmVh, tmVw, tmW, tmHt;
+    CUtensorMap tmVo;  // f64: V in the objective's box (the ratio H pass's)
     void *Ht = nullptr;  // H^T, written by the H epilogue, streamed by the W pass
     void *Wc = nullptr;  // f32 copy of W (f32 only; f64 streams the master W)
     // Split-bf16 form (tensor-core passes): V hi/lo maps for the H pass (box
@@ -604,6 +584,9 @@ nmfcu_status make_passset(nmfcu_context *c, const Plan &pl, bool f32, bool ratio
                                                 : CU_TENSOR_MAP_SWIZZLE_128B;
     NMF_TRY(encode_2d(&ps->tmVh, V, f32, pl.n, pl.p, ldv, ps->so->h_boxc(ratio),
                       ps->so->h_brows(ratio)));
+    if (!f32)
+        NMF_TRY(encode_2d(&ps->tmVo, V, false, pl.n, pl.p, ldv, ps->so->h_boxc(true),
+                          ps->so->h_brows(true)));
     NMF_TRY(encode_2d(&ps->tmVw, V, f32, pl.n, pl.p, ldv, ps->so->w_bcols(ratio),
                       ps->so->w_boxr(ratio), wsw));
     if (f32)
@@ -721,27 +704,33 @@ struct RunArgs {
     double *Wout = nullptr;  // w_step's epilogue target when not W (column shards)
 };
 
-// The objective's per-block partials over this V (c->obj, pl.obj_blocks).
-nmfcu_status enqueue_objective_partials(nmfcu_context *c, const RunArgs &a, cudaStream_t s) {
+// The objective's per-block partials over this V into c->obj, *count of them.
+nmfcu_status enqueue_objective_partials(nmfcu_context *c, const RunArgs &a, cudaStream_t s,
+                                        int *count) {
     const Plan &pl = a.pl;
     RunState *st = c->state.as<RunState>();
     const bool kl = (a.opt->method == NMFCU_BRUNET || a.opt->method == NMFCU_NSNMF);
-    const double *West = a.W;
+    *count = 0;
     if (a.opt->method == NMFCU_NSNMF) {  // KL of V against (W S) H, lib.rs:1779-1783
+        // (p64's W map is of W S)
         nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER);
         a.ops->ns_right(a.W, pl.n, pl.r, a.opt->theta, a.Wns, st, s);
-        West = a.Wns;
     }
+    nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OBJECTIVE);
     if (a.opt->method == NMFCU_LSNMF) {  // 0.5 ||(V - W H) o S||^2, lib.rs:1024-1035
-        nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OBJECTIVE);
-        a.ops->ls_objective(a.V64, a.S64, a.ldv64, pl.n, pl.p, a.W, a.H,
-                            pl.n > 0 ? pl.obj_blocks : 0, c->obj.as<double>(), st, s);
-    } else {
-        nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OBJECTIVE);
-        a.ops->objective(a.V64, a.ldv64, pl.n, pl.p, West, a.H, kl ? 2 : 3, pl.S2,
-                         pl.cols_per_split, c->obj.as<double>(), st, s,
-                         a.opt->method == NMFCU_OFFSET ? a.off : nullptr);
+        if (pl.n <= 0) return NMFCU_OK;
+        *count = pl.obj_blocks;
+        a.ops->ls_objective(a.V64, a.S64, a.ldv64, pl.n, pl.p, a.W, a.H, pl.obj_blocks,
+                            c->obj.as<double>(), st, s);
+        return NMFCU_OK;
     }
+    const StreamOps *so = a.p64.so;
+    const StreamK sk = plan_h(so, true, pl.n, pl.p, c->sms);
+    *count = sk.G;
+    if (sk.G > 0)
+        CUDA_TRY(so->objective(kl, a.p64.tmVo, a.p64.tmW, a.H, pl.n, pl.p, sk,
+                               a.opt->method == NMFCU_OFFSET ? a.off : nullptr,
+                               c->obj.as<double>(), st, s));
     return NMFCU_OK;
 }
 
@@ -759,10 +748,10 @@ StopParams stop_params(const nmfcu_options *o, long long iter) {
 // Objective of iteration `iter` into the deviances and the stationary stop.
 nmfcu_status enqueue_objective(nmfcu_context *c, const RunArgs &a, long long iter,
                                cudaStream_t s) {
-    NMF_TRY(enqueue_objective_partials(c, a, s));
+    int count = 0;
+    NMF_TRY(enqueue_objective_partials(c, a, s, &count));
     nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER);
-    objective_finalize<<<1, kThreads, 0, s>>>(c->obj.as<double>(),
-                                              a.pl.n > 0 ? a.pl.obj_blocks : 0, a.dev,
+    objective_finalize<<<1, kThreads, 0, s>>>(c->obj.as<double>(), count, a.dev,
                                               stop_params(a.opt, iter), c->state.as<RunState>());
     return NMFCU_OK;
 }
@@ -1144,7 +1133,7 @@ std::vector<WsNeed> workspace_needs(nmfcu_context *c, const Plan &pl, bool need_
     v.push_back({&c->sw, sizeof(double) * RP});
     v.push_back({&c->sh, sizeof(double) * RP});
     v.push_back({&c->sw2, sizeof(double) * RP});
-    v.push_back({&c->obj, sizeof(double) * (size_t)std::max(pl.obj_blocks, 1)});
+    v.push_back({&c->obj, sizeof(double) * (size_t)std::max(pl.obj_blocks, c->sms)});
     v.push_back({&c->state, sizeof(RunState)});
     if (method == NMFCU_NSNMF) {
         v.push_back({&c->Wns, sizeof(double) * (size_t)pl.n * RP});
@@ -1374,11 +1363,11 @@ nmfcu_status run_snmf(nmfcu_context *c, RunArgs &a, cudaStream_t s, double *dev)
             NMF_TRY(solve_h(sb * sb, 0.0));
             NMF_TRY(solve_w(0.0, eta_eff * eta_eff));
         }
-        NMF_TRY(enqueue_objective_partials(c, a, s));
+        int count = 0;
+        NMF_TRY(enqueue_objective_partials(c, a, s, &count));
         sp.iter = it;
         nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER);
-        objective_finalize<<<1, kThreads, 0, s>>>(c->obj.as<double>(),
-                                                  pl.n > 0 ? pl.obj_blocks : 0, dev, sp, st);
+        objective_finalize<<<1, kThreads, 0, s>>>(c->obj.as<double>(), count, dev, sp, st);
     }
     return finish_checked(c, s);
 }
@@ -1692,16 +1681,21 @@ nmfcu_status objective_host(bool kl, int64_t n, int64_t p, int64_t r, const doub
     NMF_TRY(upload_v(c, V, n, p, &ldv, s));
     NMF_TRY(put_factors(c, pl, W, H, cudaMemcpyHostToDevice, s));
     CUDA_TRY(cudaMemsetAsync(c->state.ptr, 0, sizeof(RunState), s));
-    const Ops *ops = ops_for(pl.RP);
-    RunState *st = c->state.as<RunState>();
-    ops->objective(c->V64.as<double>(), ldv, pl.n, pl.p, c->W.as<double>(), c->H.as<double>(),
-                   kl ? 2 : 3, pl.S2, pl.cols_per_split, c->obj.as<double>(), st, s);
+    RunArgs a;
+    a.opt = &o;
+    a.pl = pl;
+    a.ops = ops_for(pl.RP);
+    NMF_TRY(make_passset(c, pl, false, true, c->V64.ptr, ldv, &a.p64));
+    a.W = c->W.as<double>();
+    a.H = c->H.as<double>();
+    int count = 0;
+    NMF_TRY(enqueue_objective_partials(c, a, s, &count));
     StopParams sp{};
     sp.stationary = 0;
     sp.iter = 0;
     sp.scale = kl ? 1.0 : 0.5;
-    objective_finalize<<<1, kThreads, 0, s>>>(c->obj.as<double>(), pl.n > 0 ? pl.obj_blocks : 0,
-                                              c->dev.as<double>(), sp, st);
+    objective_finalize<<<1, kThreads, 0, s>>>(c->obj.as<double>(), count, c->dev.as<double>(), sp,
+                                              c->state.as<RunState>());
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaMemcpyAsync(out, c->dev.ptr, sizeof(double), cudaMemcpyDeviceToHost, s));
     CUDA_TRY(cudaStreamSynchronize(s));
@@ -2455,10 +2449,10 @@ nmfcu_status nmfcu_shard_step(nmfcu_shard *sh, int32_t phase, void *stream) {
         case NMFCU_SHARD_OBJECTIVE: {
             if (o->stop != NMFCU_STOP_STATIONARY)
                 return fail(NMFCU_ERR_INVALID_ARG, "the objective runs with stop stationary");
-            NMF_TRY(enqueue_objective_partials(c, a, s));
+            int count = 0;
+            NMF_TRY(enqueue_objective_partials(c, a, s, &count));
             nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER);
-            sum_partials<<<1, kThreads, 0, s>>>(c->obj.as<double>(),
-                                                pl.n > 0 ? pl.obj_blocks : 0, sh->Robj);
+            sum_partials<<<1, kThreads, 0, s>>>(c->obj.as<double>(), count, sh->Robj);
             break;
         }
         case NMFCU_SHARD_STOP: {

@@ -1433,6 +1433,194 @@ __global__ void __launch_bounds__(DWRCfg<RP>::kWarps * 32, 1)
 }
 
 // ---------------------------------------------------------------------------
+// FP64 objective on the FP64 tensor cores
+// ---------------------------------------------------------------------------
+// The H ratio pass's tiling and its first MMA chain (W H of 8 x 8 tiles in
+// registers), each element then a term of
+//   KL         v ln(v / wh) - v + wh for v > 0 and wh > 0, wh for v = 0
+//              (kl_divergence lib.rs:1418-1427)
+//   Frobenius  (v - (wh + roff_i))^2   (lib.rs:1440-1441; offset :1746-1752)
+// summed per thread, then over the block in a fixed tree: part[b].
+// Bound: FP64 (KL: W H, a reciprocal and a logarithm an element).  2000 x 7750
+// rank 10, KL: 183 us with one thread a row on the CUDA cores, 99 here with
+// the library's log(), 77 with log_table.
+
+// ln x by a table (Tang, "Table-driven implementation of the logarithm
+// function in IEEE floating-point arithmetic", 1990): x = 2^k m, m in [1, 2),
+// c the middle of m's 1/128 (its seven leading fraction bits), r = m / c - 1,
+//   ln x = k ln 2 + ln c + (r - r^2/2 + ... - r^6/6),  |r| <= 1/256,
+// the term left out below 3e-18.  Above sqrt 2 the table holds ln c - ln 2 and
+// k goes up by one, so that nothing cancels near x = 1.  The error is that of
+// the final additions.  Ten FP64 operations and one 16-byte load.
+constexpr int kLogEntries = 128;
+__device__ __forceinline__ void log_table_init(double2 *t) {
+    const int j = threadIdx.x;
+    if (j < kLogEntries) {
+        const double ic = 1.0 / (1.0 + (j + 0.5) / kLogEntries);
+        t[j] = make_double2(ic, -log(2 * j >= kLogEntries - 22 ? 2.0 * ic : ic));
+    }
+}
+__device__ __forceinline__ double log_table(double x, const double2 *t) {
+    const unsigned hi = (unsigned)__double2hiint(x);
+    const int be = (int)(hi >> 20);
+    if (be == 0 || be >= 0x7ff) return log(x);  // subnormal, infinite, NaN, negative
+    const int j = (int)((hi >> 13) & (kLogEntries - 1));
+    const double m = __hiloint2double((int)((hi & 0xfffffu) | 0x3ff00000u), __double2loint(x));
+    const double2 c = t[j];
+    const double k = (double)(be - 1023 + (2 * j >= kLogEntries - 22 ? 1 : 0));
+    const double r = fma(m, c.x, -1.0);
+    double q = fma(r, -1.0 / 6.0, 1.0 / 5.0);
+    q = fma(r, q, -1.0 / 4.0);
+    q = fma(r, q, 1.0 / 3.0);
+    q = fma(r, q, -1.0 / 2.0);
+    return fma(k, 0.693147180559945309417, c.y) + fma(r * r, q, r);
+}
+template <int RP, bool KL>
+__global__ void __launch_bounds__(DHRCfg<RP>::kWarps * 32, 1)
+    objective_dmma(const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmW,
+                   const double *__restrict__ H, int n, int p, StreamK sk,
+                   const double *__restrict__ roff, double *__restrict__ part, RunState *st) {
+    using C = DHRCfg<RP>;
+    if (run_stopped(st)) return;
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem + C::STAGES * C::STAGE);
+    int *arrivals = reinterpret_cast<int *>(full + C::STAGES);
+    __shared__ double red[C::kWarps];
+    __shared__ double2 logs[KL ? kLogEntries : 1];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool producer = (threadIdx.x == 0);
+    const int b = blockIdx.x;
+    const long long u0 = sk.start(b), u1 = sk.start(b + 1);
+    const long long nunits = u1 - u0;
+
+    auto issue = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
+        const int rb = c.along(sk);
+        tma_load_2d(stg, &tmV, bar, c.major * C::TCOLS, rb * C::BROWS);
+        tma_load_2d(stg + C::VBYTES, &tmW, bar, 0, rb * C::BROWS);
+    };
+    UnitCursor ahead;
+    ahead.init(sk, u0);
+    if (producer) {
+        for (int s = 0; s < C::STAGES; s++) {
+            mbar_init(&full[s], 1);
+            arrivals[s] = 0;
+        }
+        fence_mbar_init();
+        for (int j = 0; j < C::STAGES; j++) {
+            if (j < nunits) {
+                mbar_expect_tx(&full[j], C::VBYTES + C::WBYTES);
+                issue(smem + j * C::STAGE, &full[j], ahead);
+            }
+            ahead.next(sk);
+        }
+    } else {
+        for (int j = 0; j < C::STAGES; j++) ahead.next(sk);
+    }
+    if (KL) log_table_init(logs);
+    __syncthreads();
+
+    const int g = lane >> 2, q4 = lane & 3;
+    const int wc0 = warp * C::WCOLS;
+    double hreg[C::NT][C::KST];  // H[ks * 4 + q4][column of row g]
+    bool in[C::NT];              // the thread's columns are V's
+    double sum[C::NT];
+    int cur_major = -1;
+#pragma unroll
+    for (int nt = 0; nt < C::NT; nt++) {
+        sum[nt] = 0.0;
+        in[nt] = false;
+    }
+    UnitCursor uc;
+    uc.init(sk, u0);
+    int s = 0, rnd = 0;
+    for (long long i = 0; i < nunits; ++i) {
+        if (uc.major != cur_major) {
+            cur_major = uc.major;
+#pragma unroll
+            for (int nt = 0; nt < C::NT; nt++) {
+                const int j = uc.major * C::TCOLS + wc0 + nt * 8 + g;
+                in[nt] = j < p;
+#pragma unroll
+                for (int ks = 0; ks < C::KST; ks++) {
+                    const int k = ks * 4 + q4;
+                    hreg[nt][ks] = (k < RP && j < p) ? H[(size_t)k * p + j] : 0.0;
+                }
+            }
+        }
+        if (!mbar_wait(&full[s], (uint32_t)(rnd & 1))) {
+            record_timeout(st, TIMEOUT_FULL);
+            break;
+        }
+        const unsigned char *stg = smem + s * C::STAGE;
+        const double *sv = reinterpret_cast<const double *>(stg) + wc0 + g;
+        const double *sw = reinterpret_cast<const double *>(stg + C::VBYTES);
+#pragma unroll 1
+        for (int r0 = 0; r0 < C::BROWS; r0 += 8) {
+            double b1[C::KST];  // W[r0 + g][ks * 4 + q4]
+#pragma unroll
+            for (int ks = 0; ks < C::KST; ks++) {
+                const int k = ks * 4 + q4;
+                b1[ks] = (k < RP) ? sw[(r0 + g) * C::RPS + k] : 0.0;
+            }
+            double wh[C::NT][2];
+#pragma unroll
+            for (int nt = 0; nt < C::NT; nt++) wh[nt][0] = wh[nt][1] = 0.0;
+#pragma unroll
+            for (int ks = 0; ks < C::KST; ks++)
+#pragma unroll
+                for (int nt = 0; nt < C::NT; nt++) dmma_8x8x4(wh[nt], hreg[nt][ks], b1[ks]);
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const int row = r0 + 2 * q4 + e;
+                double ro = 0.0;
+                if (!KL && roff != nullptr) {
+                    const int ri = uc.along(sk) * C::BROWS + row;
+                    ro = ri < n ? roff[ri] : 0.0;
+                }
+#pragma unroll
+                for (int nt = 0; nt < C::NT; nt++) {
+                    // Past V's edge v and wh are 0: no term but roff's.
+                    const double v = sv[row * C::BOXC + nt * 8], w = wh[nt][e];
+                    if (KL) {
+                        if (v > 0.0) {
+                            if (w > 0.0) sum[nt] += v * log_table(ratio_div(v, w), logs) - v + w;
+                        } else {
+                            sum[nt] += w;
+                        }
+                    } else {
+                        const double d = v - (w + ro);
+                        sum[nt] += in[nt] ? d * d : 0.0;
+                    }
+                }
+            }
+        }
+        __syncwarp();
+        if (lane == 0)
+            release_stage<C::STAGE, C::VBYTES + C::WBYTES>(smem, full, arrivals, s, C::kWarps,
+                                                           i + C::STAGES < nunits, ahead, issue);
+        ahead.next(sk);
+        if (++s == C::STAGES) {
+            s = 0;
+            ++rnd;
+        }
+        uc.next(sk);
+    }
+    double a = 0.0;
+#pragma unroll
+    for (int nt = 0; nt < C::NT; nt++) a += sum[nt];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if (lane == 0) red[warp] = a;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int w = 0; w < C::kWarps; w++) t += red[w];
+        part[b] = t;
+    }
+}
+
+// ---------------------------------------------------------------------------
 // Epilogues for the stream-K partials
 // ---------------------------------------------------------------------------
 

@@ -165,6 +165,28 @@ struct StreamOpsT final : StreamOps {
         else
             return cudaErrorNotSupported;
     }
+    template <bool KL>
+    static cudaError_t launch_objective(const CUtensorMap &tmV, const CUtensorMap &tmW,
+                                        const double *H, int n, int p, const StreamK &sk,
+                                        const double *roff, double *part, RunState *st,
+                                        cudaStream_t s) {
+        using C = DHRCfg<RP>;
+        auto *kern = nmfcu::objective_dmma<RP, KL>;
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             C::SMEM);
+        if (e != cudaSuccess) return e;
+        kern<<<sk.G, 32 * C::kWarps, C::SMEM, s>>>(tmV, tmW, H, n, p, sk, roff, part, st);
+        return cudaGetLastError();
+    }
+    cudaError_t objective(bool kl, const CUtensorMap &tmV, const CUtensorMap &tmW, const double *H,
+                          int n, int p, const StreamK &sk, const double *roff, double *part,
+                          RunState *st, cudaStream_t s) const override {
+        if constexpr (kDmma)
+            return kl ? launch_objective<true>(tmV, tmW, H, n, p, sk, roff, part, st, s)
+                      : launch_objective<false>(tmV, tmW, H, n, p, sk, roff, part, st, s);
+        else
+            return cudaErrorNotSupported;
+    }
     void h_epi(double *H, void *Ht, int p, const double *part, const StreamK &sk, int tcols,
                const EpiParams &e, const GramOut &g, GramPlan gp, const RunState *st,
                cudaStream_t s) const override {
