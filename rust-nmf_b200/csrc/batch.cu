@@ -37,29 +37,41 @@ constexpr int kThreads = 128;      // threads per CTA
 constexpr int kRowChunk = 64;      // W rows staged per chunk (H step)
 constexpr int kPrefetch = 4;       // V rows in flight per thread (H step)
 
-// Per element type: a thread owns CPT adjacent columns (H step) or rows
-// (W step) of V, held in one "lane pack" P.  f32 packs four as two float2
-// halves (one FFMA2 updates each half), so a staged factor value times an
-// H (or W) pack is two instructions that share the value's register pair;
-// the staged factor sits in shared memory as a duplicated pair (SV), so
-// one 128-bit load brings two values for eight columns' worth of FFMA2.
-// f64 owns one column (DFMA).
+// A thread owns CPT adjacent columns (H step) or rows (W step) of V, held in
+// one "lane pack" P.  f32 packs four as two float2 halves or two as one
+// float2 (one FFMA2 updates each float2), so a staged factor value times an
+// H (or W) pack is one or two instructions that share the value's register
+// pair; the staged factor sits in shared memory as a duplicated pair (SV),
+// so one 128-bit load brings two values for every column's FFMA2.  f64 owns
+// one column (DFMA).
 struct F4 {
     float2 a, b;  // columns 0, 1 and 2, 3
+};
+template <typename T, int CPT>
+struct Pack;
+template <>
+struct Pack<float, 4> {
+    using P = F4;
+};
+template <>
+struct Pack<float, 2> {
+    using P = float2;
+};
+template <>
+struct Pack<double, 1> {
+    using P = double;
 };
 template <typename T>
 struct BTraits;
 template <>
 struct BTraits<float> {
-    using P = F4;
     using SV = float2;  // a staged value in shared memory
-    static constexpr int CPT = 4;
+    static constexpr int CPT = 4, NARROW = 2;
 };
 template <>
 struct BTraits<double> {
-    using P = double;
     using SV = double;
-    static constexpr int CPT = 1;
+    static constexpr int CPT = 1, NARROW = 1;
 };
 
 // Kernel shapes the autotuner chooses from (run_batch_t): `comp` bounds the
@@ -93,11 +105,14 @@ struct BCfg {
 constexpr int kMaxRow = 16;             // >= ROW for every (T, R, COMP)
 template <typename T>
 constexpr int kTile = kThreads * BTraits<T>::CPT;  // columns / rows per CTA
+template <typename T>
+constexpr int kNarrowTile = kThreads * BTraits<T>::NARROW;
 
 // A staged value (SV) times a pack plus a pack.
 __device__ __forceinline__ F4 pfma(float2 s, F4 b, F4 c) {
     return F4{__ffma2_rn(s, b.a, c.a), __ffma2_rn(s, b.b, c.b)};
 }
+__device__ __forceinline__ float2 pfma(float2 s, float2 b, float2 c) { return __ffma2_rn(s, b, c); }
 __device__ __forceinline__ double pfma(double a, double b, double c) { return fma(a, b, c); }
 __device__ __forceinline__ float2 sdup(float x) { return make_float2(x, x); }
 __device__ __forceinline__ double sdup(double x) { return x; }
@@ -105,10 +120,12 @@ __device__ __forceinline__ void pzero(F4 &x) {
     x.a = make_float2(0.f, 0.f);
     x.b = make_float2(0.f, 0.f);
 }
+__device__ __forceinline__ void pzero(float2 &x) { x = make_float2(0.f, 0.f); }
 __device__ __forceinline__ void pzero(double &x) { x = 0.0; }
 __device__ __forceinline__ float &plane(F4 &a, int c) {
     return c == 0 ? a.a.x : c == 1 ? a.a.y : c == 2 ? a.b.x : a.b.y;
 }
+__device__ __forceinline__ float &plane(float2 &a, int c) { return c == 0 ? a.x : a.y; }
 __device__ __forceinline__ double &plane(double &a, int) { return a; }
 
 // The brunet ratio V / (WH), 0 where WH == 0 (lib.rs:93-99).  f32 uses the
@@ -120,11 +137,12 @@ __device__ __forceinline__ float rcp1(float wh) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(wh));
     return r;
 }
+__device__ __forceinline__ float2 ratio(float2 v, float2 wh) {
+    const float2 q = __fmul2_rn(v, make_float2(rcp1(wh.x), rcp1(wh.y)));
+    return make_float2(wh.x != 0.f ? q.x : 0.f, wh.y != 0.f ? q.y : 0.f);
+}
 __device__ __forceinline__ F4 ratio(F4 v, F4 wh) {
-    const float2 qa = __fmul2_rn(v.a, make_float2(rcp1(wh.a.x), rcp1(wh.a.y)));
-    const float2 qb = __fmul2_rn(v.b, make_float2(rcp1(wh.b.x), rcp1(wh.b.y)));
-    return F4{make_float2(wh.a.x != 0.f ? qa.x : 0.f, wh.a.y != 0.f ? qa.y : 0.f),
-              make_float2(wh.b.x != 0.f ? qb.x : 0.f, wh.b.y != 0.f ? qb.y : 0.f)};
+    return F4{ratio(v.a, wh.a), ratio(v.b, wh.b)};
 }
 // f64: v * (1 / wh) with the reciprocal from the hardware approximation
 // (rcp.approx.ftz.f64) refined by two Newton-Raphson steps
@@ -176,7 +194,7 @@ struct BSmem {
 };
 
 // One unit of a step: NS solves of rank R (offsets at goff[0..NS)) on one
-// tile of kTile output columns.
+// tile of kTile (or kNarrowTile) output columns.
 struct BItem {
     int R;
     int goff;  // index of the first offset in the group-offset table
@@ -190,12 +208,11 @@ struct BItem {
 // aligned, and A must be zero in columns [cols, round_up(cols, CPT)).
 // kComponentFast: the staged factor is contiguous along components (W in
 // the H step) -- staging loads walk components; otherwise (H^T) they walk rows.
-template <typename T, int R, int COMP, bool kComponentFast>
+template <typename T, int CPT, int R, int COMP, bool kComponentFast>
 __device__ __forceinline__ void mu_item(BSmem<T> &sm, const MuArgs<T> &a,
                                         const int *__restrict__ goff, int tile) {
     using C = BCfg<T, R, COMP>;
-    using P = typename BTraits<T>::P;
-    constexpr int CPT = BTraits<T>::CPT;
+    using P = typename Pack<T, CPT>::P;
     constexpr int NS = C::NS, ROW = C::ROW;
     constexpr int SPT = (kRowChunk * ROW + kThreads - 1) / kThreads;  // staged values per thread
     static_assert(ROW <= kMaxRow && NS <= kMaxRow, "staging row too long");
@@ -203,7 +220,7 @@ __device__ __forceinline__ void mu_item(BSmem<T> &sm, const MuArgs<T> &a,
     if (threadIdx.x < NS) sm.off[threadIdx.x] = goff[threadIdx.x];
     __syncthreads();
     const int rows = a.rows, cols = a.cols;
-    const int j0 = tile * kTile<T> + threadIdx.x * CPT;
+    const int j0 = (tile * kThreads + threadIdx.x) * CPT;
     const bool colok = j0 < cols;
     P x[NS][R], acc[NS][R];
 #pragma unroll
@@ -314,20 +331,22 @@ __device__ __forceinline__ void mu_item(BSmem<T> &sm, const MuArgs<T> &a,
 // Within a bucket one launch covers every rank class: CTA b runs item b.
 constexpr int kBuckets = 3;
 constexpr int kBucketHi[kBuckets] = {8, 10, kMaxBatchRank};  // largest rank of each
+// Bucket kBuckets: every rank, two columns a thread (f32) -- a step with too
+// few warps of four columns to fill the chip.
 template <int B>
 struct BBucket {
-    static constexpr int kLo = B == 0 ? 1 : kBucketHi[B - 1] + 1;
-    static constexpr int kHi = kBucketHi[B];
+    static constexpr int kLo = B == 0 || B == kBuckets ? 1 : kBucketHi[B - 1] + 1;
+    static constexpr int kHi = B == kBuckets ? kMaxBatchRank : kBucketHi[B];
 };
 constexpr int bucket_of(int R) { return R <= kBucketHi[0] ? 0 : R <= kBucketHi[1] ? 1 : 2; }
 
 // CTAs a multiprocessor keeps resident (the register cap) for a bucket and
 // shape.  f32 carries four columns a thread, x and acc holding 8 R
 // registers of packs: ranks 1..8 keep four CTAs (128 registers), 9..10
-// three (168), 11..16 two (255).
+// three (168), 11..16 two (255).  Two columns a thread: four CTAs throughout.
 template <typename T, int B, int SHAPE>
 constexpr int min_blocks_for() {
-    if constexpr (sizeof(T) == 4) return B == 0 ? 4 : B == 1 ? 3 : 2;
+    if constexpr (sizeof(T) == 4) return B == 0 || B == kBuckets ? 4 : B == 1 ? 3 : 2;
     return BShapes<T>::min_blocks[SHAPE];
 }
 
@@ -337,26 +356,51 @@ __global__ void __launch_bounds__(kThreads, (min_blocks_for<T, B, SHAPE>()))
     __shared__ __align__(16) BSmem<T> sm;
     const BItem it = items[blockIdx.x];
     constexpr int COMP = BShapes<T>::comp[SHAPE];
+    constexpr int CPT = B == kBuckets ? BTraits<T>::NARROW : BTraits<T>::CPT;
     switch (it.R) {
 #define MU_CASE(r)                                                                     \
     case r:                                                                            \
         if constexpr (r >= BBucket<B>::kLo && r <= BBucket<B>::kHi)                    \
-            mu_item<T, r, COMP, kComponentFast>(sm, a, off + it.goff, it.tile);        \
+            mu_item<T, CPT, r, COMP, kComponentFast>(sm, a, off + it.goff, it.tile);   \
         break;
         BATCH_RANK_CASES(MU_CASE)
 #undef MU_CASE
     }
 }
 
-// Column sums of W_all (one thread per stacked column, rows in forward
-// order as lib.rs:1563-1568) and row sums of H_all (one warp per row).
+// Column sums of W_all, rows in forward order as lib.rs:1563-1568: 32 stacked
+// columns a block, whose warps bring kColRows rows at a time to shared memory
+// (the next ones in flight) and whose first warp adds them.  One thread a
+// column reading its rows itself waited for them: 77 us at 2000 x 432, this 19.
+constexpr int kColRows = 64;
 template <typename T>
-__global__ void batch_colsum(const T *__restrict__ W, int n, int ldw, int rtot, T *__restrict__ out) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= rtot) return;
+__global__ void __launch_bounds__(256)
+    batch_colsum(const T *__restrict__ W, int n, int ldw, int rtot, T *__restrict__ out) {
+    __shared__ T tile[2][kColRows][32];
+    constexpr int PER = kColRows / 8;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int c = blockIdx.x * 32 + lane;
+    T v[PER];
+    const auto fetch = [&](int u0) {
+#pragma unroll
+        for (int i = 0; i < PER; i++) {
+            const int u = u0 + warp + 8 * i;
+            v[i] = c < rtot && u < n ? W[(size_t)u * ldw + c] : (T)0;
+        }
+    };
     T s = (T)0;
-    for (int u = 0; u < n; u++) s += W[(size_t)u * ldw + c];
-    out[c] = s;
+    int buf = 0;
+    fetch(0);
+    for (int u0 = 0; u0 < n; u0 += kColRows, buf ^= 1) {
+#pragma unroll
+        for (int i = 0; i < PER; i++) tile[buf][warp + 8 * i][lane] = v[i];
+        __syncthreads();
+        fetch(u0 + kColRows);
+        if (warp == 0)  // rows past n are zero
+#pragma unroll 16
+            for (int u = 0; u < kColRows; u++) s += tile[buf][u][lane];
+    }
+    if (warp == 0 && c < rtot) out[c] = s;
 }
 template <typename T>
 __global__ void batch_rowsum(const T *__restrict__ H, int p, int rtot, T *__restrict__ out) {
@@ -524,17 +568,31 @@ void launch_consensus(const unsigned char *lab, int p, int nsel, unsigned *plane
 // Solves of rank R a CTA of shape `comp` carries (BCfg::NS).
 int ns_for(int R, int comp) { return comp / R > 0 ? comp / R : 1; }
 
+// One step's items: bucket 0's, then bucket 1's, then bucket 2's, or, narrow,
+// all of them by falling rank.
+struct StepPlan {
+    std::vector<BItem> items;
+    int count[kBuckets] = {};
+    bool narrow = false;
+};
 struct BatchPlan {
     int rtot = 0;
-    std::vector<int> group_off;           // per group, NS offsets (-1 padded)
-    std::vector<BItem> hitems, witems;    // bucket 0 items, then bucket 1, then 2
-    int nh[kBuckets] = {}, nw[kBuckets] = {};  // items per bucket
+    std::vector<int> group_off;  // per group, NS offsets (-1 padded)
+    StepPlan h, w;
 };
+
+// Warps a multiprocessor below which a step takes two columns a thread: its
+// warps of four columns, one launch a bucket, leave a multiprocessor too few
+// to cover the latency of their chains.  72 solves of ranks 2..10 at 2000 x
+// 5000: H step 1260 us with four columns (17 warps a multiprocessor, buckets
+// in turn), 678 with two; W step 927 (7 warps), 765 with two.  The same
+// columns, one by one, in either.
+constexpr int kNarrowWarps = 32;
 
 // Solves of one rank form a class; a class is cut into groups of NS solves;
 // every (group, tile) pair is one CTA of its bucket's launch.
 template <typename T>
-BatchPlan plan_batch(int n, int p, int nsolves, const int32_t *ranks, int comp) {
+BatchPlan plan_batch(int n, int p, int nsolves, const int32_t *ranks, int comp, int sms) {
     BatchPlan bp;
     std::vector<int> offsets(nsolves);
     std::map<int, std::vector<int>> by_rank;
@@ -543,28 +601,34 @@ BatchPlan plan_batch(int n, int p, int nsolves, const int32_t *ranks, int comp) 
         bp.rtot += ranks[s];
         by_rank[ranks[s]].push_back(s);
     }
-    const int htiles = (p + kTile<T> - 1) / kTile<T>, wtiles = (n + kTile<T> - 1) / kTile<T>;
-    for (int b = 0; b < kBuckets; b++) {
-        // Larger ranks first: their CTAs are the longest, so they start first.
-        for (auto it = by_rank.rbegin(); it != by_rank.rend(); ++it) {
-            const int R = it->first;
-            if (bucket_of(R) != b) continue;
-            const auto &members = it->second;
-            const int ns = ns_for(R, comp);
-            const int groups = (int)((members.size() + ns - 1) / ns);
-            for (int g = 0; g < groups; g++) {
-                const int at = (int)bp.group_off.size();
-                for (int i = 0; i < ns; i++) {
-                    const size_t idx = (size_t)g * ns + i;
-                    bp.group_off.push_back(idx < members.size() ? offsets[members[idx]] : -1);
-                }
-                for (int t = 0; t < htiles; t++) bp.hitems.push_back({R, at, t, 0});
-                for (int t = 0; t < wtiles; t++) bp.witems.push_back({R, at, t, 0});
-                bp.nh[b] += htiles;
-                bp.nw[b] += wtiles;
-            }
+    struct Group {
+        int R, at;
+    };
+    std::vector<Group> groups;  // larger ranks first: their CTAs are the longest
+    for (auto it = by_rank.rbegin(); it != by_rank.rend(); ++it) {
+        const int R = it->first;
+        const auto &members = it->second;
+        const int ns = ns_for(R, comp);
+        for (size_t g = 0; g < members.size(); g += ns) {
+            groups.push_back({R, (int)bp.group_off.size()});
+            for (int i = 0; i < ns; i++)
+                bp.group_off.push_back(g + i < members.size() ? offsets[members[g + i]] : -1);
         }
     }
+    const auto plan_step = [&](int cols, StepPlan &sp) {
+        const int wide = (cols + kTile<T> - 1) / kTile<T>;
+        sp.narrow = BTraits<T>::NARROW != BTraits<T>::CPT &&
+                    (int64_t)groups.size() * wide * (kThreads / 32) < (int64_t)kNarrowWarps * sms;
+        const int tiles = sp.narrow ? (cols + kNarrowTile<T> - 1) / kNarrowTile<T> : wide;
+        for (int b = 0; b < (sp.narrow ? 1 : kBuckets); b++)
+            for (const Group &g : groups) {
+                if (!sp.narrow && bucket_of(g.R) != b) continue;
+                for (int t = 0; t < tiles; t++) sp.items.push_back({g.R, g.at, t, 0});
+                sp.count[b] += tiles;
+            }
+    };
+    plan_step(p, bp.h);
+    plan_step(n, bp.w);
     return bp;
 }
 
@@ -581,10 +645,18 @@ struct BatchSteps {
 // One step's launches, one per bucket with items (bucket b's items follow
 // those of the buckets before it).
 template <typename T, int SHAPE, bool kComponentFast>
-void launch_buckets(const MuArgs<T> &a, const int *off, const BItem *items,
-                    const int (&count)[kBuckets], cudaStream_t s, int64_t *launches) {
+void launch_buckets(const MuArgs<T> &a, const int *off, const BItem *items, const StepPlan &sp,
+                    cudaStream_t s, int64_t *launches) {
     static_assert(kBuckets == 3, "one launch per bucket");
+    const int(&count)[kBuckets] = sp.count;
     const BItem *at = items;
+    if constexpr (BTraits<T>::NARROW != BTraits<T>::CPT) {
+        if (sp.narrow) {
+            batch_mu<T, kBuckets, SHAPE, kComponentFast><<<count[0], kThreads, 0, s>>>(a, off, at);
+            *launches += 1;
+            return;
+        }
+    }
     if (count[0]) batch_mu<T, 0, SHAPE, kComponentFast><<<count[0], kThreads, 0, s>>>(a, off, at);
     at += count[0];
     if (count[1]) batch_mu<T, 1, SHAPE, kComponentFast><<<count[1], kThreads, 0, s>>>(a, off, at);
@@ -600,10 +672,10 @@ void enqueue_batch_iters_s(long long it0, long long it1, const BatchPlan &bp, co
                            cudaStream_t s, int64_t *launches) {
     const int rtot = bp.rtot;
     for (long long it = it0; it <= it1; it++) {
-        batch_colsum<T><<<(rtot + 127) / 128, 128, 0, s>>>(W, n, rtot, rtot, sw);
-        launch_buckets<T, SHAPE, true>(st.h, d.off, d.hitems, bp.nh, s, launches);
+        batch_colsum<T><<<(rtot + 31) / 32, 256, 0, s>>>(W, n, rtot, rtot, sw);
+        launch_buckets<T, SHAPE, true>(st.h, d.off, d.hitems, bp.h, s, launches);
         batch_rowsum<T><<<(rtot + 7) / 8, 256, 0, s>>>(H, p, rtot, sh);
-        launch_buckets<T, SHAPE, false>(st.w, d.off, d.witems, bp.nw, s, launches);
+        launch_buckets<T, SHAPE, false>(st.w, d.off, d.witems, bp.w, s, launches);
         *launches += 2;
         if (it % 10 == 0) {
             batch_clamp<T><<<592, 256, 0, s>>>(W, (int64_t)n * rtot, H, (int64_t)rtot * p,
@@ -653,12 +725,12 @@ std::string shape_key(int device, size_t es, int n, int p, int nsolves, const in
 nmfcu_status upload_plan(nmfcu_context *c, const BatchPlan &bp, cudaStream_t s, BatchDev *d) {
     // One upload: group offsets, then H items, then W items (16-byte aligned).
     const size_t off_bytes = (sizeof(int) * bp.group_off.size() + 15) / 16 * 16;
-    const size_t item_bytes = sizeof(BItem) * (bp.hitems.size() + bp.witems.size());
+    const size_t item_bytes = sizeof(BItem) * (bp.h.items.size() + bp.w.items.size());
     std::vector<unsigned char> table(off_bytes + item_bytes, 0);
     std::memcpy(table.data(), bp.group_off.data(), sizeof(int) * bp.group_off.size());
-    std::memcpy(table.data() + off_bytes, bp.hitems.data(), sizeof(BItem) * bp.hitems.size());
-    std::memcpy(table.data() + off_bytes + sizeof(BItem) * bp.hitems.size(), bp.witems.data(),
-                sizeof(BItem) * bp.witems.size());
+    std::memcpy(table.data() + off_bytes, bp.h.items.data(), sizeof(BItem) * bp.h.items.size());
+    std::memcpy(table.data() + off_bytes + sizeof(BItem) * bp.h.items.size(), bp.w.items.data(),
+                sizeof(BItem) * bp.w.items.size());
     void *p_tab = nullptr;
     NMFCU_TRY(nmfcu_internal::context_buffer(c, 0, table.size(), &p_tab));
     // A pageable host source is staged before cudaMemcpyAsync returns, so the
@@ -666,7 +738,7 @@ nmfcu_status upload_plan(nmfcu_context *c, const BatchPlan &bp, cudaStream_t s, 
     NMFCU_CUDA_TRY(cudaMemcpyAsync(p_tab, table.data(), table.size(), cudaMemcpyHostToDevice, s));
     d->off = static_cast<const int *>(p_tab);
     d->hitems = reinterpret_cast<const BItem *>(static_cast<unsigned char *>(p_tab) + off_bytes);
-    d->witems = d->hitems + bp.hitems.size();
+    d->witems = d->hitems + bp.h.items.size();
     return NMFCU_OK;
 }
 
@@ -706,7 +778,8 @@ nmfcu_status pick_shape(nmfcu_context *c, int64_t max_iter, int n, int p, const 
     cudaError_t ce = cudaEventCreate(&e1);
     float best = 0.f;
     for (int v = 0; ce == cudaSuccess && v < BShapes<T>::kN; v++) {
-        const BatchPlan bp = plan_batch<T>(n, p, nsolves, ranks, BShapes<T>::comp[v]);
+        const BatchPlan bp = plan_batch<T>(n, p, nsolves, ranks, BShapes<T>::comp[v],
+                                           nmfcu_internal::context_sms(c));
         BatchDev d;
         const nmfcu_status ps = upload_plan(c, bp, s, &d);
         if (ps != NMFCU_OK) {
@@ -770,7 +843,8 @@ nmfcu_status run_batch_t(nmfcu_context *c, int64_t max_iter, int n, int p, const
         std::lock_guard<std::mutex> lk(g_shape_mu);
         g_last_shape = shape;
     }
-    const BatchPlan bp = plan_batch<T>(n, p, nsolves, ranks, BShapes<T>::comp[shape]);
+    const BatchPlan bp = plan_batch<T>(n, p, nsolves, ranks, BShapes<T>::comp[shape],
+                                       nmfcu_internal::context_sms(c));
     BatchDev d;
     NMFCU_TRY(upload_plan(c, bp, s, &d));
     BatchSteps<T> st;
