@@ -460,8 +460,9 @@ __device__ __forceinline__ double h_update_row(const EpiParams &e, double numi, 
 // ways (GramPlan):
 //   few tiles   a block a tile of kTileRows rows of W / kTileCols columns of
 //               H, its warps sharing the tile;
-//   many tiles  a warp a tile of 32 rows / columns, a block's warps each
-//               every (warps of the launch)-th tile.
+//   many tiles  a warp a tile of 32 rows / columns: tile t goes to block
+//               t mod B, whose warps take its tiles in turn, so that a
+//               launch has a warp on every multiprocessor before it has two.
 // A warp adds four rows (columns) of its tile at a time on the FP64 tensor
 // cores (mma.sync.m8n8k4: a fragment of X is both operands), a block adds its
 // warps in a fixed tree, publishes its entries and takes a ticket; the last
@@ -498,8 +499,8 @@ inline GramPlan gram_plan(int64_t len, int tile, int sms) {
     if (g.few) {
         g.blocks = (int)(tiles < 1 ? 1 : tiles);
     } else {
-        const int64_t b = (len + kWideThreads - 1) / kWideThreads;
-        g.blocks = (int)(b < cap ? b : cap);
+        const int64_t b = (len + 31) / 32;
+        g.blocks = (int)(b < sms ? b : sms);  // its registers leave room for one
     }
     // the tickets count at most 32 groups
     const int most = 32 * kGramGroup;
@@ -784,7 +785,7 @@ __global__ void __launch_bounds__(THREADS)
         if (warp < kTileRows / 4) steps(i0, min(kTileRows, n - i0), warp, warp + 1);
     } else {
         const int tiles = (n + 31) / 32;
-        for (int t = blockIdx.x * GA::WARPS + warp; t < tiles; t += gridDim.x * GA::WARPS)
+        for (int t = blockIdx.x + gridDim.x * warp; t < tiles; t += gridDim.x * GA::WARPS)
             steps(t * 32, min(32, n - t * 32), 0, 8);
     }
     ga.finish(g, scratch);
@@ -812,7 +813,7 @@ __global__ void __launch_bounds__(THREADS)
         if (warp < kTileCols / 4) steps(blockIdx.x * kTileCols, warp, warp + 1);
     } else {
         const int tiles = (p + kTileCols - 1) / kTileCols;
-        for (int t = blockIdx.x * GA::WARPS + warp; t < tiles; t += gridDim.x * GA::WARPS)
+        for (int t = blockIdx.x + gridDim.x * warp; t < tiles; t += gridDim.x * GA::WARPS)
             steps(t * kTileCols, 0, kTileCols / 4);
     }
     ga.finish(g, scratch);

@@ -1796,7 +1796,7 @@ __global__ void __launch_bounds__(THREADS, EpiSmem<RP, THREADS>::BLOCKS)
         __syncthreads();
         if (stopped) return;
         const int tiles = (p + TC - 1) / TC;
-        for (int t = blockIdx.x * WARPS + warp; t < tiles; t += gridDim.x * WARPS) {
+        for (int t = blockIdx.x + gridDim.x * warp; t < tiles; t += gridDim.x * WARPS) {
             const int j0 = t * TC, j = j0 + lane;
             const int ct = j0 / tcols, c = j0 - ct * tcols + lane;
             tp.find(sk, ct);
@@ -1955,21 +1955,25 @@ __global__ void __launch_bounds__(THREADS, EpiSmem<RP, THREADS>::BLOCKS)
         __syncthreads();
         if (stopped) return;
         const int tiles = (n + 31) / 32;
-        for (int t = blockIdx.x * WARPS + warp; t < tiles; t += gridDim.x * WARPS) {
+        for (int t = blockIdx.x + gridDim.x * warp; t < tiles; t += gridDim.x * WARPS) {
             const int i0 = t * 32, i = i0 + lane;
             const int rt = i0 / trows, rl = i0 - rt * trows;
             const int elems = min(32, n - i0) * RP;
             tp.find(sk, rt);
             double num[RP], wr[RP];
+            // The tile's 32 RP sums, RP of them a lane, a CTA's at a time.
+#pragma unroll
+            for (int i = 0; i < RP; i++) num[i] = 0.0;
+            for (int b = tp.lo; b <= tp.hi; b++) {
+                const double *src = part + tp.slot(sk, b) * trows * RP + (size_t)rl * RP + lane;
+#pragma unroll
+                for (int i = 0; i < RP; i++) num[i] += lane + 32 * i < elems ? src[32 * i] : 0.0;
+            }
             __syncwarp();  // the last tile's readers of sRow
-#pragma unroll 4
-            for (int x = lane; x < 32 * RP; x += 32) {
-                double a = 0.0;
-                if (x < elems) {
-                    const double *src = part + (size_t)rl * RP + x;
-                    for (int b = tp.lo; b <= tp.hi; b++) a += src[tp.slot(sk, b) * trows * RP];
-                }
-                sRow[(x / RP) * LD + x % RP] = a;
+#pragma unroll
+            for (int i = 0; i < RP; i++) {
+                const int x = lane + 32 * i;
+                sRow[(x / RP) * LD + x % RP] = num[i];
             }
             __syncwarp();
 #pragma unroll
