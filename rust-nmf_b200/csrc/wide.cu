@@ -48,69 +48,105 @@ inline size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 
 // ---------------------------------------------------------------------------
 // Grams: G[k][l] = sum_u X(u, k) X(u, l) and sums[k] = sum_u X(u, k) for
-// X(u, k) = X[u * sr + k * sc] (W: sr = r, sc = 1; H^T: sr = 1, sc = p).
-// Stage 1: block (b, g) adds rows [b * rpb, (b + 1) * rpb) for pairs
-// g * kT * kPPT + i * kT + t, pair = k * (r + 1) + l (l == r: the sum);
-// rows staged kRowsChunk at a time.  Stage 2 adds the blocks in order.
+// X(u, k) = X[u * sr + k * sc] (W: sr = r, sc = 1; H^T: sr = 1, sc = p), on the
+// FP64 tensor cores (mma.sync.m8n8k4, kernels.cuh dmma_8x8x4) over X with a
+// column of ones behind it, whose products are the sums.
+// Stage 1: block (b, y) takes rows [b * rpb, (b + 1) * rpb), kRowsChunk at a
+// time through shared memory, and the 8 x 8 tiles (mt <= nt) y * 64 .. + 63 of
+// the product, eight a warp.  Stage 2 adds the blocks in order.
+// One thread eight entries on the CUDA cores took 94 us for H at 50 x 20000,
+// this 20.
 // ---------------------------------------------------------------------------
-constexpr int kPPT = 8;
-constexpr int kRowsChunk = 16;  // 16 x 256 f64 = 32 KB of staging at the largest rank
+constexpr int kRowsChunk = 32;
+constexpr int kGramLd = 36;  // a warp's fragment loads meet every bank once
+constexpr int kWarpPairs = 8;
+constexpr int kBlockPairs = kWarpPairs * (kT / 32);
+
+__host__ __device__ inline int wide_mt(int r) { return (r + 1 + 7) / 8; }
+__host__ __device__ inline int wide_pairs(int r) { return wide_mt(r) * (wide_mt(r) + 1) / 2; }
+// Tile number -> (mt, nt), mt <= nt.
+__device__ __forceinline__ void wide_pair(int t, int MT, int &mt, int &nt) {
+    mt = 0;
+    while (t >= MT - mt) {
+        t -= MT - mt;
+        mt++;
+    }
+    nt = mt + t;
+}
 
 __global__ void __launch_bounds__(kT)
     wide_gram_partial(const double *__restrict__ X, int64_t m, int r, int64_t sr, int64_t sc,
                       int64_t rpb, double *__restrict__ part, const RunState *st) {
     if (nmfcu::run_stopped(st)) return;
-    extern __shared__ double chunk[];  // [kRowsChunk][r]
-    const int npairs = r * (r + 1);
+    extern __shared__ double chunk[];  // [8 MT columns][kGramLd]
+    const int MT = wide_mt(r), pairs = wide_pairs(r);
     const int64_t u0 = blockIdx.x * rpb, u1 = min(m, u0 + rpb);
-    int pk[kPPT], pl[kPPT];
-    double acc[kPPT];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int g = lane >> 2, q = lane & 3;
+    const int t0 = blockIdx.y * kBlockPairs + warp * kWarpPairs;
+    int am[kWarpPairs], an[kWarpPairs];  // the tiles' fragments in chunk
+    double acc[kWarpPairs][2];
 #pragma unroll
-    for (int i = 0; i < kPPT; i++) {
-        const int pr = (blockIdx.y * kPPT + i) * kT + threadIdx.x;
-        pk[i] = pr < npairs ? pr / (r + 1) : -1;
-        pl[i] = pr < npairs ? pr - pk[i] * (r + 1) : 0;
-        acc[i] = 0.0;
+    for (int i = 0; i < kWarpPairs; i++) {
+        int mt = 0, nt = 0;
+        if (t0 + i < pairs) wide_pair(t0 + i, MT, mt, nt);
+        am[i] = (mt * 8 + g) * kGramLd + q;
+        an[i] = (nt * 8 + g) * kGramLd + q;
+        acc[i][0] = acc[i][1] = 0.0;
     }
     for (int64_t c0 = u0; c0 < u1; c0 += kRowsChunk) {
         const int nr = (int)min((int64_t)kRowsChunk, u1 - c0);
         __syncthreads();
-        for (int e = threadIdx.x; e < nr * r; e += kT) {
-            const int uu = e / r, k = e - uu * r;
-            chunk[e] = X[(c0 + uu) * sr + (int64_t)k * sc];
+        for (int e = threadIdx.x; e < MT * 8 * kRowsChunk; e += kT) {
+            int uu, k;
+            if (sr == 1) {  // neighbours along the rows
+                k = e / kRowsChunk;
+                uu = e - k * kRowsChunk;
+            } else {
+                uu = e / (MT * 8);
+                k = e - uu * (MT * 8);
+            }
+            double v = 0.0;
+            if (uu < nr) v = k < r ? X[(c0 + uu) * sr + (int64_t)k * sc] : k == r ? 1.0 : 0.0;
+            chunk[k * kGramLd + uu] = v;
         }
         __syncthreads();
+        if (t0 < pairs)
+#pragma unroll 2
+            for (int s = 0; s < kRowsChunk; s += 4)
 #pragma unroll
-        for (int i = 0; i < kPPT; i++) {
-            if (pk[i] < 0) continue;
-            double a = acc[i];
-            if (pl[i] == r) {
-                for (int uu = 0; uu < nr; uu++) a += chunk[uu * r + pk[i]];
-            } else {
-                for (int uu = 0; uu < nr; uu++) a += chunk[uu * r + pk[i]] * chunk[uu * r + pl[i]];
-            }
-            acc[i] = a;
-        }
+                for (int i = 0; i < kWarpPairs; i++)
+                    if (t0 + i < pairs)
+                        nmfcu::dmma_8x8x4(acc[i], chunk[am[i] + s], chunk[an[i] + s]);
     }
 #pragma unroll
-    for (int i = 0; i < kPPT; i++)
-        if (pk[i] >= 0) part[(int64_t)blockIdx.x * npairs + pk[i] * (r + 1) + pl[i]] = acc[i];
+    for (int i = 0; i < kWarpPairs; i++)
+        if (t0 + i < pairs) {
+            double *d = part + ((size_t)blockIdx.x * pairs + t0 + i) * 64 + g * 8 + 2 * q;
+            d[0] = acc[i][0];
+            d[1] = acc[i][1];
+        }
 }
 
 __global__ void wide_gram_final(const double *__restrict__ part, int B, int r,
                                 double *__restrict__ G, double *__restrict__ sums,
                                 const RunState *st) {
     if (nmfcu::run_stopped(st)) return;
-    const int npairs = r * (r + 1);
-    const int pr = blockIdx.x * kT + threadIdx.x;
-    if (pr >= npairs) return;
-    double a = 0.0;
-    for (int b = 0; b < B; b++) a += part[(int64_t)b * npairs + pr];
-    const int k = pr / (r + 1), l = pr - k * (r + 1);
-    if (l == r)
+    const int MT = wide_mt(r), pairs = wide_pairs(r);
+    const int x = blockIdx.x * kT + threadIdx.x;
+    if (x >= pairs * 64) return;
+    int mt, nt;
+    wide_pair(x >> 6, MT, mt, nt);
+    const int k = mt * 8 + ((x >> 3) & 7), l = nt * 8 + (x & 7);
+    if (k >= r || l > r || l < k) return;
+    const double a = nmfcu::sum_strided(0.0, part + x, (size_t)pairs * 64, B,
+                                        [](const double *p) { return *p; });
+    if (l == r) {
         sums[k] = a;
-    else
+    } else {
         G[k * r + l] = a;
+        G[l * r + k] = a;
+    }
 }
 
 // Ht (p x r) = H (r x p)^T through 32 x 32 shared-memory tiles.
@@ -134,74 +170,148 @@ __global__ void wide_transpose(const double *__restrict__ H, int r, int64_t p,
 }
 
 // ---------------------------------------------------------------------------
-// W H in 64 x 64 tiles (16 x 16 threads, 4 x 4 outputs a thread, the rank
-// in chunks of 16 through shared memory), and what each use makes of it:
+// W H in 128 x 64 tiles on the FP64 tensor cores (eight warps of 32 x 32, the
+// rank in chunks of 16 through shared memory, the next chunk in registers),
+// and what each use makes of it:
 //   MODE 0  Q[i][j] = V[i][j] / (W H)[i][j], 0 where W H is 0 (brunet's ratio)
 //   MODE 1  per-block partial of the KL objective (kl_divergence lib.rs:1418-1427)
 //   MODE 2  per-block partial of sum (V - W H)^2 (euclidean_distance :1440-1441)
+// Bound: FP64.  5000 x 20000 rank 50, MODE 0: 1062 us on the CUDA cores, 797
+// here (two blocks a multiprocessor; 983 with one).
 // ---------------------------------------------------------------------------
+// v / w: the refined reciprocal of the dense passes (ratio_div) and one residual
+// correction (Markstein 1990), so the quotient is as good as a division's,
+// which takes its slow way out for every v of 0.
+__device__ __forceinline__ double quotient(double v, double w) {
+    const double q = nmfcu::ratio_div(v, w);
+    const double a = fabs(w);
+    if (!(a > 0x1p-500 && a < 0x1p500 && q < 0x1p500)) return q;
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(w));
+    return fma(fma(-q, w, v), r, q);
+}
+constexpr int kWhRows = 128, kWhCols = 64, kWhK = 16;
+constexpr int kWhLdW = 20, kWhLdH = 68;  // fragment loads meet every bank once
+
 template <int MODE>
-__global__ void __launch_bounds__(kT)
+__global__ void __launch_bounds__(kT, 2)
     wide_wh(const double *__restrict__ V, int64_t ldv, const double *__restrict__ W,
             const double *__restrict__ H, int n, int64_t p, int r, double *__restrict__ Q,
             int64_t ldq, double *__restrict__ part, const RunState *st) {
     if (nmfcu::run_stopped(st)) return;
-    __shared__ double sW[64][17];
-    __shared__ double sH[16][64];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int i0 = blockIdx.y * 64;
-    const int64_t j0 = (int64_t)blockIdx.x * 64;
-    double acc[4][4];
+    __shared__ double sW[kWhRows][kWhLdW];
+    __shared__ double sH[kWhK][kWhLdH];
+    constexpr int PW = kWhRows * kWhK / kT, PH = kWhK * kWhCols / kT;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int g = lane >> 2, q = lane & 3;
+    const int wr = (warp >> 1) * 32, wc = (warp & 1) * 32;  // the warp's tile
+    const int i0 = blockIdx.y * kWhRows;
+    const int64_t j0 = (int64_t)blockIdx.x * kWhCols;
+    double acc[4][4][2];
 #pragma unroll
     for (int a = 0; a < 4; a++)
 #pragma unroll
-        for (int b = 0; b < 4; b++) acc[a][b] = 0.0;
-    for (int k0 = 0; k0 < r; k0 += 16) {
+        for (int b = 0; b < 4; b++) acc[a][b][0] = acc[a][b][1] = 0.0;
+    double vw[PW], vh[PH];
+    const auto fetch = [&](int k0) {
+#pragma unroll
+        for (int t = 0; t < PW; t++) {
+            const int e = threadIdx.x + t * kT;
+            const int i = i0 + e / kWhK, k = k0 + e % kWhK;
+            vw[t] = (i < n && k < r) ? W[(int64_t)i * r + k] : 0.0;
+        }
+#pragma unroll
+        for (int t = 0; t < PH; t++) {
+            const int e = threadIdx.x + t * kT;
+            const int k = k0 + e / kWhCols;
+            const int64_t j = j0 + e % kWhCols;
+            vh[t] = (k < r && j < p) ? H[(int64_t)k * p + j] : 0.0;
+        }
+    };
+    fetch(0);
+    for (int k0 = 0; k0 < r; k0 += kWhK) {
         __syncthreads();
-        for (int e = threadIdx.x; e < 64 * 16; e += kT) {
-            const int ii = e >> 4, kk = e & 15;
-            const int i = i0 + ii, k = k0 + kk;
-            sW[ii][kk] = (i < n && k < r) ? W[(int64_t)i * r + k] : 0.0;
-            const int kh = e >> 6, jj = e & 63;
-            const int64_t j = j0 + jj;
-            sH[kh][jj] = (k0 + kh < r && j < p) ? H[(int64_t)(k0 + kh) * p + j] : 0.0;
+#pragma unroll
+        for (int t = 0; t < PW; t++) {
+            const int e = threadIdx.x + t * kT;
+            sW[e / kWhK][e % kWhK] = vw[t];
+        }
+#pragma unroll
+        for (int t = 0; t < PH; t++) {
+            const int e = threadIdx.x + t * kT;
+            sH[e / kWhCols][e % kWhCols] = vh[t];
         }
         __syncthreads();
+        if (k0 + kWhK < r) fetch(k0 + kWhK);
 #pragma unroll
-        for (int kk = 0; kk < 16; kk++) {
-            double w[4], h[4];
+        for (int ks = 0; ks < kWhK; ks += 4) {
+            if (k0 + ks >= r) break;
+            double a[4], b[4];
 #pragma unroll
-            for (int a = 0; a < 4; a++) w[a] = sW[ty + 16 * a][kk];
+            for (int t = 0; t < 4; t++) {
+                a[t] = sW[wr + t * 8 + g][ks + q];
+                b[t] = sH[ks + q][wc + t * 8 + g];
+            }
 #pragma unroll
-            for (int b = 0; b < 4; b++) h[b] = sH[kk][tx + 16 * b];
+            for (int x = 0; x < 4; x++)
 #pragma unroll
-            for (int a = 0; a < 4; a++)
-#pragma unroll
-                for (int b = 0; b < 4; b++) acc[a][b] = fma(w[a], h[b], acc[a][b]);
+                for (int y = 0; y < 4; y++) nmfcu::dmma_8x8x4(acc[x][y], a[x], b[y]);
         }
     }
+    // A row's eight elements a thread are loaded together, the next row's while
+    // this one's are divided (or their logarithms taken).
     double term = 0.0;
+    const auto load_row = [&](int x, double (&v)[8]) {
+        const int i = i0 + wr + x * 8 + g;
 #pragma unroll
-    for (int a = 0; a < 4; a++) {
-        const int i = i0 + ty + 16 * a;
-        if (i >= n) continue;
+        for (int y = 0; y < 4; y++) {
+            const int64_t j = j0 + wc + y * 8 + 2 * q;
+            const double *src = V + (int64_t)i * ldv + j;  // 16-byte aligned
+            double2 d = make_double2(0.0, 0.0);
+            if (i < n && j + 1 < p)
+                d = *reinterpret_cast<const double2 *>(src);
+            else if (i < n && j < p)
+                d.x = *src;
+            v[2 * y] = d.x;
+            v[2 * y + 1] = d.y;
+        }
+    };
+    double vn[8];
+    load_row(0, vn);
 #pragma unroll
-        for (int b = 0; b < 4; b++) {
-            const int64_t j = j0 + tx + 16 * b;
-            if (j >= p) continue;
-            const double v = V[(int64_t)i * ldv + j];
-            const double wh = acc[a][b];
-            if (MODE == 0) {
-                Q[(int64_t)i * ldq + j] = (wh != 0.0) ? v / wh : 0.0;
-            } else if (MODE == 1) {
-                if (v > 0.0) {
-                    if (wh > 0.0) term = add(term, add(sub(mul(v, log(v / wh)), v), wh));
+    for (int x = 0; x < 4; x++) {
+        const int i = i0 + wr + x * 8 + g;
+        double v[8];
+#pragma unroll
+        for (int t = 0; t < 8; t++) v[t] = vn[t];
+        if (x < 3) load_row(x + 1, vn);
+#pragma unroll
+        for (int y = 0; y < 4; y++) {
+            const int64_t j = j0 + wc + y * 8 + 2 * q;
+            double o[2];
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const double ve = v[2 * y + e], wh = acc[x][y][e];
+                // past V's edge v and W H are 0: no term
+                if (MODE == 0) {
+                    o[e] = (wh != 0.0) ? quotient(ve, wh) : 0.0;
+                } else if (MODE == 1) {
+                    if (ve > 0.0) {
+                        if (wh > 0.0) term = add(term, add(sub(mul(ve, log(ve / wh)), ve), wh));
+                    } else {
+                        term = add(term, wh);
+                    }
                 } else {
-                    term = add(term, wh);
+                    const double d = sub(ve, wh);
+                    term = add(term, mul(d, d));
                 }
-            } else {
-                const double d = sub(v, wh);
-                term = add(term, mul(d, d));
+            }
+            if (MODE == 0 && i < n) {
+                double *dst = Q + (int64_t)i * ldq + j;
+                if (j + 1 < p)
+                    *reinterpret_cast<double2 *>(dst) = make_double2(o[0], o[1]);
+                else if (j < p)
+                    *dst = o[0];
             }
         }
     }
@@ -218,87 +328,194 @@ __global__ void __launch_bounds__(kT)
 }
 
 // ---------------------------------------------------------------------------
-// Updates, one thread per column of H / row of W, in the dense epilogues'
-// operation order (kernels.cuh h_update / w_update).
+// Updates, in the dense epilogues' operation order (kernels.cuh h_update /
+// w_update).  A block takes kUpd columns of H / rows of W, their old values
+// in shared memory, a lane a column / row; lee's and brunet's entries are
+// independent and go to the warps in turn, four at a time; so do the old
+// values' terms of the HALS / dnmf sweeps, which then go eight entries at a time.  (One
+// thread a column, reading H from L2 for every term, took 124 us for H at 50 x
+// 20000 and 188 us for W at 5000 x 50 with lee; now 47 and 17.)
 // ---------------------------------------------------------------------------
+constexpr int kUpd = 32;
 struct WideEpi {
     int method;
     int r;
     double eps, lambda, gamma;
-    const double *G;     // r x r
+    const double *G;     // r x r, symmetric
     const double *sums;  // r
 };
 
-// H (r x p); num: p x r (num[j * r + k]); lee writes Hn, the others H.
-__global__ void __launch_bounds__(kT)
-    wide_h_update(double *__restrict__ H, double *__restrict__ Hn, int64_t p,
-                  const double *__restrict__ num, WideEpi e, const RunState *st) {
-    if (nmfcu::run_stopped(st)) return;
-    const int64_t j = (int64_t)blockIdx.x * kT + threadIdx.x;
-    if (j >= p) return;
+// The Gauss-Seidel sweeps (hals_update_{h,w} lib.rs:595-605, :622-632; their
+// regularised forms :1079-1089, :1106-1116): entry k becomes
+//   max(eps, (num_k [- lambda] - sum_{j != k} G_kj x_j) / max(G_kk [+ gamma], eps))
+// with x_j new for j < k.  Written as one sum it is a chain of r dependent
+// subtractions an entry, r^2 a line: 357 us for H at 90 x 10000, 132 this way.  x_j is old for
+// j > k, so those terms go first, for all entries at once, and a new value's
+// term goes to every later entry as soon as it is there.  The same terms in
+// another order, by FMA: the rounding of a sum differs by an ulp or so of its
+// largest term.
+struct SweepDiv {
+    double d, r;  // the divisor and RN(1 / d)
+};
+__device__ __forceinline__ SweepDiv sweep_div(const WideEpi &e, double gkk) {
+    const double d = e.method == nmfcu::M_DNMF ? fmax(add(gkk, e.gamma), e.eps) : fmax(gkk, e.eps);
+    return {d, __drcp_rn(d)};
+}
+// max(eps, s / d): the quotient from the reciprocal with one residual
+// correction (Markstein 1990), three dependent operations.
+__device__ __forceinline__ double sweep_value(double s, SweepDiv v, double eps) {
+    double q = __dmul_rn(s, v.r);
+    if (fabs(s) < 0x1p900) q = fma(fma(-q, v.d, s), v.r, q);
+    return q > eps ? q : eps;
+}
+
+// The new values of one line (a column of H or a row of W): line x of the
+// block's, its old values at old[k * (kUpd + 1) + x], its contraction at
+// sum[k * (kUpd + 1) + x] (both may be overwritten); out(k, v) stores entry k.
+template <bool HSIDE, typename Out>
+__device__ __forceinline__ void wide_line(double *old, double *sum, int x, bool in,
+                                          const WideEpi &e, int warp, int warps, Out &&out) {
     const int r = e.r;
-    const double *nj = num + j * r;
+    double *o = old + x;
+    constexpr int LD = kUpd + 1;
+    const auto num = [&](int k) { return sum[k * LD + x]; };
     if (e.method == nmfcu::M_LEE) {
-        // euclidean_update_h_inner lib.rs:227-241
-        for (int i = 0; i < r; i++) {
-            double den = 0.0;
-            for (int l = r - 1; l >= 0; l--) den = add(den, mul(e.G[i * r + l], H[(int64_t)l * p + j]));
-            const double temp = mul(H[(int64_t)i * p + j], nj[i]);
-            Hn[(int64_t)i * p + j] = (temp > e.eps ? temp : e.eps) / add(den, e.eps);
+        // euclidean_update_h_inner lib.rs:227-241, euclidean_update_w_impl :307-318
+        for (int i = warp * 4; i < r; i += warps * 4) {
+            double den[4] = {0.0, 0.0, 0.0, 0.0};
+            const int m = min(4, r - i);
+            if (m == 4) {
+#pragma unroll 4
+                for (int l = r - 1; l >= 0; l--) {
+                    const double h = o[l * LD];
+                    const double *gl = e.G + (int64_t)l * r + i;
+#pragma unroll
+                    for (int t = 0; t < 4; t++) den[t] = add(den[t], mul(gl[t], h));
+                }
+            } else {
+                for (int l = r - 1; l >= 0; l--) {
+                    const double h = o[l * LD];
+#pragma unroll
+                    for (int t = 0; t < 3; t++)
+                        if (t < m) den[t] = add(den[t], mul(e.G[(int64_t)l * r + i + t], h));
+                }
+            }
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                if (t >= m || !in) continue;
+                const double temp = mul(o[(i + t) * LD], num(i + t));
+                // H keeps a NaN's clamp at eps, W the NaN (lib.rs:240, :317)
+                const double top = HSIDE ? (temp > e.eps ? temp : e.eps)
+                                         : (temp < e.eps ? e.eps : temp);
+                out(i + t, top / add(den[t], e.eps));
+            }
         }
     } else if (e.method == nmfcu::M_BRUNET) {
-        // divergence_update_h_inner lib.rs:105-111
-        for (int i = 0; i < r; i++) {
-            double &h = H[(int64_t)i * p + j];
-            h = mul(h, nj[i]) / e.sums[i];
-        }
+        // divergence_update_h_inner lib.rs:105-111, divergence_update_w_impl :194-200
+        if (in)
+            for (int i = warp; i < r; i += warps) out(i, mul(o[i * LD], num(i)) / e.sums[i]);
     } else {
-        // hals_update_h lib.rs:595-605; hals_update_h_reg lib.rs:1079-1089
-        const bool reg = (e.method == nmfcu::M_DNMF);
-        for (int k = 0; k < r; k++) {
-            double s = reg ? sub(nj[k], e.lambda) : nj[k];
-            for (int jj = 0; jj < r; jj++)
-                if (jj != k) s = sub(s, mul(e.G[k * r + jj], H[(int64_t)jj * p + j]));
-            const double d = reg ? fmax(add(e.G[k * r + k], e.gamma), e.eps) : fmax(e.G[k * r + k], e.eps);
-            const double val = s / d;
-            H[(int64_t)k * p + j] = val > e.eps ? val : e.eps;
+        // The sweep: the old values' terms of every entry first, four entries
+        // a warp at a time; then eight entries in order by one warp, and their
+        // terms of every later entry by all.  Entry k's sum is in num(k)'s place.
+        const bool reg = e.method == nmfcu::M_DNMF;
+        double *sm = sum + x;
+        for (int i = warp * 4; i < r; i += warps * 4) {
+            const int m = min(4, r - i);
+            double a[4];
+#pragma unroll
+            for (int t = 0; t < 4; t++)
+                a[t] = t < m ? (reg ? sub(sm[(i + t) * LD], e.lambda) : sm[(i + t) * LD]) : 0.0;
+#pragma unroll 4
+            for (int l = i + 1; l < r; l++) {
+                const double h = o[l * LD];
+                const double *gl = e.G + (int64_t)l * r + i;
+#pragma unroll
+                for (int t = 0; t < 4; t++)
+                    if (t < m && l > i + t) a[t] = fma(-gl[t], h, a[t]);
+            }
+#pragma unroll
+            for (int t = 0; t < 4; t++)
+                if (t < m) sm[(i + t) * LD] = a[t];
+        }
+        for (int k0 = 0; k0 < r; k0 += 8) {
+            __syncthreads();
+            const int m = min(8, r - k0);
+            if (warp == 0) {
+                double sv[8], g[8][8];
+                SweepDiv dv[8];
+#pragma unroll
+                for (int a = 0; a < 8; a++) {
+                    sv[a] = a < m ? sm[(k0 + a) * LD] : 0.0;
+#pragma unroll
+                    for (int b = a; b < 8; b++)
+                        g[a][b] = b < m ? e.G[(int64_t)(k0 + a) * r + k0 + b] : 0.0;
+                    dv[a] = sweep_div(e, g[a][a]);
+                }
+#pragma unroll
+                for (int a = 0; a < 8; a++) {
+                    if (a >= m) continue;
+                    const double v = sweep_value(sv[a], dv[a], e.eps);
+#pragma unroll
+                    for (int b = a + 1; b < 8; b++) sv[b] = fma(-g[a][b], v, sv[b]);
+                    o[(k0 + a) * LD] = v;
+                    if (in) out(k0 + a, v);
+                }
+            }
+            __syncthreads();
+            for (int i = k0 + 8 + warp; i < r; i += warps) {
+                const double *gi = e.G + (int64_t)i * r + k0;
+                double a = sm[i * LD];
+#pragma unroll
+                for (int t = 0; t < 8; t++)  // (no later entry unless all eight are there)
+                    a = fma(-gi[t], o[(k0 + t) * LD], a);
+                sm[i * LD] = a;
+            }
         }
     }
 }
 
-// W (n x r); num: n x r; lee writes Wn, the others W.
+// H (r x p) in place; num: p x r (num[j * r + k]).
 __global__ void __launch_bounds__(kT)
-    wide_w_update(double *__restrict__ W, double *__restrict__ Wn, int n,
-                  const double *__restrict__ num, WideEpi e, const RunState *st) {
+    wide_h_update(double *__restrict__ H, int64_t p, const double *__restrict__ num, WideEpi e,
+                  const RunState *st) {
     if (nmfcu::run_stopped(st)) return;
-    const int i = blockIdx.x * kT + threadIdx.x;
-    if (i >= n) return;
-    const int r = e.r;
-    double *wr = W + (int64_t)i * r;
-    const double *ni = num + (int64_t)i * r;
-    if (e.method == nmfcu::M_LEE) {
-        // euclidean_update_w_impl lib.rs:307-318
-        for (int j = 0; j < r; j++) {
-            double den = 0.0;
-            for (int l = r - 1; l >= 0; l--) den = add(den, mul(wr[l], e.G[l * r + j]));
-            const double temp = mul(wr[j], ni[j]);
-            Wn[(int64_t)i * r + j] = (temp < e.eps ? e.eps : temp) / add(den, e.eps);
-        }
-    } else if (e.method == nmfcu::M_BRUNET) {
-        // divergence_update_w_impl lib.rs:194-200
-        for (int j = 0; j < r; j++) wr[j] = mul(wr[j], ni[j]) / e.sums[j];
-    } else {
-        // hals_update_w lib.rs:622-632; hals_update_w_reg lib.rs:1106-1116
-        const bool reg = (e.method == nmfcu::M_DNMF);
-        for (int k = 0; k < r; k++) {
-            double s = reg ? sub(ni[k], e.lambda) : ni[k];
-            for (int jj = 0; jj < r; jj++)
-                if (jj != k) s = sub(s, mul(e.G[k * r + jj], wr[jj]));
-            const double d = reg ? fmax(add(e.G[k * r + k], e.gamma), e.eps) : fmax(e.G[k * r + k], e.eps);
-            const double val = s / d;
-            wr[k] = val > e.eps ? val : e.eps;
-        }
+    extern __shared__ double upd[];
+    double *old = upd, *sn = upd + (size_t)e.r * (kUpd + 1);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int64_t j0 = (int64_t)blockIdx.x * kUpd;
+    const int cols = (int)min((int64_t)kUpd, p - j0), r = e.r;
+    for (int k = warp; k < r; k += warps)
+        old[k * (kUpd + 1) + lane] = lane < cols ? H[(int64_t)k * p + j0 + lane] : 0.0;
+    for (int x = threadIdx.x; x < kUpd * r; x += blockDim.x)
+        sn[(x % r) * (kUpd + 1) + x / r] = x < cols * r ? num[j0 * r + x] : 0.0;
+    __syncthreads();
+    wide_line<true>(old, sn, lane, lane < cols, e, warp, warps,
+                    [&](int k, double v) { H[(int64_t)k * p + j0 + lane] = v; });
+}
+
+// W (n x r) in place; num: n x r.
+__global__ void __launch_bounds__(kT)
+    wide_w_update(double *__restrict__ W, int n, const double *__restrict__ num, WideEpi e,
+                  const RunState *st) {
+    if (nmfcu::run_stopped(st)) return;
+    extern __shared__ double upd[];
+    double *old = upd, *sn = upd + (size_t)e.r * (kUpd + 1);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int64_t i0 = (int64_t)blockIdx.x * kUpd;
+    const int rows = (int)min((int64_t)kUpd, n - i0), r = e.r;
+    for (int x = threadIdx.x; x < kUpd * r; x += blockDim.x) {
+        const int at = (x % r) * (kUpd + 1) + x / r;
+        old[at] = x < rows * r ? W[i0 * r + x] : 0.0;
+        sn[at] = x < rows * r ? num[i0 * r + x] : 0.0;
     }
+    __syncthreads();
+    // the new values take num's place, then go out contiguously
+    wide_line<false>(old, sn, lane, lane < rows, e, warp, warps,
+                     [&](int k, double v) { sn[k * (kUpd + 1) + lane] = v; });
+    __syncthreads();
+    for (int x = threadIdx.x; x < rows * r; x += blockDim.x)
+        W[i0 * r + x] = sn[(x % r) * (kUpd + 1) + x / r];
 }
 
 // lee's col_rescale (lib.rs:1461-1470): W[:, k] /= colsum_k when > 0.
@@ -350,7 +567,7 @@ __global__ void wide_dnmf_rescale(double *__restrict__ W, int64_t n, double *__r
 // ---------------------------------------------------------------------------
 
 struct Bufs {
-    double *W, *H, *Ht, *NW, *NH, *Wn, *Hn, *part, *Gw, *sw, *Gh, *sh, *Gw2, *sw2, *opart;
+    double *W, *H, *Ht, *NW, *NH, *part, *Gw, *sw, *Gh, *sh, *Gw2, *sw2, *opart;
     double *Q;
     int64_t ldq;
     int Bw, Bh, gy;
@@ -373,9 +590,12 @@ struct Loop {
     nmfcu_status gram(const double *X, int64_t m, int64_t sr, int64_t sc, int B, int64_t rpb,
                       double *G, double *sums) {
         nmfcu_internal::TimedScope sc_(c, s, NMFCU_KCLASS_OTHER, 2);
-        const size_t sm = sizeof(double) * kRowsChunk * r;
+        const size_t sm = sizeof(double) * 8 * wide_mt(r) * kGramLd;
+        NMFCU_CUDA_TRY(cudaFuncSetAttribute(
+            wide_gram_partial, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
         wide_gram_partial<<<dim3(B, b.gy), kT, sm, s>>>(X, m, r, sr, sc, rpb, b.part, st);
-        wide_gram_final<<<cdiv((int64_t)r * (r + 1), kT), kT, 0, s>>>(b.part, B, r, G, sums, st);
+        wide_gram_final<<<cdiv((int64_t)wide_pairs(r) * 64, kT), kT, 0, s>>>(b.part, B, r, G, sums,
+                                                                            st);
         NMFCU_CUDA_TRY(cudaGetLastError());
         return NMFCU_OK;
     }
@@ -401,6 +621,8 @@ struct Loop {
         e.sums = sums;
         return e;
     }
+    // Old values and contraction of a block's lines: at most 135 KB.
+    size_t update_smem() const { return sizeof(double) * 2 * (size_t)r * (kUpd + 1); }
     // The H step: numerator p x r (V^T W, or Q^T W for brunet), then the update.
     nmfcu_status h_step(const WideEpi &e) {
         const bool kl = o->method == NMFCU_BRUNET;
@@ -409,10 +631,11 @@ struct Loop {
         NMFCU_TRY(nmfcu_internal::v_product_locked(c, 1, n, p, r, kl ? b.Q : V, kl ? b.ldq : ldv,
                                                    b.W, r, b.NH, r, s, false, false));
         nmfcu_internal::TimedScope sc_(c, s, NMFCU_KCLASS_OTHER);
-        wide_h_update<<<std::max(1u, cdiv(p, kT)), kT, 0, s>>>(b.H, b.Hn, p, b.NH, e, st);
-        if (o->method == NMFCU_LEE)
-            NMFCU_CUDA_TRY(cudaMemcpyAsync(b.H, b.Hn, sizeof(double) * (size_t)r * p,
-                                           cudaMemcpyDeviceToDevice, s));
+        const size_t sm = update_smem();
+        NMFCU_CUDA_TRY(cudaFuncSetAttribute(
+            wide_h_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        if (p > 0) wide_h_update<<<cdiv(p, kUpd), kT, sm, s>>>(b.H, p, b.NH, e, st);
+        NMFCU_CUDA_TRY(cudaGetLastError());
         return NMFCU_OK;
     }
     // The W step: numerator n x r (V H'^T, or Q H'^T for brunet), then the update.
@@ -424,10 +647,12 @@ struct Loop {
         NMFCU_TRY(nmfcu_internal::v_product_locked(c, 0, n, p, r, kl ? b.Q : V, kl ? b.ldq : ldv,
                                                    b.Ht, r, b.NW, r, s, false, false));
         nmfcu_internal::TimedScope sc_(c, s, NMFCU_KCLASS_OTHER);
-        wide_w_update<<<std::max(1u, cdiv(n, kT)), kT, 0, s>>>(b.W, b.Wn, (int)n, b.NW, e, st);
-        if (o->method == NMFCU_LEE)
-            NMFCU_CUDA_TRY(cudaMemcpyAsync(b.W, b.Wn, sizeof(double) * (size_t)n * r,
-                                           cudaMemcpyDeviceToDevice, s));
+        const size_t sm = update_smem();
+        NMFCU_CUDA_TRY(cudaFuncSetAttribute(
+            wide_w_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        if (n > 0)
+            wide_w_update<<<cdiv(n, kUpd), kT, sm, s>>>(b.W, (int)n, b.NW, e, st);
+        NMFCU_CUDA_TRY(cudaGetLastError());
         return NMFCU_OK;
     }
     nmfcu_status objective(long long iter) {
@@ -503,26 +728,25 @@ struct Loop {
 nmfcu_status make_bufs(nmfcu_context *c, const nmfcu_options *o, int64_t n, int64_t p, int r,
                        Bufs &b) {
     const int sms = nmfcu_internal::context_sms(c);
-    b.Bw = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, sms));
+    b.Bw = (int)std::max<int64_t>(1, std::min<int64_t>((n + 63) / 64, sms));
     b.rpw = std::max<int64_t>(1, (n + b.Bw - 1) / b.Bw);
-    b.Bh = (int)std::max<int64_t>(1, std::min<int64_t>((p + 255) / 256, sms));
+    b.Bh = (int)std::max<int64_t>(1, std::min<int64_t>((p + 63) / 64, sms));
     b.rph = std::max<int64_t>(1, (p + b.Bh - 1) / b.Bh);
-    b.gy = (int)cdiv((int64_t)r * (r + 1), (int64_t)kT * kPPT);
-    b.gx_obj = (int)std::max<int64_t>(1, (p + 63) / 64);
-    b.gy_obj = (int)std::max<int64_t>(1, (n + 63) / 64);
-    const int npairs = r * (r + 1);
+    b.gy = (int)cdiv(wide_pairs(r), kBlockPairs);
+    b.gx_obj = (int)std::max<int64_t>(1, (p + kWhCols - 1) / kWhCols);
+    b.gy_obj = (int)std::max<int64_t>(1, (n + kWhRows - 1) / kWhRows);
     const size_t d = sizeof(double);
     const size_t nr = (size_t)n * r, pr = (size_t)p * r;
     const std::vector<size_t> sizes = {
-        d * nr, d * pr, d * pr, d * nr, d * pr, d * nr, d * pr,
-        d * (size_t)std::max(b.Bw, b.Bh) * npairs,
+        d * nr, d * pr, d * pr, d * nr, d * pr,
+        d * (size_t)std::max(b.Bw, b.Bh) * wide_pairs(r) * 64,
         d * r * r, d * r, d * r * r, d * r, d * r * r, d * r,
         d * (size_t)b.gx_obj * b.gy_obj};
     size_t total = 0;
     for (size_t z : sizes) total += align256(std::max<size_t>(z, 1));
     void *base = nullptr;
     NMFCU_TRY(nmfcu_internal::context_buffer(c, kSlotBuf, total, &base));
-    double **dst[] = {&b.W, &b.H, &b.Ht, &b.NW, &b.NH, &b.Wn, &b.Hn, &b.part, &b.Gw, &b.sw,
+    double **dst[] = {&b.W, &b.H, &b.Ht, &b.NW, &b.NH, &b.part, &b.Gw, &b.sw,
                       &b.Gh, &b.sh, &b.Gw2, &b.sw2, &b.opart};
     char *q = static_cast<char *>(base);
     for (size_t i = 0; i < sizes.size(); i++) {
