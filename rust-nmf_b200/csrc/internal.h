@@ -44,7 +44,7 @@ nmfcu_status default_context(int device, nmfcu_context **out);
 // 0..25, one owner per slot; the contents survive between calls).  Owners:
 // 0..12, 16, 17 batch.cu; 13..15 linkage.cu; 18..23 sparse.cu (serve.cu
 // uses the slots of its own contexts).
-constexpr int kContextSlots = 26;
+constexpr int kContextSlots = 27;
 nmfcu_status context_buffer(nmfcu_context *c, int slot, size_t bytes, void **out);
 
 cudaStream_t context_stream(nmfcu_context *c);

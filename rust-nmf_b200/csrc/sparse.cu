@@ -56,6 +56,7 @@ constexpr int kSlotCsc = 19;    // the CSC copy
 constexpr int kSlotSort = 20;   // the radix sort's buffers (CSC build only)
 constexpr int kSlotFac = 21;    // padded W, H, H^T and the two contractions
 constexpr int kSlotSmall = 22;  // Grams, sums, objective partials, state, deviances
+constexpr int kSlotSeg = 26;    // the blocked passes' segments and line ranges
 constexpr int kSlotCheck = 23;  // validation flags of the device entry
 
 inline unsigned cdiv(int64_t a, int64_t b) { return (unsigned)((a + b - 1) / b); }
@@ -199,6 +200,242 @@ __global__ void __launch_bounds__(kT)
     }
 }
 
+// ---------------------------------------------------------------------------
+// The same contraction with the gathered factor rows in shared memory.
+// ---------------------------------------------------------------------------
+// sparse_pass pulls an RP x 8-byte factor row from L2 for every stored entry:
+// 16 GB a pass at 10^8 entries and rank 20, 2.4 ms (plain) and 4.0 ms (ratio).
+// Here a block keeps B consecutive rows of F in shared memory (one bulk copy)
+// and its warps run over the entries that index them, line by line; a line's
+// entries are sorted, so those of one block of F are a segment of it
+// (line_segments).  A block owns a range of lines with about the same number
+// of entries, goes through the blocks of F in order, and adds each segment's
+// sum to the line's (always the same warp, in block order: the same bits from
+// run to run).
+//
+// A warp takes 32 entries at a time, one a lane.  A group of GL lanes goes
+// through its GL entries, each lane with every GL-th pair of the entry's row;
+// W H comes together so that each lane ends with its own entry's, and divides
+// it once.  A fixed butterfly adds the groups at the segment's end.  Bound:
+// shared-memory reads of factor rows at random bank phases, about 2.6 cycles
+// an entry, and at the ratio the latency of its FP64 chain.
+constexpr int kBlkBytes = 200 * 1024;  // of F in shared memory
+template <int RP>
+struct BlkCfg {
+    static constexpr int PAIRS = RP / 2;
+    static constexpr int GL = PAIRS >= 4 ? 4 : PAIRS >= 2 ? 2 : 1;  // lanes of an entry
+    static constexpr int UPL = (PAIRS + GL - 1) / GL;               // pairs of a lane
+    // Warps: as many as the registers of GL rows' pairs leave room for.
+    static constexpr int WARPS = UPL >= 4 ? 12 : 16;
+    static constexpr int ROWS = kBlkBytes / (RP * 8) / 32 * 32;     // rows of F a block
+    static constexpr int SMEM = ROWS * RP * 8 + 16;
+};
+
+// seg[b * lines + m] = entries of line m that index rows below b * rows of F
+// (b = 0 .. blocks).
+__global__ void line_segments(const int64_t *__restrict__ ptr, const int32_t *__restrict__ idx,
+                              int lines, int rows, int blocks, int32_t *__restrict__ seg) {
+    const int64_t total = (int64_t)lines * (blocks + 1);
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
+         t += (int64_t)gridDim.x * blockDim.x) {
+        const int b = (int)(t / lines), m = (int)(t - (int64_t)b * lines);
+        const int64_t t0 = ptr[m], t1 = ptr[m + 1];
+        const int64_t key = (int64_t)b * rows;
+        int64_t lo = t0, hi = t1;
+        while (lo < hi) {
+            const int64_t mid = (lo + hi) >> 1;
+            if (idx[mid] < key)
+                lo = mid + 1;
+            else
+                hi = mid;
+        }
+        seg[t] = (int32_t)(lo - t0);
+    }
+}
+// *unsorted = 1 if a line's indices ever decrease.
+__global__ void lines_sorted(const int64_t *__restrict__ ptr, const int32_t *__restrict__ idx,
+                             int lines, int *__restrict__ unsorted) {
+    const int lane = threadIdx.x & 31;
+    const int gw = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
+    const int nw = (int)(((int64_t)gridDim.x * blockDim.x) >> 5);
+    bool bad = false;
+    for (int m = gw; m < lines; m += nw)
+        for (int64_t t = ptr[m] + lane; t + 1 < ptr[m + 1]; t += 32) bad |= idx[t] > idx[t + 1];
+    if (bad) *unsorted = 1;
+}
+// bound[g] = the first line of block g's range: ranges of equal entries.
+__global__ void line_bounds(const int64_t *__restrict__ ptr, int lines, int64_t nnz, int G,
+                            int *__restrict__ bound) {
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g > G) return;
+    const int64_t key = nnz * g / G;
+    int lo = 0, hi = lines;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (ptr[mid] < key)
+            lo = mid + 1;
+        else
+            hi = mid;
+    }
+    bound[g] = g == G ? lines : lo;
+}
+
+// acc: lines x RP; OUT_KM writes the finished sums to out[k * ldo + m]
+// (otherwise acc is the output).
+template <int RP, bool RATIO, bool OUT_KM>
+__global__ void __launch_bounds__(32 * BlkCfg<RP>::WARPS, 1)
+    sparse_pass_blocked(const int64_t *__restrict__ ptr, const int32_t *__restrict__ idx,
+                        const double *__restrict__ val, const int32_t *__restrict__ seg,
+                        const int *__restrict__ bound, int lines, int64_t ldo,
+                        const double *__restrict__ G, const double *__restrict__ F, int frows,
+                        double *__restrict__ acc_out, double *__restrict__ out, RunState *st) {
+    using C = BlkCfg<RP>;
+    if (nmfcu::run_stopped(st)) return;
+    extern __shared__ __align__(16) unsigned char blk_smem[];
+    double *sF = reinterpret_cast<double *>(blk_smem);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(blk_smem + (size_t)C::ROWS * RP * 8);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int gl = lane % C::GL, slot = lane / C::GL, first = lane - gl;
+    const int m0 = bound[blockIdx.x], m1 = bound[blockIdx.x + 1];
+    const int blocks = (frows + C::ROWS - 1) / C::ROWS;
+    if (threadIdx.x == 0) {
+        nmfcu::mbar_init(bar, 1);
+        nmfcu::fence_mbar_init();
+    }
+    for (int b = 0; b < blocks; b++) {
+        __syncthreads();  // everyone is done with the last block of F (and sees the barrier)
+        const int x0 = b * C::ROWS, nx = min(C::ROWS, frows - x0);
+        if (threadIdx.x == 0) {
+            nmfcu::fence_proxy_async_smem();
+            const uint32_t bytes = (uint32_t)nx * RP * 8;
+            nmfcu::mbar_expect_tx(bar, bytes);
+            asm volatile(
+                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, "
+                "[%3];" ::"r"(nmfcu::smem_u32(sF)),
+                "l"(F + (size_t)x0 * RP), "r"(bytes), "r"(nmfcu::smem_u32(bar))
+                : "memory");
+        }
+        if (!nmfcu::mbar_wait(bar, (uint32_t)(b & 1))) {
+            nmfcu::record_timeout(st, nmfcu::TIMEOUT_FULL);
+            return;
+        }
+        const int32_t *s0 = seg + (size_t)b * lines, *s1 = s0 + lines;
+        // The next line's segment is read while this one is worked on.
+        int m = m0 + warp;
+        int64_t nt0 = 0, nt1 = 0;
+        const auto segment = [&](int l) {
+            nt0 = nt1 = 0;
+            if (l < m1) {
+                const int64_t base = ptr[l];
+                nt0 = base + s0[l];
+                nt1 = base + s1[l];
+            }
+        };
+        segment(m);
+        for (; m < m1; m += C::WARPS) {
+            const int64_t t0 = nt0, t1 = nt1;
+            double2 g[RATIO ? C::UPL : 1], a[C::UPL];
+            int xo;
+            double vo;
+            const auto entry = [&](int64_t t) {
+                xo = t + lane < t1 ? idx[t + lane] - x0 : -1;
+                vo = t + lane < t1 ? val[t + lane] : 0.0;
+            };
+            entry(t0);
+#pragma unroll
+            for (int u = 0; u < C::UPL; u++) {
+                const int pr = gl + C::GL * u;
+                a[u] = make_double2(0.0, 0.0);
+                if (RATIO)
+                    g[u] = pr < C::PAIRS
+                               ? reinterpret_cast<const double2 *>(G + (int64_t)m * RP)[pr]
+                               : make_double2(0.0, 0.0);
+            }
+            segment(m + C::WARPS);
+            for (int64_t t = t0; t < t1; t += 32) {
+                // The group's entries side by side.
+                double2 f[C::GL][C::UPL];
+#pragma unroll
+                for (int q = 0; q < C::GL; q++) {
+                    const int x = __shfl_sync(0xffffffffu, xo, first + q);
+                    const double2 *row =
+                        reinterpret_cast<const double2 *>(sF + (size_t)max(x, 0) * RP);
+#pragma unroll
+                    for (int u = 0; u < C::UPL; u++) {
+                        const int pr = gl + C::GL * u;
+                        f[q][u] = pr < C::PAIRS && x >= 0 ? row[pr] : make_double2(0.0, 0.0);
+                    }
+                }
+                double w = vo;
+                if (t + 32 < t1) entry(t + 32);
+                if (RATIO) {
+                    double wh[C::GL];
+#pragma unroll
+                    for (int q = 0; q < C::GL; q++) wh[q] = 0.0;
+#pragma unroll
+                    for (int u = 0; u < C::UPL; u++)
+#pragma unroll
+                        for (int q = 0; q < C::GL; q++)
+                            wh[q] = fma(g[u].y, f[q][u].y, fma(g[u].x, f[q][u].x, wh[q]));
+                    // Each lane ends with the sum of its own entry: halves of
+                    // the list change places with the other half of the group.
+#pragma unroll
+                    for (int o = C::GL / 2; o >= 1; o >>= 1) {
+                        const bool hi = (gl & o) != 0;
+#pragma unroll
+                        for (int q = 0; q < o; q++) {
+                            const double keep = hi ? wh[q + o] : wh[q];
+                            const double give = hi ? wh[q] : wh[q + o];
+                            wh[q] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                        }
+                    }
+                    w = (wh[0] != 0.0) ? nmfcu::ratio_div(w, wh[0]) : 0.0;
+                }
+#pragma unroll
+                for (int q = 0; q < C::GL; q++) {
+                    const double wq = __shfl_sync(0xffffffffu, w, first + q);
+#pragma unroll
+                    for (int u = 0; u < C::UPL; u++) {
+                        a[u].x = fma(wq, f[q][u].x, a[u].x);
+                        a[u].y = fma(wq, f[q][u].y, a[u].y);
+                    }
+                }
+            }
+            double2 old[C::UPL];
+#pragma unroll
+            for (int u = 0; u < C::UPL; u++) {
+                const int pr = gl + C::GL * u;
+                old[u] = b > 0 && slot == 0 && pr < C::PAIRS
+                             ? reinterpret_cast<const double2 *>(acc_out + (int64_t)m * RP)[pr]
+                             : make_double2(0.0, 0.0);
+            }
+#pragma unroll
+            for (int u = 0; u < C::UPL; u++)
+#pragma unroll
+                for (int o = C::GL; o < 32; o <<= 1) {
+                    a[u].x += __shfl_xor_sync(0xffffffffu, a[u].x, o);
+                    a[u].y += __shfl_xor_sync(0xffffffffu, a[u].y, o);
+                }
+            if (slot == 0) {
+                double2 *dst = reinterpret_cast<double2 *>(acc_out + (int64_t)m * RP);
+#pragma unroll
+                for (int u = 0; u < C::UPL; u++) {
+                    const int pr = gl + C::GL * u;
+                    if (pr >= C::PAIRS) continue;
+                    a[u].x += old[u].x;
+                    a[u].y += old[u].y;
+                    if (OUT_KM && b == blocks - 1) {
+                        out[(int64_t)(2 * pr) * ldo + m] = a[u].x;
+                        out[(int64_t)(2 * pr + 1) * ldo + m] = a[u].y;
+                    } else {
+                        dst[pr] = a[u];
+                    }
+                }
+            }
+        }
+    }
+}
+
 // Stored-entry part of the objective, one warp a CSR row; per block two
 // partials: part[2 b] the stored terms, part[2 b + 1] (KL) the sum of W H
 // over the stored entries with v > 0.
@@ -315,10 +552,14 @@ struct SparseV {
     int32_t *cidx;
     double *cval;
     int64_t nnz;
+    // The blocked passes' segments and line ranges (null: the pass gathers
+    // from L2): rows against blocks of H^T, columns against blocks of W.
+    int32_t *rseg = nullptr, *cseg = nullptr;
+    int *rbound = nullptr, *cbound = nullptr;
 };
 
 struct Work {
-    double *W, *H, *Ht, *numW, *numH;          // padded factors, contractions
+    double *W, *H, *Ht, *numW, *numH, *accH;   // padded factors, contractions
     double *pg, *Gw, *sw, *Gh, *sh, *Gw2, *sw2;
     double *opart, *obj, *dev;
     RunState *st;
@@ -396,6 +637,15 @@ struct Loop {
     cudaStream_t s;
     int sms;
 
+    template <bool RATIO, bool OUT_KM>
+    void blocked(const int64_t *ptr, const int32_t *idx, const double *val, const int32_t *seg,
+                 const int *bound, int lines, const double *G, const double *F, int frows,
+                 double *acc, double *out) {
+        auto *k = sparse_pass_blocked<RP, RATIO, OUT_KM>;
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, BlkCfg<RP>::SMEM);
+        k<<<sms, 32 * BlkCfg<RP>::WARPS, BlkCfg<RP>::SMEM, s>>>(ptr, idx, val, seg, bound, lines, lines, G, F,
+                                                     frows, acc, out, w.st);
+    }
     // H^T of an H the last epilogue did not write.
     void transpose_h() {
         if (p <= 0) return;
@@ -443,6 +693,14 @@ struct Loop {
     void h_step(bool ratio, const EpiParams &e, const nmfcu::GramOut &g) {
         {
             nmfcu_internal::TimedScope sc(c, s, NMFCU_KCLASS_HSTEP);
+            if (sv.cseg) {
+                if (ratio)
+                    blocked<true, true>(sv.cptr, sv.cidx, sv.cval, sv.cseg, sv.cbound, p, w.Ht,
+                                        w.W, n, w.accH, w.numH);
+                else
+                    blocked<false, true>(sv.cptr, sv.cidx, sv.cval, sv.cseg, sv.cbound, p, nullptr,
+                                         w.W, n, w.accH, w.numH);
+            } else {
             const unsigned grid = line_grid(p, sms);
             if (ratio)
                 sparse_pass<RP, true, true><<<grid, kT, 0, s>>>(sv.cptr, sv.cidx, sv.cval, p, p, w.Ht,
@@ -450,6 +708,7 @@ struct Loop {
             else
                 sparse_pass<RP, false, true><<<grid, kT, 0, s>>>(sv.cptr, sv.cidx, sv.cval, p, p,
                                                               nullptr, w.W, w.numH, w.st);
+            }
         }
         nmfcu_internal::TimedScope sc(c, s, NMFCU_KCLASS_OTHER);
         nmfcu::launch_h_epilogue<RP, double, RP>(w.H, w.Ht, p, w.numH, one_slot(), std::max(p, 1),
@@ -458,6 +717,14 @@ struct Loop {
     void w_step(bool ratio, const EpiParams &e, const nmfcu::GramOut &g) {
         {
             nmfcu_internal::TimedScope sc(c, s, NMFCU_KCLASS_WSTEP);
+            if (sv.rseg) {
+                if (ratio)
+                    blocked<true, false>(sv.rptr, sv.ridx, sv.rval, sv.rseg, sv.rbound, n, w.W,
+                                         w.Ht, p, w.numW, nullptr);
+                else
+                    blocked<false, false>(sv.rptr, sv.ridx, sv.rval, sv.rseg, sv.rbound, n,
+                                          nullptr, w.Ht, p, w.numW, nullptr);
+            } else {
             const unsigned grid = line_grid(n, sms);
             if (ratio)
                 sparse_pass<RP, true, false><<<grid, kT, 0, s>>>(sv.rptr, sv.ridx, sv.rval, n, 0, w.W,
@@ -465,6 +732,7 @@ struct Loop {
             else
                 sparse_pass<RP, false, false><<<grid, kT, 0, s>>>(sv.rptr, sv.ridx, sv.rval, n, 0,
                                                                nullptr, w.Ht, w.numW, w.st);
+            }
         }
         nmfcu_internal::TimedScope sc(c, s, NMFCU_KCLASS_OTHER);
         nmfcu::launch_w_epilogue<RP>(w.W, n, w.numW, one_slot(), std::max(n, 1), e, g, w.gw, w.st,
@@ -558,12 +826,14 @@ nmfcu_status make_work(nmfcu_context *c, int64_t n, int64_t p, int RP, int64_t m
     const int sms = nmfcu_internal::context_sms(c);
     std::vector<void *> b;
     const size_t d = sizeof(double);
-    NMFCU_TRY(carve(c, kSlotFac, {d * n * RP, d * RP * p, d * p * RP, d * n * RP, d * RP * p}, b));
+    NMFCU_TRY(carve(c, kSlotFac,
+                    {d * n * RP, d * RP * p, d * p * RP, d * n * RP, d * RP * p, d * RP * p}, b));
     w.W = static_cast<double *>(b[0]);
     w.H = static_cast<double *>(b[1]);
     w.Ht = static_cast<double *>(b[2]);
     w.numW = static_cast<double *>(b[3]);
     w.numH = static_cast<double *>(b[4]);
+    w.accH = static_cast<double *>(b[5]);
     w.gw = nmfcu::gram_plan(n, nmfcu::kTileRows, sms);
     w.gh = nmfcu::gram_plan(p, nmfcu::kTileCols, sms);
     w.Bo = (int)line_grid(n, sms);
@@ -587,10 +857,60 @@ nmfcu_status make_work(nmfcu_context *c, int64_t n, int64_t p, int RP, int64_t m
     return NMFCU_OK;
 }
 
+// Entries of an average segment from which the blocked passes run: a segment
+// costs a warp its line's pointers, factor row and sum (about as much as 16
+// entries), which a few entries do not pay for.
+constexpr int64_t kBlkEntries = 16;
+
+// Segments and line ranges of the blocked passes, for the passes that take
+// them (lines sorted, enough entries a segment).
+template <int RP>
+nmfcu_status plan_blocked(nmfcu_context *c, int64_t n, int64_t p, SparseV &sv, cudaStream_t s) {
+    using C = BlkCfg<RP>;
+    if (n <= 0 || p <= 0 || sv.nnz <= 0) return NMFCU_OK;
+    const int rb = (int)cdiv(p, C::ROWS), cb = (int)cdiv(n, C::ROWS);
+    const bool rows = sv.nnz >= kBlkEntries * n * rb, cols = sv.nnz >= kBlkEntries * p * cb;
+    if (!rows && !cols) return NMFCU_OK;
+    const int sms = nmfcu_internal::context_sms(c);
+    std::vector<void *> b;
+    NMFCU_TRY(carve(c, kSlotSeg,
+                    {rows ? sizeof(int32_t) * (size_t)n * (rb + 1) : 0,
+                     cols ? sizeof(int32_t) * (size_t)p * (cb + 1) : 0, sizeof(int) * (sms + 1),
+                     sizeof(int) * (sms + 1), sizeof(int)},
+                    b));
+    int *unsorted = static_cast<int *>(b[4]);
+    NMFCU_CUDA_TRY(cudaMemsetAsync(unsorted, 0, sizeof(int), s));
+    nmfcu_internal::TimedScope sc(c, s, NMFCU_KCLASS_OTHER, 5);
+    lines_sorted<<<(unsigned)sms * 16, kT, 0, s>>>(sv.rptr, sv.ridx, (int)n, unsorted);
+    int hu = 0;
+    NMFCU_CUDA_TRY(cudaMemcpyAsync(&hu, unsorted, sizeof(int), cudaMemcpyDeviceToHost, s));
+    NMFCU_CUDA_TRY(cudaStreamSynchronize(s));
+    if (hu) return NMFCU_OK;  // (the CSC copy of such a CSR is sorted, but is not needed alone)
+    const auto plan = [&](const int64_t *ptr, const int32_t *idx, int64_t lines, int blocks,
+                          int32_t *seg, int *bound) {
+        line_segments<<<std::min<unsigned>(cdiv(lines * (blocks + 1), kT), (unsigned)sms * 32), kT,
+                        0, s>>>(ptr, idx, (int)lines, C::ROWS, blocks, seg);
+        line_bounds<<<cdiv(sms + 1, kT), kT, 0, s>>>(ptr, (int)lines, sv.nnz, sms, bound);
+    };
+    if (rows) {
+        sv.rseg = static_cast<int32_t *>(b[0]);
+        sv.rbound = static_cast<int *>(b[2]);
+        plan(sv.rptr, sv.ridx, n, rb, sv.rseg, sv.rbound);
+    }
+    if (cols) {
+        sv.cseg = static_cast<int32_t *>(b[1]);
+        sv.cbound = static_cast<int *>(b[3]);
+        plan(sv.cptr, sv.cidx, p, cb, sv.cseg, sv.cbound);
+    }
+    NMFCU_CUDA_TRY(cudaGetLastError());
+    return NMFCU_OK;
+}
+
 template <int RP>
 nmfcu_status run_loop_t(nmfcu_context *c, const nmfcu_options *o, int64_t n, int64_t p, int64_t r,
                         SparseV sv, Work w, cudaStream_t s, bool stat, int64_t *n_dev,
                         int64_t *n_iter) {
+    NMFCU_TRY(plan_blocked<RP>(c, n, p, sv, s));
     Loop<RP> L{c, o, (int)n, (int)p, (int)r, sv, w, s, nmfcu_internal::context_sms(c)};
     NMFCU_CUDA_TRY(cudaMemsetAsync(w.st, 0, sizeof(RunState), s));
     L.transpose_h();
@@ -604,6 +924,9 @@ nmfcu_status run_loop_t(nmfcu_context *c, const nmfcu_options *o, int64_t n, int
     NMFCU_CUDA_TRY(cudaMemcpyAsync(&hs, w.st, sizeof(RunState), cudaMemcpyDeviceToHost, s));
     NMFCU_CUDA_TRY(cudaStreamSynchronize(s));
     nmfcu_internal::drain_timing(c);
+    if (hs.timeout != 0)
+        return fail(NMFCU_ERR_TIMEOUT, "a sparse pass gave up waiting for its copies (code " +
+                                           std::to_string(hs.timeout) + ")");
     if (hs.error == 1)
         return fail(NMFCU_ERR_INVALID_ARG,
                     "check_interval must be > 0 (the stationary stop evaluates iter % check_interval)");
