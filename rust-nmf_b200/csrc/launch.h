@@ -102,6 +102,6 @@ int tcr_concat_rank(int rank);
 // bf16 in the tile layout ([Th Th Th Tm Tm Tl], blocks of R) and the unit
 // layout ([Fh Fm Fl Fh Fm Fh]), zero-padded; either output may be null.
 void tcr_split_factor(const double *F, int64_t fk, int64_t fx, int R, int K, int64_t xpad,
-                      void *tile, void *unit, const RunState *st, int sms, cudaStream_t s);
+                      void *tile, void *unit, const RunState *st, cudaStream_t s);
 
 }  // namespace nmfcu

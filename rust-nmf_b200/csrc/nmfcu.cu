@@ -794,10 +794,8 @@ nmfcu_status h_step(nmfcu_context *c, const RunArgs &a, const PassSet &ps, const
         const TcrTerms x = tcr_terms(c, ps, pl.r);
         {
             nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER);
-            tcr_split_factor(a.W, 1, pl.RP, pl.r, pl.n, ps.xpadW, nullptr, x.w_unit, st, c->sms,
-                             s);
-            tcr_split_factor(a.H, pl.p, 1, pl.r, pl.p, ps.xpadH, x.h_tile, nullptr, st, c->sms,
-                             s);
+            tcr_split_factor(a.W, 1, pl.RP, pl.r, pl.n, ps.xpadW, nullptr, x.w_unit, st, s);
+            tcr_split_factor(a.H, pl.p, 1, pl.r, pl.p, ps.xpadH, x.h_tile, nullptr, st, s);
         }
         if (sk.G > 0) {
             nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_HSTEP);
@@ -864,10 +862,8 @@ nmfcu_status w_step(nmfcu_context *c, const RunArgs &a, const PassSet &ps, const
         const TcrTerms x = tcr_terms(c, ps, pl.r);
         {
             nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER);
-            tcr_split_factor(a.H, pl.p, 1, pl.r, pl.p, ps.xpadH, nullptr, x.h_unit, st, c->sms,
-                             s);
-            tcr_split_factor(a.W, 1, pl.RP, pl.r, pl.n, ps.xpadW, x.w_tile, nullptr, st, c->sms,
-                             s);
+            tcr_split_factor(a.H, pl.p, 1, pl.r, pl.p, ps.xpadH, nullptr, x.h_unit, st, s);
+            tcr_split_factor(a.W, 1, pl.RP, pl.r, pl.n, ps.xpadW, x.w_tile, nullptr, st, s);
         }
         if (sk.G > 0) {
             nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_WSTEP);
@@ -1538,8 +1534,10 @@ nmfcu_status make_f32(nmfcu_context *c, const double *V64, int64_t ldv64, int64_
     const int64_t ld = std::max<int64_t>(32, round_up(p, 32));
     NMF_TRY(c->V32.ensure(sizeof(float) * (size_t)(n * ld)));
     if (n > 0 && p > 0) {
-        const unsigned blocks = std::min<unsigned>(cdiv(n * p, kThreads), (unsigned)c->sms * 16);
-        convert_f64_f32<<<blocks, kThreads, 0, s>>>(V64, ldv64, c->V32.as<float>(), ld, (int)n, (int)p);
+        const bool aligned = reinterpret_cast<uintptr_t>(V64) % 16 == 0 && ldv64 % 2 == 0;
+        const dim3 grid(cdiv(p, 4 * kThreads), (unsigned)std::min<int64_t>(n, 65535));
+        convert_f64_f32<<<grid, kThreads, 0, s>>>(V64, ldv64, c->V32.as<float>(), ld, (int)n,
+                                                  (int)p, aligned);
         CUDA_TRY(cudaGetLastError());
     }
     *ldv32 = ld;

@@ -25,29 +25,68 @@ __device__ __forceinline__ void split3(double f, __nv_bfloat16 &h, __nv_bfloat16
 // k < R) holds term tile_term[b] of F(k, x) in `tile` and term unit_term[b]
 // in `unit`; everything else (x >= K, positions >= 6 R) is zero.  Either
 // output may be null.
-__global__ void split_factor_concat(const double *__restrict__ F, int64_t fk, int64_t fx, int R,
-                                    int K, int KC, int64_t xpad,
-                                    __nv_bfloat16 *__restrict__ tile,
-                                    __nv_bfloat16 *__restrict__ unit, const RunState *st) {
+//
+// A block takes kSplitRows rows x: their R x kSplitRows values come in
+// contiguously, are split once, and the rows go out 16 bytes a thread.  Bound:
+// the rows' store.  (One thread an element, which read F strided by the
+// rank's pitch and split it anew for each of its positions, took 42 us a
+// launch, W and H on average, at 20000 x 60000 rank 20; this takes 10.)
+constexpr int kSplitRows = 64;
+constexpr int kSplitLd = kSplitRows + 2;
+__global__ void __launch_bounds__(256)
+    split_factor_concat(const double *__restrict__ F, int64_t fk, int64_t fx, int R, int K, int KC,
+                        int64_t xpad, __nv_bfloat16 *__restrict__ tile,
+                        __nv_bfloat16 *__restrict__ unit, const RunState *st) {
     if (run_stopped(st)) return;
-    const int64_t total = xpad * KC;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += stride) {
-        const int64_t x = t / KC;
-        const int p = (int)(t - x * KC);
-        __nv_bfloat16 vt = __float2bfloat16(0.f), vu = vt;
-        if (x < K && p < 6 * R) {
-            const int blk = p / R, k = p - blk * R;
-            __nv_bfloat16 th[3];
-            split3(F[k * fk + x * fx], th[0], th[1], th[2]);
-            // Products Th Fh, Th Fm, Th Fl, Tm Fh, Tm Fm, Tl Fh.
-            constexpr int tile_term[6] = {0, 0, 0, 1, 1, 2};
-            constexpr int unit_term[6] = {0, 1, 2, 0, 1, 0};
-            vt = th[tile_term[blk]];
-            vu = th[unit_term[blk]];
+    __shared__ __nv_bfloat16 terms[3][32][kSplitLd];
+    // For the block's 8-position chunks: where each position's term is.
+    __shared__ short from_tile[192], from_unit[192];
+    const int64_t x0 = (int64_t)blockIdx.x * kSplitRows;
+    if (threadIdx.x < KC) {
+        // Products Th Fh, Th Fm, Th Fl, Tm Fh, Tm Fm, Tl Fh.
+        constexpr int tile_term[6] = {0, 0, 0, 1, 1, 2};
+        constexpr int unit_term[6] = {0, 1, 2, 0, 1, 0};
+        const int p = threadIdx.x, blk = p / R, k = p - blk * R;
+        const bool in = p < 6 * R;
+        from_tile[p] = in ? (short)((tile_term[in ? blk : 0] * 32 + k) * kSplitLd) : (short)-1;
+        from_unit[p] = in ? (short)((unit_term[in ? blk : 0] * 32 + k) * kSplitLd) : (short)-1;
+    }
+    for (int e = threadIdx.x; e < R * kSplitRows; e += 256) {
+        int k, u;
+        if (fx == 1) {  // H: neighbours along x
+            k = e / kSplitRows;
+            u = e - k * kSplitRows;
+        } else {  // W: neighbours along k
+            u = e / R;
+            k = e - u * R;
         }
-        if (tile) tile[t] = vt;
-        if (unit) unit[t] = vu;
+        const int64_t x = x0 + u;
+        split3(x < K ? F[k * fk + x * fx] : 0.0, terms[0][k][u], terms[1][k][u], terms[2][k][u]);
+    }
+    __syncthreads();
+    const __nv_bfloat16 *flat = &terms[0][0][0];
+    const int chunks = KC / 8;
+    for (int e = threadIdx.x; e < kSplitRows * chunks; e += 256) {
+        const int u = e / chunks, c = e - u * chunks;
+        if (x0 + u >= xpad) continue;
+        __align__(16) __nv_bfloat16 v[8];
+        const int64_t at = (x0 + u) * KC + 8 * c;
+        if (tile) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int f = from_tile[8 * c + i];
+                v[i] = f >= 0 ? flat[f + u] : __float2bfloat16(0.f);
+            }
+            *reinterpret_cast<uint4 *>(tile + at) = *reinterpret_cast<const uint4 *>(v);
+        }
+        if (unit) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int f = from_unit[8 * c + i];
+                v[i] = f >= 0 ? flat[f + u] : __float2bfloat16(0.f);
+            }
+            *reinterpret_cast<uint4 *>(unit + at) = *reinterpret_cast<const uint4 *>(v);
+        }
     }
 }
 
@@ -90,11 +129,9 @@ cudaError_t tcr_pass_launch(bool hpass, const CUtensorMap &v, const void *t,
 }
 
 void tcr_split_factor(const double *F, int64_t fk, int64_t fx, int R, int K, int64_t xpad,
-                      void *tile, void *unit, const RunState *st, int sms, cudaStream_t s) {
+                      void *tile, void *unit, const RunState *st, cudaStream_t s) {
     const int KC = tcr_concat_rank(R);
-    const int64_t work = xpad * KC;
-    const unsigned blocks =
-        (unsigned)std::max<int64_t>(1, std::min<int64_t>((work + 255) / 256, (int64_t)sms * 8));
+    const unsigned blocks = (unsigned)((xpad + tcr::kSplitRows - 1) / tcr::kSplitRows);
     tcr::split_factor_concat<<<blocks, 256, 0, s>>>(F, fk, fx, R, K, KC, xpad,
                                                     static_cast<__nv_bfloat16 *>(tile),
                                                     static_cast<__nv_bfloat16 *>(unit), st);
