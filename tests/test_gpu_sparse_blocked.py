@@ -90,3 +90,43 @@ def test_unsorted_rows(method):
         _native._ptr(W0), _native._ptr(H0), _native._ptr(W), _native._ptr(H), None, 0,
         ctypes.byref(nd), ctypes.byref(ni)))
     assert rel_max(W, want.W) <= TOL and rel_max(H, want.H) <= TOL
+
+
+# Above 2^22 entries the CSC copy is made by 128 x 2048 tiles, 256 columns of
+# one at a time: one row and a few columns past whole tiles; nearly full ones,
+# whose sub-tiles hold more entries than their lists; rows of one tile.
+@pytest.mark.parametrize("n,p,density", [(2177, 4099, 0.5), (1500, 3300, 0.9), (100, 50001, 0.9),
+                                         (40001, 300, 0.4)])
+def test_csc_tiles(oracle, n, p, density):
+    V, W0, H0 = _inputs(n, p, 3, density, n + p)
+    assert np.count_nonzero(V) > 1 << 22
+    _check(oracle, "lee", V, W0, H0, iters=2)
+
+
+@pytest.mark.parametrize("n,p", [(127, 2047), (1, 300), (700, 3)])
+def test_csc_sort(oracle, n, p):
+    V, W0, H0 = _inputs(n, p, 3, 0.15, n + p)
+    V[0, 0] = V[-1, -1] = 1.0
+    _check(oracle, "lee", V, W0, H0)
+
+
+def test_repeated_entries():
+    """Two stored entries of one place count as their sum (lee: linear in V)."""
+    n, p, r = 300, 500, 4
+    V, W0, H0 = _inputs(n, p, r, 0.2, 4)
+    M = sp.csr_matrix(V)
+    want = nmf_rs.nmf(M, r, "lee", W0=W0, H0=H0, max_iter=3)
+    ptr = (2 * M.indptr).astype(np.int64)
+    idx = np.repeat(M.indices, 2).astype(np.int32)
+    dat = np.repeat(M.data / 2, 2)
+    o = _native.default_options()
+    o.method = _native.parse_method("lee")
+    o.max_iter = 3
+    W, H = np.empty_like(W0), np.empty_like(H0)
+    nd, ni = ctypes.c_int64(0), ctypes.c_int64(0)
+    _native.check(_native.load().nmfcu_run_csr(
+        ctypes.byref(o), n, p, r, dat.size, ptr.ctypes.data_as(_native._i64p),
+        idx.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)), _native._ptr(dat),
+        _native._ptr(W0), _native._ptr(H0), _native._ptr(W), _native._ptr(H), None, 0,
+        ctypes.byref(nd), ctypes.byref(ni)))
+    assert rel_max(W, want.W) <= TOL and rel_max(H, want.H) <= TOL
