@@ -57,54 +57,6 @@ __device__ __forceinline__ bool run_stopped(const RunState *st) {
     return st != nullptr && st->stopped != 0;
 }
 
-// Chained launches.  A small iteration is four to six kernels of a few
-// microseconds, and a plain launch starts only when the kernel before it has
-// drained.  A chained one (programmatic stream serialization) may start as
-// soon as every block of the kernel before has called chain_next() or ended.
-// Its chain_wait() returns when that kernel is complete and its writes are
-// visible; what a kernel does before it may touch only what the kernel before
-// does not write.  Every chained kernel calls chain_wait() in every thread,
-// and chain_next() only after it, so that when a kernel starts all but the
-// one before it are complete.  In a plain launch both do nothing.
-// Brunet 200 x 60 at rank 5: 22 -> 17 us an iteration; lee 1500 x 3000 at rank
-// 8: 38 -> 36; brunet 2000 x 7750 at rank 10: 120 -> 116.
-__device__ __forceinline__ void chain_wait() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-__device__ __forceinline__ void chain_next() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
-// While one lives with on = true, this thread's launch_chained launches are
-// chained: the kernels before them in the stream must be the run's own.
-struct ChainLaunches {
-    static bool &active() {
-        static thread_local bool on = false;
-        return on;
-    }
-    const bool before;
-    explicit ChainLaunches(bool on) : before(active()) { active() = on; }
-    ~ChainLaunches() { active() = before; }
-    ChainLaunches(const ChainLaunches &) = delete;
-    ChainLaunches &operator=(const ChainLaunches &) = delete;
-};
-
-template <typename... P, typename... A>
-inline cudaError_t launch_chained(void (*kern)(P...), unsigned grid, unsigned block, size_t smem,
-                                  cudaStream_t s, A &&...args) {
-    cudaLaunchAttribute attr = {};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cfg.attrs = &attr;
-    cfg.numAttrs = ChainLaunches::active() ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
-}
-
 // ---------------------------------------------------------------------------
 // Arithmetic helpers
 // ---------------------------------------------------------------------------
@@ -814,9 +766,7 @@ struct GramAcc {
 template <int RP, int THREADS>
 __global__ void __launch_bounds__(THREADS)
     gram_w_tiles(const double *__restrict__ W, int n, GramOut g, const RunState *st) {
-    chain_wait();
     if (run_stopped(st)) return;
-    chain_next();
     constexpr bool FEW = THREADS == kEpiThreads;
     using GA = GramAcc<RP, THREADS, FEW ? kTileRows / 4 : THREADS / 32>;
     extern __shared__ double scratch[];
@@ -845,9 +795,7 @@ __global__ void __launch_bounds__(THREADS)
 template <int RP, int THREADS>
 __global__ void __launch_bounds__(THREADS)
     gram_h_tiles(const double *__restrict__ H, int p, GramOut g, const RunState *st) {
-    chain_wait();
     if (run_stopped(st)) return;
-    chain_next();
     constexpr bool FEW = THREADS == kEpiThreads;
     using GA = GramAcc<RP, THREADS, FEW ? kTileCols / 4 : THREADS / 32>;
     extern __shared__ double scratch[];
@@ -875,9 +823,7 @@ __global__ void __launch_bounds__(THREADS)
 template <int RP>
 __global__ void col_rescale(double *__restrict__ W, int n, int r, const double *__restrict__ sums,
                             const RunState *st) {
-    chain_wait();
     if (run_stopped(st)) return;
-    chain_next();
     __shared__ double s[RP];
     if (threadIdx.x < RP) s[threadIdx.x] = sums[threadIdx.x];
     __syncthreads();
@@ -896,9 +842,7 @@ template <int RP>
 __global__ void dnmf_rescale(double *__restrict__ W, double *__restrict__ H, int n, int p, int r,
                              const double *__restrict__ Gw, const double *__restrict__ Gh,
                              const RunState *st) {
-    chain_wait();
     if (run_stopped(st)) return;
-    chain_next();
     __shared__ double nw[RP], nh[RP], dk[RP];
     if (threadIdx.x < RP) {
         const int k = threadIdx.x;
@@ -929,9 +873,7 @@ __global__ void dnmf_rescale(double *__restrict__ W, double *__restrict__ H, int
 template <int RP>
 __global__ void clamp_wh(double *__restrict__ W, double *__restrict__ H, int n, int p, int r,
                          double eps, const RunState *st) {
-    chain_wait();
     if (run_stopped(st)) return;
-    chain_next();
     const int64_t tw = (int64_t)n * RP;
     const int64_t th = (int64_t)r * p;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -995,9 +937,7 @@ __global__ void __launch_bounds__(kThreads)
 
 static __global__ void objective_finalize(const double *__restrict__ part, int B, double *__restrict__ dev,
                                    StopParams sp, RunState *st) {
-    chain_wait();
     if (st->stopped) return;
-    chain_next();
     __shared__ double red[kThreads];
     const int tid = threadIdx.x;
     double a = 0.0;

@@ -170,19 +170,19 @@ struct OpsT final : Ops {
                  cudaStream_t s) const override {
         if (n <= 0) return;
         const unsigned blocks = std::min<unsigned>(cdiv((int64_t)n * RP, kThreads), 1184u);
-        launch_chained(col_rescale<RP>, blocks, kThreads, 0, s, W, n, r, sums, st);
+        col_rescale<RP><<<blocks, kThreads, 0, s>>>(W, n, r, sums, st);
     }
     void dnmf_scale(double *W, double *H, int n, int p, int r, const double *Gw,
                     const double *Gh, const RunState *st, cudaStream_t s) const override {
         const int64_t m = std::max<int64_t>((int64_t)n * RP, (int64_t)r * p);
         const unsigned blocks = std::max(1u, std::min<unsigned>(cdiv(m, kThreads), 1184u));
-        launch_chained(dnmf_rescale<RP>, blocks, kThreads, 0, s, W, H, n, p, r, Gw, Gh, st);
+        dnmf_rescale<RP><<<blocks, kThreads, 0, s>>>(W, H, n, p, r, Gw, Gh, st);
     }
     void clamp(double *W, double *H, int n, int p, int r, double eps, const RunState *st,
                cudaStream_t s) const override {
         const int64_t m = std::max<int64_t>((int64_t)n * RP, (int64_t)r * p);
         const unsigned blocks = std::max(1u, std::min<unsigned>(cdiv(m, kThreads), 1184u));
-        launch_chained(clamp_wh<RP>, blocks, kThreads, 0, s, W, H, n, p, r, eps, st);
+        clamp_wh<RP><<<blocks, kThreads, 0, s>>>(W, H, n, p, r, eps, st);
     }
 };
 
@@ -751,8 +751,8 @@ nmfcu_status enqueue_objective(nmfcu_context *c, const RunArgs &a, long long ite
     int count = 0;
     NMF_TRY(enqueue_objective_partials(c, a, s, &count));
     nmfcu_context::Scope sc(c, s, NMFCU_KCLASS_OTHER);
-    CUDA_TRY(launch_chained(objective_finalize, 1, kThreads, 0, s, c->obj.as<double>(), count, a.dev,
-                            stop_params(a.opt, iter), c->state.as<RunState>()));
+    objective_finalize<<<1, kThreads, 0, s>>>(c->obj.as<double>(), count, a.dev,
+                                              stop_params(a.opt, iter), c->state.as<RunState>());
     return NMFCU_OK;
 }
 
@@ -1399,10 +1399,8 @@ nmfcu_status run_graphed(nmfcu_context *c, RunArgs &a, long long refine_from, cu
     cudaGraphExec_t exec = nullptr;
     CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     nmfcu_status st = NMFCU_OK;
-    for (long long k = 0; k < kGraphPeriod && st == NMFCU_OK; k++) {
-        ChainLaunches chain(k > 0);  // (the graph's first kernels have none before them)
+    for (long long k = 0; k < kGraphPeriod && st == NMFCU_OK; k++)
         st = enqueue_iteration(c, a, *it + k, fp64, s);
-    }
     const cudaError_t ec = cudaStreamEndCapture(s, &graph);
     if (st == NMFCU_OK && ec == cudaSuccess && graph &&
         cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess) {
@@ -1441,9 +1439,6 @@ nmfcu_status run_loop(nmfcu_context *c, RunArgs &a, cudaStream_t s, int64_t *n_d
     if (!stat && !c->timing) NMF_TRY(run_graphed(c, a, refine_from, s, &it));
     for (; it <= o->max_iter; it++) {
         const bool fp64 = (o->precision == NMFCU_PREC_FP64) || (it > refine_from);
-        // (Not the first iteration, which may follow a copy or a clear, nor
-        // with events between the launches.)
-        ChainLaunches chain(it > 1 && !c->timing);
         NMF_TRY(enqueue_iteration(c, a, it, fp64, s));
         if (stat) NMF_TRY(enqueue_objective(c, a, it, s));
     }

@@ -247,49 +247,6 @@ __device__ __forceinline__ void release_stage(unsigned char *smem, uint64_t *ful
     }
 }
 
-// The start of a pass: its barriers and its first stages' copies, and between
-// V's and the factor's the wait for the kernels before it.  V is written
-// before the loop and never in it, so a chained pass fetches its first units
-// of V while the kernel before drains.  Leaves `ahead` at the unit STAGES
-// after the first.  False: the run has stopped, and nothing is in flight (a
-// stop is for good, so a pass that sees it early fetches nothing).
-template <int STAGES, int STAGE_BYTES, int TX_BYTES, typename IssueV, typename IssueF>
-__device__ __forceinline__ bool fill_stages(unsigned char *smem, uint64_t *full, int *arrivals,
-                                            long long nunits, UnitCursor &ahead,
-                                            const StreamK &sk, RunState *st, IssueV &&issue_v,
-                                            IssueF &&issue_f) {
-    const bool producer = threadIdx.x == 0;
-    UnitCursor first = ahead;
-    bool early = false;
-    if (producer) {
-        for (int s = 0; s < STAGES; s++) {
-            mbar_init(&full[s], 1);
-            arrivals[s] = 0;
-        }
-        fence_mbar_init();
-        early = !run_stopped(st);
-    }
-    for (int j = 0; j < STAGES; j++) {
-        if (early && j < nunits) {
-            mbar_expect_tx(&full[j], TX_BYTES);
-            issue_v(smem + j * STAGE_BYTES, &full[j], ahead);
-        }
-        ahead.next(sk);
-    }
-    chain_wait();
-    const bool stopped = run_stopped(st);
-    chain_next();
-    if (early)
-        for (int j = 0; j < STAGES && j < nunits; j++) {
-            issue_f(smem + j * STAGE_BYTES, &full[j], first);
-            first.next(sk);
-        }
-    if (!stopped) return true;
-    if (early)
-        for (int j = 0; j < STAGES && j < nunits; j++) mbar_wait(&full[j], 0);
-    return false;
-}
-
 template <typename T, int RP>
 struct RankPad {
     // W rows / H^T rows padded to 16 bytes (the TMA inner-box granule).
@@ -442,6 +399,7 @@ __global__ void __launch_bounds__(HCfg<T, RP, RATIO>::kWarps * 32, 1)
           RunState *st) {
     using C = HCfg<T, RP, RATIO>;
     constexpr int CPT = C::CPT, KB = C::KB;
+    if (run_stopped(st)) return;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     // 1024 B alignment for the boxes, by offsetting the shared array itself so
     // that every access stays a shared-memory (LDS) access.
@@ -449,32 +407,40 @@ __global__ void __launch_bounds__(HCfg<T, RP, RATIO>::kWarps * 32, 1)
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + C::STAGES * C::STAGE);
     int *arrivals = reinterpret_cast<int *>(full + C::STAGES);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool producer = (threadIdx.x == 0);
     const int b = blockIdx.x;
     const long long u0 = sk.start(b), u1 = sk.start(b + 1);
     const long long nunits = u1 - u0;
 
     // Loads of one unit: the V boxes of its columns and rows, and its W rows.
-    auto issue_v = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
+    auto issue = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
         const int rb = c.along(sk);
 #pragma unroll
         for (int q = 0; q < C::NBOX; q++)
             tma_load_2d(stg + q * C::BROWS * C::BOXC * (int)sizeof(T), &tmV, bar,
                         c.major * C::TCOLS + q * C::BOXC, rb * C::BROWS);
-    };
-    auto issue_f = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
-        tma_load_2d(stg + C::VBYTES, &tmW, bar, 0, c.along(sk) * C::BROWS);
-    };
-    auto issue = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
-        issue_v(stg, bar, c);
-        issue_f(stg, bar, c);
+        tma_load_2d(stg + C::VBYTES, &tmW, bar, 0, rb * C::BROWS);
     };
     // `ahead`: the unit STAGES after the one being consumed (lane 0 of each
     // warp keeps one, for the refill it may have to issue).
     UnitCursor ahead;
     ahead.init(sk, u0);
-    if (!fill_stages<C::STAGES, C::STAGE, C::VBYTES + C::WBYTES>(smem, full, arrivals, nunits, ahead, sk, st,
-                                              issue_v, issue_f))
-        return;
+    if (producer) {
+        for (int s = 0; s < C::STAGES; s++) {
+            mbar_init(&full[s], 1);
+            arrivals[s] = 0;
+        }
+        fence_mbar_init();
+        for (int j = 0; j < C::STAGES; j++) {
+            if (j < nunits) {
+                mbar_expect_tx(&full[j], C::VBYTES + C::WBYTES);
+                issue(smem + j * C::STAGE, &full[j], ahead);
+            }
+            ahead.next(sk);
+        }
+    } else {
+        for (int j = 0; j < C::STAGES; j++) ahead.next(sk);
+    }
     __syncthreads();
 
     const int kh = lane / C::LPK, cl = lane % C::LPK;
@@ -612,38 +578,47 @@ __global__ void __launch_bounds__(WCfg<T, RP, RATIO>::kWarps * 32, 1)
     using C = WCfg<T, RP, RATIO>;
     constexpr int RT = C::RT, KB = C::KB;
     constexpr int VEC = 16 / (int)sizeof(T);  // columns per 16-byte chunk
+    if (run_stopped(st)) return;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + C::STAGES * C::STAGE);
     int *arrivals = reinterpret_cast<int *>(full + C::STAGES);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool producer = (threadIdx.x == 0);
     const int b = blockIdx.x;
     const long long u0 = sk.start(b), u1 = sk.start(b + 1);
     const long long nunits = u1 - u0;
 
     // Loads of one unit: NBOX boxes of BOXR rows x BCOLS columns of V
     // (swizzled) and the matching BCOLS rows of H^T.
-    auto issue_v = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
+    auto issue = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
         const int cb = c.along(sk);
 #pragma unroll
         for (int q = 0; q < C::NBOX; q++)
             tma_load_2d(stg + q * C::BOXR * C::ROWB, &tmV, bar, cb * C::BCOLS,
                         c.major * C::TROWS + q * C::BOXR);
-    };
-    auto issue_f = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
-        tma_load_2d(stg + C::VBYTES, &tmH, bar, 0, c.along(sk) * C::BCOLS);
-    };
-    auto issue = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
-        issue_v(stg, bar, c);
-        issue_f(stg, bar, c);
+        tma_load_2d(stg + C::VBYTES, &tmH, bar, 0, cb * C::BCOLS);
     };
     // `ahead`: the unit STAGES after the one being consumed (lane 0 of each
     // warp keeps one, for the refill it may have to issue).
     UnitCursor ahead;
     ahead.init(sk, u0);
-    if (!fill_stages<C::STAGES, C::STAGE, C::VBYTES + C::HBYTES>(smem, full, arrivals, nunits, ahead, sk, st,
-                                              issue_v, issue_f))
-        return;
+    if (producer) {
+        for (int s = 0; s < C::STAGES; s++) {
+            mbar_init(&full[s], 1);
+            arrivals[s] = 0;
+        }
+        fence_mbar_init();
+        for (int j = 0; j < C::STAGES; j++) {
+            if (j < nunits) {
+                mbar_expect_tx(&full[j], C::VBYTES + C::HBYTES);
+                issue(smem + j * C::STAGE, &full[j], ahead);
+            }
+            ahead.next(sk);
+        }
+    } else {
+        for (int j = 0; j < C::STAGES; j++) ahead.next(sk);
+    }
     __syncthreads();
 
     const int kh = lane / C::LPK, rl = lane % C::LPK;
@@ -792,34 +767,43 @@ __global__ void __launch_bounds__(DHCfg<RP>::kWarps * 32, 1)
     hpass_dmma(const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmW,
                int n, int p, StreamK sk, double *__restrict__ part, RunState *st) {
     using C = DHCfg<RP>;
+    if (run_stopped(st)) return;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + C::STAGES * C::STAGE);
     int *arrivals = reinterpret_cast<int *>(full + C::STAGES);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool producer = (threadIdx.x == 0);
     const int b = blockIdx.x;
     const long long u0 = sk.start(b), u1 = sk.start(b + 1);
     const long long nunits = u1 - u0;
 
-    auto issue_v = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
+    auto issue = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
         const int rb = c.along(sk);
 #pragma unroll
         for (int q = 0; q < C::NBOX; q++)
             tma_load_2d(stg + q * C::BROWS * C::BOXC * 8, &tmV, bar,
                         c.major * C::TCOLS + q * C::BOXC, rb * C::BROWS);
-    };
-    auto issue_f = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
-        tma_load_2d(stg + C::VBYTES, &tmW, bar, 0, c.along(sk) * C::BROWS);
-    };
-    auto issue = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
-        issue_v(stg, bar, c);
-        issue_f(stg, bar, c);
+        tma_load_2d(stg + C::VBYTES, &tmW, bar, 0, rb * C::BROWS);
     };
     UnitCursor ahead;
     ahead.init(sk, u0);
-    if (!fill_stages<C::STAGES, C::STAGE, C::VBYTES + C::WBYTES>(smem, full, arrivals, nunits, ahead, sk, st,
-                                              issue_v, issue_f))
-        return;
+    if (producer) {
+        for (int s = 0; s < C::STAGES; s++) {
+            mbar_init(&full[s], 1);
+            arrivals[s] = 0;
+        }
+        fence_mbar_init();
+        for (int j = 0; j < C::STAGES; j++) {
+            if (j < nunits) {
+                mbar_expect_tx(&full[j], C::VBYTES + C::WBYTES);
+                issue(smem + j * C::STAGE, &full[j], ahead);
+            }
+            ahead.next(sk);
+        }
+    } else {
+        for (int j = 0; j < C::STAGES; j++) ahead.next(sk);
+    }
     __syncthreads();
 
     const int g = lane >> 2, q4 = lane & 3;
@@ -932,34 +916,43 @@ __global__ void __launch_bounds__(DWCfg<RP>::kWarps * 32, 1)
     wpass_dmma(const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmH,
                int n, int p, StreamK sk, double *__restrict__ part, RunState *st) {
     using C = DWCfg<RP>;
+    if (run_stopped(st)) return;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + C::STAGES * C::STAGE);
     int *arrivals = reinterpret_cast<int *>(full + C::STAGES);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool producer = (threadIdx.x == 0);
     const int b = blockIdx.x;
     const long long u0 = sk.start(b), u1 = sk.start(b + 1);
     const long long nunits = u1 - u0;
 
-    auto issue_v = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
+    auto issue = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
         const int cb = c.along(sk);
 #pragma unroll
         for (int q = 0; q < C::NBOX; q++)
             tma_load_2d(stg + q * C::BOXR * C::ROWB, &tmV, bar, cb * C::BCOLS,
                         c.major * C::TROWS + q * C::BOXR);
-    };
-    auto issue_f = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
-        tma_load_2d(stg + C::VBYTES, &tmH, bar, 0, c.along(sk) * C::BCOLS);
-    };
-    auto issue = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
-        issue_v(stg, bar, c);
-        issue_f(stg, bar, c);
+        tma_load_2d(stg + C::VBYTES, &tmH, bar, 0, cb * C::BCOLS);
     };
     UnitCursor ahead;
     ahead.init(sk, u0);
-    if (!fill_stages<C::STAGES, C::STAGE, C::VBYTES + C::HBYTES>(smem, full, arrivals, nunits, ahead, sk, st,
-                                              issue_v, issue_f))
-        return;
+    if (producer) {
+        for (int s = 0; s < C::STAGES; s++) {
+            mbar_init(&full[s], 1);
+            arrivals[s] = 0;
+        }
+        fence_mbar_init();
+        for (int j = 0; j < C::STAGES; j++) {
+            if (j < nunits) {
+                mbar_expect_tx(&full[j], C::VBYTES + C::HBYTES);
+                issue(smem + j * C::STAGE, &full[j], ahead);
+            }
+            ahead.next(sk);
+        }
+    } else {
+        for (int j = 0; j < C::STAGES; j++) ahead.next(sk);
+    }
     __syncthreads();
 
     const int g = lane >> 2, q4 = lane & 3;
@@ -1089,31 +1082,40 @@ __global__ void __launch_bounds__(DHRCfg<RP>::kWarps * 32, 1)
                      const __grid_constant__ CUtensorMap tmW, const double *__restrict__ H, int n,
                      int p, StreamK sk, double *__restrict__ part, RunState *st) {
     using C = DHRCfg<RP>;
+    if (run_stopped(st)) return;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + C::STAGES * C::STAGE);
     int *arrivals = reinterpret_cast<int *>(full + C::STAGES);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool producer = (threadIdx.x == 0);
     const int b = blockIdx.x;
     const long long u0 = sk.start(b), u1 = sk.start(b + 1);
     const long long nunits = u1 - u0;
 
-    auto issue_v = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
+    auto issue = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
         const int rb = c.along(sk);
         tma_load_2d(stg, &tmV, bar, c.major * C::TCOLS, rb * C::BROWS);
-    };
-    auto issue_f = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
-        tma_load_2d(stg + C::VBYTES, &tmW, bar, 0, c.along(sk) * C::BROWS);
-    };
-    auto issue = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
-        issue_v(stg, bar, c);
-        issue_f(stg, bar, c);
+        tma_load_2d(stg + C::VBYTES, &tmW, bar, 0, rb * C::BROWS);
     };
     UnitCursor ahead;
     ahead.init(sk, u0);
-    if (!fill_stages<C::STAGES, C::STAGE, C::VBYTES + C::WBYTES>(smem, full, arrivals, nunits, ahead, sk, st,
-                                              issue_v, issue_f))
-        return;
+    if (producer) {
+        for (int s = 0; s < C::STAGES; s++) {
+            mbar_init(&full[s], 1);
+            arrivals[s] = 0;
+        }
+        fence_mbar_init();
+        for (int j = 0; j < C::STAGES; j++) {
+            if (j < nunits) {
+                mbar_expect_tx(&full[j], C::VBYTES + C::WBYTES);
+                issue(smem + j * C::STAGE, &full[j], ahead);
+            }
+            ahead.next(sk);
+        }
+    } else {
+        for (int j = 0; j < C::STAGES; j++) ahead.next(sk);
+    }
     __syncthreads();
 
     const int g = lane >> 2, q4 = lane & 3;
@@ -1269,31 +1271,40 @@ __global__ void __launch_bounds__(DWRCfg<RP>::kWarps * 32, 1)
                      const __grid_constant__ CUtensorMap tmH, const double *__restrict__ W, int n,
                      int p, StreamK sk, double *__restrict__ part, RunState *st) {
     using C = DWRCfg<RP>;
+    if (run_stopped(st)) return;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + C::STAGES * C::STAGE);
     int *arrivals = reinterpret_cast<int *>(full + C::STAGES);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool producer = (threadIdx.x == 0);
     const int b = blockIdx.x;
     const long long u0 = sk.start(b), u1 = sk.start(b + 1);
     const long long nunits = u1 - u0;
 
-    auto issue_v = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
+    auto issue = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
         const int cb = c.along(sk);
         tma_load_2d(stg, &tmV, bar, cb * C::BCOLS, c.major * C::TROWS);
-    };
-    auto issue_f = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
-        tma_load_2d(stg + C::VBYTES, &tmH, bar, 0, c.along(sk) * C::BCOLS);
-    };
-    auto issue = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
-        issue_v(stg, bar, c);
-        issue_f(stg, bar, c);
+        tma_load_2d(stg + C::VBYTES, &tmH, bar, 0, cb * C::BCOLS);
     };
     UnitCursor ahead;
     ahead.init(sk, u0);
-    if (!fill_stages<C::STAGES, C::STAGE, C::VBYTES + C::HBYTES>(smem, full, arrivals, nunits, ahead, sk, st,
-                                              issue_v, issue_f))
-        return;
+    if (producer) {
+        for (int s = 0; s < C::STAGES; s++) {
+            mbar_init(&full[s], 1);
+            arrivals[s] = 0;
+        }
+        fence_mbar_init();
+        for (int j = 0; j < C::STAGES; j++) {
+            if (j < nunits) {
+                mbar_expect_tx(&full[j], C::VBYTES + C::HBYTES);
+                issue(smem + j * C::STAGE, &full[j], ahead);
+            }
+            ahead.next(sk);
+        }
+    } else {
+        for (int j = 0; j < C::STAGES; j++) ahead.next(sk);
+    }
     __syncthreads();
 
     const int g = lane >> 2, q4 = lane & 3;
@@ -1470,6 +1481,7 @@ __global__ void __launch_bounds__(DHRCfg<RP>::kWarps * 32, 1)
                    const double *__restrict__ H, int n, int p, StreamK sk,
                    const double *__restrict__ roff, double *__restrict__ part, RunState *st) {
     using C = DHRCfg<RP>;
+    if (run_stopped(st)) return;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + C::STAGES * C::STAGE);
@@ -1477,27 +1489,35 @@ __global__ void __launch_bounds__(DHRCfg<RP>::kWarps * 32, 1)
     __shared__ double red[C::kWarps];
     __shared__ double2 logs[KL ? kLogEntries : 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool producer = (threadIdx.x == 0);
     const int b = blockIdx.x;
     const long long u0 = sk.start(b), u1 = sk.start(b + 1);
     const long long nunits = u1 - u0;
 
-    auto issue_v = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
+    auto issue = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
         const int rb = c.along(sk);
         tma_load_2d(stg, &tmV, bar, c.major * C::TCOLS, rb * C::BROWS);
-    };
-    auto issue_f = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
-        tma_load_2d(stg + C::VBYTES, &tmW, bar, 0, c.along(sk) * C::BROWS);
-    };
-    auto issue = [&](unsigned char *stg, uint64_t *bar, const UnitCursor &c) {
-        issue_v(stg, bar, c);
-        issue_f(stg, bar, c);
+        tma_load_2d(stg + C::VBYTES, &tmW, bar, 0, rb * C::BROWS);
     };
     UnitCursor ahead;
     ahead.init(sk, u0);
+    if (producer) {
+        for (int s = 0; s < C::STAGES; s++) {
+            mbar_init(&full[s], 1);
+            arrivals[s] = 0;
+        }
+        fence_mbar_init();
+        for (int j = 0; j < C::STAGES; j++) {
+            if (j < nunits) {
+                mbar_expect_tx(&full[j], C::VBYTES + C::WBYTES);
+                issue(smem + j * C::STAGE, &full[j], ahead);
+            }
+            ahead.next(sk);
+        }
+    } else {
+        for (int j = 0; j < C::STAGES; j++) ahead.next(sk);
+    }
     if (KL) log_table_init(logs);
-    if (!fill_stages<C::STAGES, C::STAGE, C::VBYTES + C::WBYTES>(smem, full, arrivals, nunits, ahead, sk, st,
-                                              issue_v, issue_f))
-        return;
     __syncthreads();
 
     const int g = lane >> 2, q4 = lane & 3;
@@ -1673,6 +1693,7 @@ __global__ void __launch_bounds__(THREADS, EpiSmem<RP, THREADS>::BLOCKS)
     extern __shared__ double smem_epi[];
     double *sG = smem_epi, *tile = smem_epi + ES::G;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool stopped = run_stopped(st);
     EpiParams es = e;
     es.G = sG;
     typename ES::GH ga;
@@ -1684,8 +1705,7 @@ __global__ void __launch_bounds__(THREADS, EpiSmem<RP, THREADS>::BLOCKS)
         double *sNum = tile, *sOld = tile + NS * RP * LD, *sNew = sOld + RP * LD;
         const int j0 = blockIdx.x * TC, j = j0 + lane;
         const int ct = j0 / tcols, c = j0 - ct * tcols + lane;
-        // All loads in flight before the first is used; the Gram and the old
-        // factor, which the pass does not write, before the wait for it.
+        // All loads in flight before the first is used.
         double gv[PG], ov[PK];
 #pragma unroll
         for (int i = 0; i < PG; i++) {
@@ -1698,9 +1718,6 @@ __global__ void __launch_bounds__(THREADS, EpiSmem<RP, THREADS>::BLOCKS)
             ov[i] = k < RP && j < p ? H[(size_t)k * p + j] : 0.0;
         }
         tp.find(sk, ct);
-        chain_wait();
-        const bool stopped = run_stopped(st);
-        chain_next();
         const size_t step = (size_t)sk.slots * RP * tcols;
         for (int it = warp; it < RP * NS; it += WARPS) {
             const int s = it / RP, k = it - s * RP;
@@ -1776,9 +1793,6 @@ __global__ void __launch_bounds__(THREADS, EpiSmem<RP, THREADS>::BLOCKS)
         double *sNew = tile + warp * RP * LD;  // this warp's
         if (e.G != nullptr)
             for (int x = threadIdx.x; x < RP * RP; x += THREADS) sG[x] = e.G[x];
-        chain_wait();
-        const bool stopped = run_stopped(st);
-        chain_next();
         __syncthreads();
         if (stopped) return;
         const int tiles = (p + TC - 1) / TC;
@@ -1841,6 +1855,7 @@ __global__ void __launch_bounds__(THREADS, EpiSmem<RP, THREADS>::BLOCKS)
     extern __shared__ double smem_epi[];
     double *sG = smem_epi, *tile = smem_epi + ES::G;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool stopped = run_stopped(st);
     EpiParams es = e;
     es.G = sG;
     typename ES::GW ga;
@@ -1854,8 +1869,7 @@ __global__ void __launch_bounds__(THREADS, EpiSmem<RP, THREADS>::BLOCKS)
         const int i0 = blockIdx.x * TR;
         const int rt = i0 / trows, rl = i0 - rt * trows;
         const int elems = min(TR, n - i0) * RP;
-        // All loads in flight before the first is used; the Gram and the old
-        // factor, which the pass does not write, before the wait for it.
+        // All loads in flight before the first is used.
         double gv[PG], ov[PO];
 #pragma unroll
         for (int i = 0; i < PG; i++) {
@@ -1868,9 +1882,6 @@ __global__ void __launch_bounds__(THREADS, EpiSmem<RP, THREADS>::BLOCKS)
             ov[i] = x < elems ? W[(size_t)i0 * RP + x] : 0.0;
         }
         tp.find(sk, rt);
-        chain_wait();
-        const bool stopped = run_stopped(st);
-        chain_next();
         const size_t step = (size_t)sk.slots * trows * RP;
         for (int it = threadIdx.x; it < EL * NS; it += THREADS) {
             const int s = it / EL, x = it - s * EL;
@@ -1941,9 +1952,6 @@ __global__ void __launch_bounds__(THREADS, EpiSmem<RP, THREADS>::BLOCKS)
         double *sRow = tile + warp * 32 * LD;  // this warp's 32 rows
         if (e.G != nullptr)
             for (int x = threadIdx.x; x < RP * RP; x += THREADS) sG[x] = e.G[x];
-        chain_wait();
-        const bool stopped = run_stopped(st);
-        chain_next();
         __syncthreads();
         if (stopped) return;
         const int tiles = (n + 31) / 32;
@@ -2011,11 +2019,9 @@ void launch_h_epilogue(double *H, TH *Ht, int p, const double *part, const Strea
                        const EpiParams &e, const GramOut &g, GramPlan gp, const RunState *st,
                        cudaStream_t s) {
     if (p <= 0 && g.want == GRAM_NONE) return;
-    // (With no units there is no pass between this and the Gram's writer.)
-    const ChainLaunches chain(ChainLaunches::active() && sk.G > 0);
     const auto go = [&](auto *k, int threads, size_t bytes) {
         allow_smem(k, bytes);
-        launch_chained(k, gp.blocks, threads, bytes, s, H, Ht, p, part, sk, tcols, e, g, st);
+        k<<<gp.blocks, threads, bytes, s>>>(H, Ht, p, part, sk, tcols, e, g, st);
     };
     if (gp.few)
         go(h_epilogue_sk<RP, TH, RPS_T, kEpiThreads>, kEpiThreads,
@@ -2029,10 +2035,9 @@ void launch_w_epilogue(double *W, int n, const double *part, const StreamK &sk, 
                        const EpiParams &e, const GramOut &g, GramPlan gp, const RunState *st,
                        cudaStream_t s) {
     if (n <= 0 && g.want == GRAM_NONE) return;
-    const ChainLaunches chain(ChainLaunches::active() && sk.G > 0);
     const auto go = [&](auto *k, int threads, size_t bytes) {
         allow_smem(k, bytes);
-        launch_chained(k, gp.blocks, threads, bytes, s, W, n, part, sk, trows, e, g, st);
+        k<<<gp.blocks, threads, bytes, s>>>(W, n, part, sk, trows, e, g, st);
     };
     if (gp.few)
         go(w_epilogue_sk<RP, kEpiThreads>, kEpiThreads,
@@ -2046,7 +2051,7 @@ void launch_gram_w(const double *W, int n, const GramOut &g, GramPlan gp, const 
                    cudaStream_t s) {
     const auto go = [&](auto *k, int threads, size_t bytes) {
         allow_smem(k, bytes);
-        launch_chained(k, gp.blocks, threads, bytes, s, W, n, g, st);
+        k<<<gp.blocks, threads, bytes, s>>>(W, n, g, st);
     };
     if (gp.few)
         go(gram_w_tiles<RP, kEpiThreads>, kEpiThreads,
@@ -2060,7 +2065,7 @@ void launch_gram_h(const double *H, int p, const GramOut &g, GramPlan gp, const 
                    cudaStream_t s) {
     const auto go = [&](auto *k, int threads, size_t bytes) {
         allow_smem(k, bytes);
-        launch_chained(k, gp.blocks, threads, bytes, s, H, p, g, st);
+        k<<<gp.blocks, threads, bytes, s>>>(H, p, g, st);
     };
     if (gp.few)
         go(gram_h_tiles<RP, kEpiThreads>, kEpiThreads,

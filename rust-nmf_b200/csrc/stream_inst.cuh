@@ -71,7 +71,8 @@ struct StreamOpsT final : StreamOps {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              C::SMEM);
         if (e != cudaSuccess) return e;
-        return launch_chained(kern, grid, 32 * C::kWarps, C::SMEM, s, tmV, tmW, H, n, p, sk, part, st);
+        kern<<<grid, 32 * C::kWarps, C::SMEM, s>>>(tmV, tmW, H, n, p, sk, part, st);
+        return cudaGetLastError();
     }
     template <bool RATIO, bool WEIGHTED = false>
     static cudaError_t launch_w(const CUtensorMap &tmV, const CUtensorMap &tmH, const double *W,
@@ -82,7 +83,8 @@ struct StreamOpsT final : StreamOps {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              C::SMEM);
         if (e != cudaSuccess) return e;
-        return launch_chained(kern, grid, 32 * C::kWarps, C::SMEM, s, tmV, tmH, W, n, p, sk, part, st);
+        kern<<<grid, 32 * C::kWarps, C::SMEM, s>>>(tmV, tmH, W, n, p, sk, part, st);
+        return cudaGetLastError();
     }
 
     // f64 ratio / weighted passes on the FP64 tensor cores.
@@ -95,7 +97,8 @@ struct StreamOpsT final : StreamOps {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              C::SMEM);
         if (e != cudaSuccess) return e;
-        return launch_chained(kern, grid, 32 * C::kWarps, C::SMEM, s, tmV, tmW, H, n, p, sk, part, st);
+        kern<<<grid, 32 * C::kWarps, C::SMEM, s>>>(tmV, tmW, H, n, p, sk, part, st);
+        return cudaGetLastError();
     }
     template <bool WEIGHTED>
     static cudaError_t launch_wr(const CUtensorMap &tmV, const CUtensorMap &tmH, const double *W,
@@ -106,7 +109,8 @@ struct StreamOpsT final : StreamOps {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              C::SMEM);
         if (e != cudaSuccess) return e;
-        return launch_chained(kern, grid, 32 * C::kWarps, C::SMEM, s, tmV, tmH, W, n, p, sk, part, st);
+        kern<<<grid, 32 * C::kWarps, C::SMEM, s>>>(tmV, tmH, W, n, p, sk, part, st);
+        return cudaGetLastError();
     }
 
     cudaError_t hpass(bool ratio, const CUtensorMap &tmV, const CUtensorMap &tmW,
@@ -119,7 +123,9 @@ struct StreamOpsT final : StreamOps {
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  C::SMEM);
             if (e != cudaSuccess) return e;
-            return launch_chained(nmfcu::hpass_dmma<RP>, grid, 32 * C::kWarps, C::SMEM, s, tmV, tmW, n, p, sk, part, st);
+            nmfcu::hpass_dmma<RP><<<grid, 32 * C::kWarps, C::SMEM, s>>>(tmV, tmW, n, p, sk, part,
+                                                                        st);
+            return cudaGetLastError();
         } else {
             if (ratio) return launch_h<true>(tmV, tmW, H, n, p, sk, part, st, grid, s);
             return launch_h<false>(tmV, tmW, H, n, p, sk, part, st, grid, s);
@@ -135,7 +141,9 @@ struct StreamOpsT final : StreamOps {
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  C::SMEM);
             if (e != cudaSuccess) return e;
-            return launch_chained(nmfcu::wpass_dmma<RP>, grid, 32 * C::kWarps, C::SMEM, s, tmV, tmH, n, p, sk, part, st);
+            nmfcu::wpass_dmma<RP><<<grid, 32 * C::kWarps, C::SMEM, s>>>(tmV, tmH, n, p, sk, part,
+                                                                        st);
+            return cudaGetLastError();
         } else {
             if (ratio) return launch_w<true>(tmV, tmH, W, n, p, sk, part, st, grid, s);
             return launch_w<false>(tmV, tmH, W, n, p, sk, part, st, grid, s);
@@ -167,7 +175,8 @@ struct StreamOpsT final : StreamOps {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              C::SMEM);
         if (e != cudaSuccess) return e;
-        return launch_chained(kern, sk.G, 32 * C::kWarps, C::SMEM, s, tmV, tmW, H, n, p, sk, roff, part, st);
+        kern<<<sk.G, 32 * C::kWarps, C::SMEM, s>>>(tmV, tmW, H, n, p, sk, roff, part, st);
+        return cudaGetLastError();
     }
     cudaError_t objective(bool kl, const CUtensorMap &tmV, const CUtensorMap &tmW, const double *H,
                           int n, int p, const StreamK &sk, const double *roff, double *part,
