@@ -62,22 +62,49 @@ __device__ __forceinline__ bool run_stopped(const RunState *st) {
 // ---------------------------------------------------------------------------
 
 // x / y for the ratio V / (WH), y != 0.  f64: x (1 / y) with the reciprocal
-// from the hardware approximation (rcp.approx.ftz.f64) refined by two
-// Newton-Raphson steps r <- r + r (1 - y r), each of which doubles the
-// correct bits, so the quotient is within about an ulp of the IEEE one (the
-// tests hold the loop to 1e-10 of the oracle's IEEE divisions); |y| outside
-// [2^-1000, 2^1000] and NaN take the IEEE division.  f32: the fast
-// reciprocal-multiply form (the FP32 form is tolerance-checked).
-__device__ __forceinline__ double ratio_div(double x, double y) {
-    const double a = fabs(y);
-    if (!(a > 0x1p-1000 && a < 0x1p1000)) return x / y;
+// r from the hardware approximation (rcp.approx.ftz.f64, correct to some 20
+// bits): with e = 1 - y r, 1 / y = r / (1 - e) = r (1 + e + e^2 + ...), and
+// the terms left out are below 2^-60, so the quotient is within about an ulp
+// of the IEEE one (the tests hold the loop to 1e-10 of the oracle's IEEE
+// divisions).  |y| outside [2^-1000, 2^1000) and NaN take the
+// IEEE division; an integer test of the exponent, since comparisons of doubles
+// share the pipe the passes are bound by.  f32: the fast reciprocal-multiply
+// form (the FP32 form is tolerance-checked).
+__device__ __forceinline__ bool ratio_plain(double y) {
+    return ((unsigned)__double2hiint(y) & 0x7fffffffu) - (23u << 20) < (2000u << 20);
+}
+__device__ __forceinline__ double ratio_fast(double x, double y) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(y));
-    double e = fma(-y, r, 1.0);
-    r = fma(r, e, r);
-    e = fma(-y, r, 1.0);
-    r = fma(r, e, r);
-    return x * r;
+    const double e = fma(-y, r, 1.0);
+    return x * fma(r, fma(e, e, e), r);
+}
+// The IEEE division, kept in the branch it stands in: the compiler takes a
+// plain one for cheap enough to do ahead of the branch, for every element
+// (20000 x 20000 at rank 20: 2.7 ms a pass for 1.5).
+__device__ __forceinline__ double ratio_ieee(double x, double y) {
+    asm volatile("" : "+d"(y));
+    return x / y;
+}
+__device__ __forceinline__ double ratio_div(double x, double y) {
+    return ratio_plain(y) ? ratio_fast(x, y) : ratio_ieee(x, y);
+}
+// q[i] = x[i] / y[i], 0 where y[i] is: the fast form of all of them side by
+// side, then at most one branch, taken where a y is 0 or at the ends of the
+// range.
+template <int N>
+__device__ __forceinline__ void ratios_or_zero(const double (&x)[N], const double (&y)[N],
+                                               double (&q)[N]) {
+    bool plain = true;
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        plain = plain && ratio_plain(y[i]);
+        q[i] = ratio_fast(x[i], y[i]);
+    }
+    if (plain) return;
+#pragma unroll
+    for (int i = 0; i < N; i++)
+        if (!ratio_plain(y[i])) q[i] = y[i] != 0.0 ? ratio_ieee(x[i], y[i]) : 0.0;
 }
 __device__ __forceinline__ float ratio_div(float x, float y) { return __fdividef(x, y); }
 
