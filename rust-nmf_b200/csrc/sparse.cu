@@ -19,14 +19,16 @@
 // Passes (one warp a line, lanes across its stored entries, a fixed
 // butterfly reduction, so results are bit-reproducible run to run):
 //   W pass  rows of the CSR:     out[i][k] = sum_t f(v_t) H^T[j_t][k]
-//   H pass  columns of a CSC copy made once a run (a stable radix sort of
-//           the column indices, so each column lists its rows in order):
+//   H pass  columns of a CSC copy made once a run (each column lists its
+//           rows in order: by tiles, or a stable sort of the column indices):
 //                                out[k][j] = sum_t f(v_t) W[i_t][k]
 // with f(v) = v, or v / (W H)_ij for brunet (0 where W H is 0).  The outputs
 // have the layouts of the dense engine's one-split epilogue partials, so its
 // update epilogues (h_epilogue / w_epilogue), Grams, rescaling, clamp and
 // stationary stop run unchanged.  Bytes per pass: nnz x 12 (value + index)
-// plus the factor rows gathered from L2 (W: n x RP, H^T: p x RP f64).
+// plus the factor rows, read from shared memory a block at a time where lines
+// have enough entries in each block, else gathered from L2 (W: n x RP, H^T:
+// p x RP f64).
 #include <cuda_runtime.h>
 
 #include <cub/cub.cuh>

@@ -738,43 +738,12 @@ __global__ void __launch_bounds__(WCfg<T, RP, RATIO>::kWarps * 32, 1)
 // H pass: A[k][j] = sum_u W[u][k] V[u][j] with M = k (rank tiles of 8), N = j
 // (4 column tiles of 8 a warp), K = u (4 rows a k-step, 4 k-steps a unit of
 // 16 rows, so that a stage's wait and release serve 4 k-steps).
-// The rank in tiles of 8 for the FP64 passes' contractions.  A remainder of 2
-// or 4 is REM plain FMAs an element instead of a tile padded to 8: both kinds
-// run on one pipe at one rate (36.8 and 36.0 TFLOP/s by themselves, 33-36 in
-// any mixture), so that only the products count, REM against 8.  Lane (g, q4)
-// sums its own row (column) residue q4 and the four lanes are added at the
-// flush.  A remainder of 6 would save too little for its registers, and a
-// plain pass, whose warps hold four tiles of 8 the other way, spills with 4 of
-// them beside two tiles (lee, 20000 x 40000 at rank 20: 29.2 ms for 27.4).
-template <int RP, bool RATIO>
-struct RankTiles {
-    static constexpr int MOST = RATIO || RP < 16 || RP > 24 ? 4 : 2;
-    static constexpr int REM = RP % 8 <= MOST ? RP % 8 : 0;
-    static constexpr int TILES = (RP - REM + 7) / 8;
-    static constexpr int T1 = TILES > 0 ? TILES : 1, R1 = REM > 0 ? REM : 1;  // array sizes
-};
-// A remainder's REM consecutive factor entries, 16-byte aligned.
-template <int REM>
-__device__ __forceinline__ void lds_rem(double *d, const double *src) {
-#pragma unroll
-    for (int x = 0; x < REM; x += 2) {
-        const double2 v = *reinterpret_cast<const double2 *>(src + x);
-        d[x] = v.x;
-        d[x + 1] = v.y;
-    }
-}
-__device__ __forceinline__ double sum_quad(double v) {
-    v += __shfl_xor_sync(0xffffffffu, v, 1);
-    return v + __shfl_xor_sync(0xffffffffu, v, 2);
-}
-
 template <int RP>
 struct DHCfg {
-    using RT = RankTiles<RP, false>;
-    static constexpr int MT = RT::TILES, REM = RT::REM;
-    // 16 warps of at most 128 registers; ranks above 24 take 8 warps and
-    // their 255 registers.
-    static constexpr int kWarps = RP > 24 ? 8 : 16;
+    static constexpr int MT = (RP + 7) / 8;
+    // 16 warps of at most 128 registers; ranks above 24 (four rank tiles of
+    // accumulators) take 8 warps and their 255 registers.
+    static constexpr int kWarps = MT >= 4 ? 8 : 16;
     static constexpr int NT = 4;
     static constexpr int WCOLS = NT * 8;
     static constexpr int TCOLS = kWarps * WCOLS;  // 512 columns a tile
@@ -840,7 +809,7 @@ __global__ void __launch_bounds__(DHCfg<RP>::kWarps * 32, 1)
     const int g = lane >> 2, q4 = lane & 3;
     const int wc0 = warp * C::WCOLS;  // this warp's first column in the tile
     const int vbox = wc0 / C::BOXC, voff = wc0 % C::BOXC;
-    double acc[C::RT::T1][C::NT][2], rem[C::NT][C::RT::R1];
+    double acc[C::MT][C::NT][2];
     int cur = -1;
     UnitCursor uc;
     uc.init(sk, u0);
@@ -865,14 +834,6 @@ __global__ void __launch_bounds__(DHCfg<RP>::kWarps * 32, 1)
                 }
             }
         }
-#pragma unroll
-        for (int nt = 0; nt < C::NT; nt++)
-#pragma unroll
-            for (int x = 0; x < C::REM; x++) {
-                const double v = sum_quad(rem[nt][x]);
-                if (q4 == x)
-                    put_partial(&dst[(size_t)(C::MT * 8 + x) * C::TCOLS + wc0 + nt * 8 + g], v, add);
-            }
     };
 
     for (long long i = 0; i < nunits; ++i) {
@@ -884,10 +845,6 @@ __global__ void __launch_bounds__(DHCfg<RP>::kWarps * 32, 1)
             for (int mt = 0; mt < C::MT; mt++)
 #pragma unroll
                 for (int nt = 0; nt < C::NT; nt++) acc[mt][nt][0] = acc[mt][nt][1] = 0.0;
-#pragma unroll
-            for (int nt = 0; nt < C::NT; nt++)
-#pragma unroll
-                for (int x = 0; x < C::REM; x++) rem[nt][x] = 0.0;
         }
         if (!mbar_wait(&full[s], (uint32_t)(rnd & 1))) {
             record_timeout(st, TIMEOUT_FULL);
@@ -901,8 +858,7 @@ __global__ void __launch_bounds__(DHCfg<RP>::kWarps * 32, 1)
 #pragma unroll
         for (int ks = 0; ks < C::BROWS / 4; ks++) {
             const int r = ks * 4 + q4;
-            double a[C::RT::T1], bv[C::NT], wx[C::RT::R1];
-            lds_rem<C::REM>(wx, sw + r * C::RPS + C::MT * 8);
+            double a[C::MT], bv[C::NT];
 #pragma unroll
             for (int mt = 0; mt < C::MT; mt++) {
                 const int k = mt * 8 + g;
@@ -914,10 +870,6 @@ __global__ void __launch_bounds__(DHCfg<RP>::kWarps * 32, 1)
             for (int mt = 0; mt < C::MT; mt++)
 #pragma unroll
                 for (int nt = 0; nt < C::NT; nt++) dmma_8x8x4(acc[mt][nt], a[mt], bv[nt]);
-#pragma unroll
-            for (int x = 0; x < C::REM; x++)
-#pragma unroll
-                for (int nt = 0; nt < C::NT; nt++) rem[nt][x] = fma(wx[x], bv[nt], rem[nt][x]);
         }
         __syncwarp();
         if (lane == 0)
@@ -938,9 +890,8 @@ __global__ void __launch_bounds__(DHCfg<RP>::kWarps * 32, 1)
 // unit of 16 columns read from a 128B-swizzled V box).
 template <int RP>
 struct DWCfg {
-    using RT = RankTiles<RP, false>;
-    static constexpr int NT = RT::TILES, REM = RT::REM;
-    static constexpr int kWarps = RP > 24 ? 8 : 16;
+    static constexpr int NT = (RP + 7) / 8;
+    static constexpr int kWarps = NT >= 4 ? 8 : 16;
     static constexpr int MW = 4;
     static constexpr int WROWS = MW * 8;
     static constexpr int TROWS = kWarps * WROWS;  // 512 rows a tile
@@ -1008,7 +959,7 @@ __global__ void __launch_bounds__(DWCfg<RP>::kWarps * 32, 1)
     // Row of A fragment mw: warp * 32 + mw * 8 + g (its swizzle key is g, the
     // row mod 8); its byte offset within the stage, before the chunk.
     const int rbase = warp * C::WROWS + g;
-    double acc[C::MW][C::RT::T1][2], rem[C::MW][C::RT::R1];
+    double acc[C::MW][C::NT][2];
     int cur = -1;
     UnitCursor uc;
     uc.init(sk, u0);
@@ -1033,11 +984,6 @@ __global__ void __launch_bounds__(DWCfg<RP>::kWarps * 32, 1)
                     put_partial(&d[1], acc[mw][nt][1], add);
                 }
             }
-#pragma unroll
-            for (int x = 0; x < C::REM; x++) {
-                const double v = sum_quad(rem[mw][x]);
-                if (q4 == x) put_partial(&dst[(size_t)row * RP + C::NT * 8 + x], v, add);
-            }
         }
     };
 
@@ -1050,10 +996,6 @@ __global__ void __launch_bounds__(DWCfg<RP>::kWarps * 32, 1)
             for (int mw = 0; mw < C::MW; mw++)
 #pragma unroll
                 for (int nt = 0; nt < C::NT; nt++) acc[mw][nt][0] = acc[mw][nt][1] = 0.0;
-#pragma unroll
-            for (int mw = 0; mw < C::MW; mw++)
-#pragma unroll
-                for (int x = 0; x < C::REM; x++) rem[mw][x] = 0.0;
         }
         if (!mbar_wait(&full[s], (uint32_t)(rnd & 1))) {
             record_timeout(st, TIMEOUT_FULL);
@@ -1066,8 +1008,7 @@ __global__ void __launch_bounds__(DWCfg<RP>::kWarps * 32, 1)
         for (int ks = 0; ks < C::BCOLS / 4; ks++) {
             const int j = ks * 4 + q4;              // column within the unit
             const int chunk = j >> 1, within = j & 1;
-            double a[C::MW], bh[C::RT::T1], hx[C::RT::R1];
-            lds_rem<C::REM>(hx, sh + j * C::RPS + C::NT * 8);
+            double a[C::MW], bh[C::NT];
 #pragma unroll
             for (int mw = 0; mw < C::MW; mw++) {
                 const int row = rbase + mw * 8;     // row & 7 == g
@@ -1083,10 +1024,6 @@ __global__ void __launch_bounds__(DWCfg<RP>::kWarps * 32, 1)
             for (int mw = 0; mw < C::MW; mw++)
 #pragma unroll
                 for (int nt = 0; nt < C::NT; nt++) dmma_8x8x4(acc[mw][nt], a[mw], bh[nt]);
-#pragma unroll
-            for (int x = 0; x < C::REM; x++)
-#pragma unroll
-                for (int mw = 0; mw < C::MW; mw++) rem[mw][x] = fma(a[mw], hx[x], rem[mw][x]);
         }
         __syncwarp();
         if (lane == 0)
@@ -1120,9 +1057,8 @@ __global__ void __launch_bounds__(DWCfg<RP>::kWarps * 32, 1)
 template <int RP>
 struct DHRCfg {
     static constexpr int KST = (RP + 3) / 4;  // k-steps of the WH chain
-    using RT = RankTiles<RP, true>;
-    static constexpr int MT = RT::TILES, REM = RT::REM;
-    static constexpr int kWarps = RP > 24 ? 8 : 16;
+    static constexpr int MT = (RP + 7) / 8;
+    static constexpr int kWarps = MT >= 4 ? 8 : 16;
     static constexpr int NT = 2;  // column tiles of 8 a warp
     static constexpr int WCOLS = NT * 8;
     static constexpr int TCOLS = kWarps * WCOLS;
@@ -1184,7 +1120,7 @@ __global__ void __launch_bounds__(DHRCfg<RP>::kWarps * 32, 1)
 
     const int g = lane >> 2, q4 = lane & 3;
     const int wc0 = warp * C::WCOLS;
-    double acc[C::RT::T1][C::NT][2], rem[C::NT][C::RT::R1];
+    double acc[C::MT][C::NT][2];
     double hreg[C::NT][C::KST];  // MMA 1's A: H[ks * 4 + q4][column of row g]
     int cur = -1, cur_major = -1;
     UnitCursor uc;
@@ -1210,14 +1146,6 @@ __global__ void __launch_bounds__(DHRCfg<RP>::kWarps * 32, 1)
                 }
             }
         }
-#pragma unroll
-        for (int nt = 0; nt < C::NT; nt++)
-#pragma unroll
-            for (int x = 0; x < C::REM; x++) {
-                const double v = sum_quad(rem[nt][x]);
-                if (q4 == x)
-                    put_partial(&dst[(size_t)(C::MT * 8 + x) * C::TCOLS + wc0 + nt * 8 + g], v, add);
-            }
     };
 
     for (long long i = 0; i < nunits; ++i) {
@@ -1229,10 +1157,6 @@ __global__ void __launch_bounds__(DHRCfg<RP>::kWarps * 32, 1)
             for (int mt = 0; mt < C::MT; mt++)
 #pragma unroll
                 for (int nt = 0; nt < C::NT; nt++) acc[mt][nt][0] = acc[mt][nt][1] = 0.0;
-#pragma unroll
-            for (int nt = 0; nt < C::NT; nt++)
-#pragma unroll
-                for (int x = 0; x < C::REM; x++) rem[nt][x] = 0.0;
             if (uc.major != cur_major) {
                 cur_major = uc.major;
 #pragma unroll
@@ -1263,7 +1187,7 @@ __global__ void __launch_bounds__(DHRCfg<RP>::kWarps * 32, 1)
                 const int k = ks * 4 + q4;
                 b1[ks] = (k < RP) ? sw[(r0 + g) * C::RPS + k] : 0.0;
             }
-            double a2[C::RT::T1][2];  // MMA 2's A: W[r0 + 2 q4 + e][mt * 8 + g]
+            double a2[C::MT][2];  // MMA 2's A: W[r0 + 2 q4 + e][mt * 8 + g]
 #pragma unroll
             for (int mt = 0; mt < C::MT; mt++) {
                 const int k = mt * 8 + g;
@@ -1297,16 +1221,6 @@ __global__ void __launch_bounds__(DHRCfg<RP>::kWarps * 32, 1)
 #pragma unroll
                     for (int nt = 0; nt < C::NT; nt++)
                         dmma_8x8x4(acc[mt][nt], a2[mt][e], qv[2 * nt + e]);
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                double wx[C::RT::R1];
-                lds_rem<C::REM>(wx, sw + (r0 + 2 * q4 + e) * C::RPS + C::MT * 8);
-#pragma unroll
-                for (int x = 0; x < C::REM; x++)
-#pragma unroll
-                    for (int nt = 0; nt < C::NT; nt++)
-                        rem[nt][x] = fma(wx[x], qv[2 * nt + e], rem[nt][x]);
-            }
         }
         __syncwarp();
         if (lane == 0)
@@ -1328,9 +1242,8 @@ __global__ void __launch_bounds__(DHRCfg<RP>::kWarps * 32, 1)
 template <int RP>
 struct DWRCfg {
     static constexpr int KST = (RP + 3) / 4;
-    using RT = RankTiles<RP, true>;
-    static constexpr int NT = RT::TILES, REM = RT::REM;
-    static constexpr int kWarps = RP > 24 ? 8 : 16;
+    static constexpr int NT = (RP + 7) / 8;
+    static constexpr int kWarps = NT >= 4 ? 8 : 16;
     static constexpr int MW = 2;  // row tiles of 8 a warp
     static constexpr int WROWS = MW * 8;
     static constexpr int TROWS = kWarps * WROWS;
@@ -1393,7 +1306,7 @@ __global__ void __launch_bounds__(DWRCfg<RP>::kWarps * 32, 1)
 
     const int g = lane >> 2, q4 = lane & 3;
     const int rbase = warp * C::WROWS + g;  // row of fragment mw: rbase + mw * 8 (row & 7 == g)
-    double acc[C::MW][C::RT::T1][2], rem[C::MW][C::RT::R1];
+    double acc[C::MW][C::NT][2];
     double wreg[C::MW][C::KST];  // MMA 1's A: W[row][ks * 4 + q4]
     int cur = -1, cur_major = -1;
     UnitCursor uc;
@@ -1419,11 +1332,6 @@ __global__ void __launch_bounds__(DWRCfg<RP>::kWarps * 32, 1)
                     put_partial(&d[1], acc[mw][nt][1], add);
                 }
             }
-#pragma unroll
-            for (int x = 0; x < C::REM; x++) {
-                const double v = sum_quad(rem[mw][x]);
-                if (q4 == x) put_partial(&dst[(size_t)row * RP + C::NT * 8 + x], v, add);
-            }
         }
     };
 
@@ -1436,10 +1344,6 @@ __global__ void __launch_bounds__(DWRCfg<RP>::kWarps * 32, 1)
             for (int mw = 0; mw < C::MW; mw++)
 #pragma unroll
                 for (int nt = 0; nt < C::NT; nt++) acc[mw][nt][0] = acc[mw][nt][1] = 0.0;
-#pragma unroll
-            for (int mw = 0; mw < C::MW; mw++)
-#pragma unroll
-                for (int x = 0; x < C::REM; x++) rem[mw][x] = 0.0;
             if (uc.major != cur_major) {
                 cur_major = uc.major;
 #pragma unroll
@@ -1469,7 +1373,7 @@ __global__ void __launch_bounds__(DWRCfg<RP>::kWarps * 32, 1)
                 const int k = ks * 4 + q4;
                 b1[ks] = (k < RP) ? sh[(j0 + g) * C::RPS + k] : 0.0;
             }
-            double b2[C::RT::T1][2];  // MMA 2's B: H^T[j0 + 2 q4 + e][nt * 8 + g]
+            double b2[C::NT][2];  // MMA 2's B: H^T[j0 + 2 q4 + e][nt * 8 + g]
 #pragma unroll
             for (int nt = 0; nt < C::NT; nt++) {
                 const int k = nt * 8 + g;
@@ -1510,16 +1414,6 @@ __global__ void __launch_bounds__(DWRCfg<RP>::kWarps * 32, 1)
 #pragma unroll
                     for (int mw = 0; mw < C::MW; mw++)
                         dmma_8x8x4(acc[mw][nt], qv[2 * mw + e], b2[nt][e]);
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                double hx[C::RT::R1];
-                lds_rem<C::REM>(hx, sh + (j0 + 2 * q4 + e) * C::RPS + C::NT * 8);
-#pragma unroll
-                for (int x = 0; x < C::REM; x++)
-#pragma unroll
-                    for (int mw = 0; mw < C::MW; mw++)
-                        rem[mw][x] = fma(qv[2 * mw + e], hx[x], rem[mw][x]);
-            }
         }
         __syncwarp();
         if (lane == 0)

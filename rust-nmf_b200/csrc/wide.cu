@@ -12,10 +12,8 @@
 //                       lib.rs:89-97 / 181-189) is written out by a tiled
 //                       kernel, then W^T Q and Q H'^T by the same passes.
 // Everything rank-dependent (Grams, updates, rescaling, objective) runs in
-// the kernels below with the rank as a run-time value: one thread per column
-// of H / row of W for the updates, in the operation order of the dense
-// engine's epilogues (kernels.cuh h_update / w_update), which follow the
-// reference term by term.  The stop state is the context's run state, so
+// the kernels below with the rank as a run-time value; the updates follow the
+// formulas of the dense engine's epilogues (kernels.cuh h_update / w_update).  The stop state is the context's run state, so
 // every pass and kernel of an iteration after a stationary stop does no work.
 #include <cuda_runtime.h>
 

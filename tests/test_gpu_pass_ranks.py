@@ -1,6 +1,5 @@
-"""The FP64 passes at ranks whose last tile of 8 is a remainder of 2 or 4 (plain
-multiply-adds beside the tensor-core tiles), over several tiles, boxes and
-units; and the quotient V / (W H) at the ends of its fast range.
+"""The FP64 passes at ranks on and off their tiles of 8, over several tiles,
+boxes and units; and the quotient V / (W H) at the ends of its fast range.
 
 Tolerances: max|d| / max|ref| <= 1e-10 on the factors, the FP64 path's bound;
 for one quotient at rank 1, 16 eps: the product, the quotient (an ulp against
@@ -22,7 +21,7 @@ EPS = np.finfo(np.float64).eps
 @pytest.mark.parametrize("method", ["lee", "brunet", "lsnmf"])
 @pytest.mark.parametrize("n,p", [(530, 1030), (1025, 513), (17, 2100)])
 @pytest.mark.parametrize("r", [2, 4, 10, 12, 18, 20, 26, 28])
-def test_remainder_ranks(oracle, method, n, p, r):
+def test_pass_ranks(oracle, method, n, p, r):
     r = min(r, n)
     gen = np.random.default_rng(100 * r + n)
     W = gen.gamma(0.6, 1.0, (n, r)) + 0.01
