@@ -81,7 +81,8 @@ __device__ __forceinline__ double ratio_fast(double x, double y) {
 }
 // The IEEE division, kept in the branch it stands in: the compiler takes a
 // plain one for cheap enough to do ahead of the branch, for every element
-// (20000 x 20000 at rank 20: 2.7 ms a pass for 1.5).
+// (20000 x 20000 at rank 20: 2.7 ms a pass; 1.52 with comparisons of doubles
+// and two Newton steps, 1.35 as it is).
 __device__ __forceinline__ double ratio_ieee(double x, double y) {
     asm volatile("" : "+d"(y));
     return x / y;
