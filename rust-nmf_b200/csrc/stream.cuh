@@ -1552,6 +1552,8 @@ __global__ void __launch_bounds__(DHRCfg<RP>::kWarps * 32, 1)
         const unsigned char *stg = smem + s * C::STAGE;
         const double *sv = reinterpret_cast<const double *>(stg) + wc0 + g;
         const double *sw = reinterpret_cast<const double *>(stg + C::VBYTES);
+        const int row0 = uc.along(sk) * C::BROWS;
+        const bool edge = n - row0 < C::BROWS || p - uc.major * C::TCOLS < C::TCOLS;
 #pragma unroll 1
         for (int r0 = 0; r0 < C::BROWS; r0 += 8) {
             double b1[C::KST];  // W[r0 + g][ks * 4 + q4]
@@ -1567,14 +1569,19 @@ __global__ void __launch_bounds__(DHRCfg<RP>::kWarps * 32, 1)
             for (int ks = 0; ks < C::KST; ks++)
 #pragma unroll
                 for (int nt = 0; nt < C::NT; nt++) dmma_8x8x4(wh[nt], hreg[nt][ks], b1[ks]);
+            // Past V's edge one operand is 0, the other a factor's entry: 0
+            // also where that is infinite.
+            if (edge)
+#pragma unroll
+                for (int e = 0; e < 2; e++)
+#pragma unroll
+                    for (int nt = 0; nt < C::NT; nt++)
+                        if (!in[nt] || row0 + r0 + 2 * q4 + e >= n) wh[nt][e] = 0.0;
 #pragma unroll
             for (int e = 0; e < 2; e++) {
                 const int row = r0 + 2 * q4 + e;
                 double ro = 0.0;
-                if (!KL && roff != nullptr) {
-                    const int ri = uc.along(sk) * C::BROWS + row;
-                    ro = ri < n ? roff[ri] : 0.0;
-                }
+                if (!KL && roff != nullptr) ro = row0 + row < n ? roff[row0 + row] : 0.0;
 #pragma unroll
                 for (int nt = 0; nt < C::NT; nt++) {
                     // Past V's edge v and wh are 0: no term but roff's.
