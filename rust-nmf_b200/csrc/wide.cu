@@ -256,6 +256,17 @@ __global__ void __launch_bounds__(kT, 2)
                 for (int y = 0; y < 4; y++) nmfcu::dmma_8x8x4(acc[x][y], a[x], b[y]);
         }
     }
+    // Past V's edge one operand is 0, the other a factor's entry: 0 also where
+    // that is infinite.
+    if (MODE != 0 && (n - i0 < kWhRows || p - j0 < kWhCols))
+#pragma unroll
+        for (int x = 0; x < 4; x++)
+#pragma unroll
+            for (int y = 0; y < 4; y++)
+#pragma unroll
+                for (int e = 0; e < 2; e++)
+                    if (i0 + wr + x * 8 + g >= n || j0 + wc + y * 8 + 2 * q + e >= p)
+                        acc[x][y][e] = 0.0;
     // A row's eight elements a thread are loaded together, the next row's while
     // this one's are divided (or their logarithms taken).
     double term = 0.0;

@@ -57,3 +57,17 @@ def test_stationary_run_goes_on(oracle, method, n, p):
     got = nmf_rs.nmf(V, 3, method, W0=W, H0=H, max_iter=3, **kw)
     assert got.n_iter == ref["n_iter"] and ref["n_iter"] > 0
     np.testing.assert_allclose(got.deviances, ref["deviances"], rtol=1e-9)
+
+
+# ranks above 32: 128 x 64 tiles
+@pytest.mark.parametrize("method", ["lee", "brunet", "hals"])
+@pytest.mark.parametrize("side", ["w", "h"])
+@pytest.mark.parametrize("n,p", [(128, 64), (129, 64), (128, 65), (100, 110), (130, 261)])
+def test_wide_objective_is_infinite(oracle, method, side, n, p):
+    V, W, H = _inputs(n, p, 34)
+    _infinite(side, V, W, H)
+    kw = dict(stop="stationary", stationary_th=0.0)
+    ref = oracle.nmf_method(method, V, W, H, 1, **kw)
+    got = nmf_rs.nmf(V, 34, method, W0=W, H0=H, max_iter=1, **kw)
+    assert ref["deviances"][0] == np.inf == got.deviances[0]
+    assert got.n_iter == ref["n_iter"] == 1
