@@ -541,7 +541,15 @@ __global__ void __launch_bounds__(32 * BlkCfg<RP>::WARPS, 1)
                             wh[q] = keep + __shfl_xor_sync(0xffffffffu, give, o);
                         }
                     }
-                    w = (wh[0] != 0.0) ? nmfcu::ratio_div(w, wh[0]) : 0.0;
+                    // 0 where W H is, and in a lane past the entries, whose W H
+                    // is 0 times the line's factor row: NaN where that is
+                    // infinite.
+                    if (nmfcu::ratio_plain(wh[0]))
+                        w = nmfcu::ratio_fast(w, wh[0]);
+                    else if (wh[0] == 0.0 || (t + 32 >= t1 && xo < 0))
+                        w = 0.0;
+                    else
+                        w = nmfcu::ratio_ieee(w, wh[0]);
                 }
 #pragma unroll
                 for (int q = 0; q < C::GL; q++) {

@@ -5,6 +5,7 @@ from __future__ import annotations
 
 import numpy as np
 import pytest
+import scipy.sparse as sp
 
 import nmf_rs
 from nmf_rs import _native
@@ -71,3 +72,46 @@ def test_wide_objective_is_infinite(oracle, method, side, n, p):
     got = nmf_rs.nmf(V, 34, method, W0=W, H0=H, max_iter=1, **kw)
     assert ref["deviances"][0] == np.inf == got.deviances[0]
     assert got.n_iter == ref["n_iter"] == 1
+
+
+def _stored_brunet(M, W, H):
+    """One brunet iteration over the stored entries of M alone."""
+    c = M.tocoo()
+    i, j, v = c.row, c.col, c.data
+
+    def quotient(W, H):
+        wh = (W[i] * H[:, j].T).sum(1)
+        return np.where(wh != 0.0, v / np.where(wh != 0.0, wh, 1.0), 0.0)
+
+    with np.errstate(all="ignore"):
+        num = np.zeros((H.shape[1], H.shape[0]))
+        np.add.at(num, j, quotient(W, H)[:, None] * W[i])
+        H = H * num.T / W.sum(0)[:, None]
+        num = np.zeros(W.shape)
+        np.add.at(num, i, quotient(W, H)[:, None] * H[:, j].T)
+        return W * num / H.sum(1)[None, :], H
+
+
+# Lines with enough entries for the blocked passes at every number of lanes an
+# entry (rank 1-2 one, 3-6 two, above four), and sparser ones, which gather.
+@pytest.mark.parametrize("side", ["w", "h"])
+@pytest.mark.parametrize("n,p,r,density", [(150, 170, 2, 0.5), (301, 500, 4, 0.6),
+                                           (300, 500, 6, 0.6), (1100, 2200, 20, 0.2),
+                                           (900, 1000, 32, 0.2), (700, 1500, 20, 0.01)])
+def test_sparse_lines_keep_infinity(n, p, r, density, side):
+    """V / (W H) is 0 at a stored entry whose W H is infinite, whatever the
+    number of entries of its line."""
+    V, W, H = _inputs(n, p, r)
+    V[np.random.default_rng(2).random(V.shape) >= density] = 0.0
+    if side == "w":
+        W[7, 1] = np.inf
+    else:
+        H[1, 9] = np.inf
+    M = sp.csr_matrix(V)
+    want_W, want_H = _stored_brunet(M, W, H)
+    got = nmf_rs.nmf(M, r, "brunet", W0=W, H0=H, max_iter=1)
+    for g, w in ((got.W, want_W), (got.H, want_H)):
+        np.testing.assert_array_equal(np.isnan(g), np.isnan(w))
+        # the FP64 path's bound, 1e-10 of the largest
+        ok = np.isfinite(w)
+        assert np.all(np.abs(g[ok] - w[ok]) <= 1e-10 * np.abs(w[ok]).max(initial=0.0))
