@@ -1696,8 +1696,7 @@ nmfcu_status objective_host(bool kl, int64_t n, int64_t p, int64_t r, const doub
                                               c->state.as<RunState>());
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaMemcpyAsync(out, c->dev.ptr, sizeof(double), cudaMemcpyDeviceToHost, s));
-    CUDA_TRY(cudaStreamSynchronize(s));
-    return NMFCU_OK;
+    return finish_checked(c, s);
 }
 
 }  // namespace
