@@ -156,6 +156,9 @@ __global__ void __launch_bounds__(kR) finish_sums(const double *__restrict__ par
 // chain's next two), where entry b alone is new: the thread that owns index b
 // has computed d(c1, b) and d(c2, b) itself.  Each thread fences its writes
 // before its warp sends that step's candidate, so the steps after it see them.
+//
+// The hardware barriers stand before and after the steps alone, so that a
+// thread whose wait has run out meets the others at the last one.
 // ---------------------------------------------------------------------------
 namespace cg = cooperative_groups;
 
@@ -233,7 +236,7 @@ __device__ __forceinline__ double average(double fa, double da, double fb, doubl
 }
 
 // E: a thread's entries of a row (0: any number, read when needed, with a
-// barrier of its own after a merge).  Writes each merge's height and pair
+// meeting of the cluster after a merge).  Writes each merge's height and pair
 // count n_a n_b.  Every loop ends: a chain of a symmetric D holds distinct
 // clusters; a chain that would exceed p (an asymmetric or NaN D) ends the
 // tree with the remaining heights NaN.
@@ -281,6 +284,23 @@ __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kTc)
     bool have_prev = false;  // vp holds prev's row
     int fresh = -1;                 // the index merged in the step before
     double new1 = 0.0, new2 = 0.0;  // its distances to x and prev (its owner)
+    bool late = false;              // this thread's wait ran out
+    // A step without candidates: every thread's writes before it are visible
+    // to the cluster's threads after it.
+    const auto meet = [&] {
+        asm volatile("fence.acq_rel.cluster;" ::: "memory");
+        __syncwarp();
+        const unsigned bar = smem_addr(&bars[par]);
+        if (tid == 0) bar_expect(bar, kCand * sizeof(ulonglong2));
+        if (lane < kCl)
+            send_async(smem_addr(&cand[par][rank * (kTc / 32) + warp]), bar, lane, ~0ull, ~0ull);
+        const bool ok = bar_wait(bar, phase);
+        if (ok) {
+            par ^= 1;
+            phase ^= (par == 0);
+        }
+        return ok;
+    };
     int k = 0;
     while (k < p - 1) {
         if (E > 0) {
@@ -358,7 +378,7 @@ __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kTc)
             }
         }
         if (!bar_wait(bar, phase)) {
-            atomicExch(gave_up, 1);
+            late = true;
             break;
         }
         key = ~0ull;
@@ -413,7 +433,10 @@ __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kTc)
         prev = c2;
         have_prev = false;
         if (E == 0 || len == 0) {
-            cl.sync();  // the merge's writes, for whichever row comes next
+            if (!meet()) {  // the merge's writes, for whichever row comes next
+                late = true;
+                break;
+            }
             fresh = -1;
             wrote = false;
         }
@@ -430,7 +453,18 @@ __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kTc)
             height[k] = NAN;
             npair[k] = 0.0;
         }
-    cl.sync();  // no block leaves while another may still write its candidates
+    if (late) atomicExch(gave_up, 1);
+    // No block leaves while another may still write its candidates.  Every
+    // thread gets here, late or not: it waits for nothing but its own bounded
+    // waits, and a warp that is late sends no more, so the others are late in
+    // the step after at most.
+    cl.sync();
+    if (late) {  // what is on its way here, of this step and the next, has as long again
+        bar_wait(smem_addr(&bars[par]), phase);
+        par ^= 1;
+        phase ^= (par == 0);
+        bar_wait(smem_addr(&bars[par]), phase);
+    }
 }
 
 // stat[4] = the cophenetic correlation of matrix blockIdx.x from its merges
