@@ -365,16 +365,22 @@ struct WideEpi {
 // largest term.
 struct SweepDiv {
     double d, r;  // the divisor and RN(1 / d)
+    bool plain;   // r and 1 / r are far from the ends of the range
 };
 __device__ __forceinline__ SweepDiv sweep_div(const WideEpi &e, double gkk) {
     const double d = e.method == nmfcu::M_DNMF ? fmax(add(gkk, e.gamma), e.eps) : fmax(gkk, e.eps);
-    return {d, __drcp_rn(d)};
+    return {d, __drcp_rn(d), d > 0x1p-900 && d < 0x1p900};
 }
 // max(eps, s / d): the quotient from the reciprocal with one residual
-// correction (Markstein 1990), three dependent operations.
+// correction (Markstein 1990), three dependent operations.  The IEEE division
+// at the ends of the range: with eps = 0 a component that has all but vanished
+// has a divisor whose reciprocal is infinite.
 __device__ __forceinline__ double sweep_value(double s, SweepDiv v, double eps) {
     double q = __dmul_rn(s, v.r);
-    if (fabs(s) < 0x1p900) q = fma(fma(-q, v.d, s), v.r, q);
+    if (v.plain && fabs(s) < 0x1p900)
+        q = fma(fma(-q, v.d, s), v.r, q);
+    else
+        q = nmfcu::ratio_ieee(s, v.d);
     return q > eps ? q : eps;
 }
 

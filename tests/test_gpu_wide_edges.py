@@ -52,3 +52,31 @@ def test_deviances(oracle, method, n, p):
     got, ref = _run(oracle, method, n, p, 41, stop="stationary", stationary_th=0.0)
     assert got.n_iter == ref["n_iter"]
     np.testing.assert_allclose(got.deviances, ref["deviances"], rtol=1e-11)
+
+
+@pytest.mark.parametrize("r", [34, 41])
+@pytest.mark.parametrize("k", [0, 9])
+@pytest.mark.parametrize("scale,size", [(2.0 ** -535, np.float64(1e150)), (2.0 ** -560, np.inf)])
+def test_vanishing_component(oracle, r, k, scale, size):
+    """eps = 0 and a column of W whose squares add up to a subnormal (64 x
+    2^-1070, exact) or to 0: H's row is the quotient by that, huge or infinite,
+    not eps."""
+    gen = np.random.default_rng(7 * r + k)
+    n, p = 64, 70
+    W = gen.gamma(0.6, 1.0, (n, r)) + 0.01
+    H = 1e-3 * gen.gamma(0.6, 1.0, (r, p))
+    W[:, k] = scale
+    V = 1e3 + gen.random((n, p))  # far above W H: the row's own sum stays positive
+    if k:  # ... and the components before it are empty
+        W[:, :k] = 0.0
+        H[:k] = 0.0
+    ref = oracle.nmf_method("hals", V, W, H, 1, eps=0.0)
+    got = nmf_rs.nmf(V, r, "hals", W0=W, H0=H, max_iter=1, eps=0.0)
+    assert ref["H"][k].min() > size if size < np.inf else np.all(ref["H"][k] == np.inf)
+    for a, b in ((got.W, ref["W"]), (got.H, ref["H"])):
+        np.testing.assert_array_equal(np.isnan(a), np.isnan(b))
+    if size == np.inf:
+        assert np.all(got.H[k] == np.inf)
+    else:
+        # the module's bound, on the row itself
+        assert rel_max(got.H[k], ref["H"][k]) <= TOL
