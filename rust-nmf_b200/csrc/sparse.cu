@@ -367,6 +367,7 @@ __global__ void __launch_bounds__(kT)
 // shared-memory reads of factor rows at random bank phases, about 2.6 cycles
 // an entry, and at the ratio the latency of its FP64 chain.
 constexpr int kBlkBytes = 200 * 1024;  // of F in shared memory
+constexpr int blk_rows(int RP) { return kBlkBytes / (RP * 8) / 32 * 32; }  // rows of F a block
 template <int RP>
 struct BlkCfg {
     static constexpr int PAIRS = RP / 2;
@@ -374,7 +375,7 @@ struct BlkCfg {
     static constexpr int UPL = (PAIRS + GL - 1) / GL;               // pairs of a lane
     // Warps: as many as the registers of GL rows' pairs leave room for.
     static constexpr int WARPS = UPL >= 4 ? 12 : 16;
-    static constexpr int ROWS = kBlkBytes / (RP * 8) / 32 * 32;     // rows of F a block
+    static constexpr int ROWS = blk_rows(RP);
     static constexpr int SMEM = ROWS * RP * 8 + 16;
 };
 
@@ -744,6 +745,17 @@ nmfcu_status carve(nmfcu_context *c, int slot, const std::vector<size_t> &sizes,
     return NMFCU_OK;
 }
 
+// Entries of an average segment from which the blocked passes run: a segment
+// costs a warp its line's pointers, factor row and sum (about as much as 16
+// entries), which a few entries do not pay for.
+constexpr int64_t kBlkEntries = 16;
+inline bool blk_rows_pass(int64_t n, int64_t p, int RP, int64_t nnz) {
+    return nnz >= kBlkEntries * n * cdiv(p, blk_rows(RP));
+}
+inline bool blk_cols_pass(int64_t n, int64_t p, int RP, int64_t nnz) {
+    return nnz >= kBlkEntries * p * cdiv(n, blk_rows(RP));
+}
+
 // Whether the rows of the CSR are in (strict) column order.
 nmfcu_status check_order(nmfcu_context *c, int64_t n, SparseV &sv, cudaStream_t s) {
     void *fl = nullptr;
@@ -795,7 +807,8 @@ nmfcu_status build_csc_tiles(nmfcu_context *c, int64_t n, int64_t p, SparseV &sv
 // stable radix sort of the column indices.  10^8 entries, 20000 x 50000: 5.2
 // ms by the sort, 1.8 by tiles; 1.5 10^6, 5000 x 10000: 0.08 and 0.11.
 constexpr int64_t kCscTileEntries = 1 << 22;
-nmfcu_status build_csc(nmfcu_context *c, int64_t n, int64_t p, SparseV &sv, cudaStream_t s) {
+nmfcu_status build_csc(nmfcu_context *c, int64_t n, int64_t p, int RP, SparseV &sv,
+                       cudaStream_t s) {
     const int64_t nnz = sv.nnz;
     std::vector<void *> cb;
     NMFCU_TRY(carve(c, kSlotCsc,
@@ -805,11 +818,13 @@ nmfcu_status build_csc(nmfcu_context *c, int64_t n, int64_t p, SparseV &sv, cuda
     sv.cptr = static_cast<int64_t *>(cb[0]);
     sv.cidx = static_cast<int32_t *>(cb[1]);
     sv.cval = static_cast<double *>(cb[2]);
-    if (nnz > 0) NMFCU_TRY(check_order(c, n, sv, s));
     const int64_t tile_rows = (n + kCscRows - 1) / kCscRows;
-    if (sv.strict && nnz >= kCscTileEntries && p < INT32_MAX && tile_rows <= 65535 &&
-        tile_rows * p <= nnz)
-        return build_csc_tiles(c, n, p, sv, s);
+    const bool tiles = nnz >= kCscTileEntries && p < INT32_MAX && tile_rows <= 65535 &&
+                       tile_rows * p <= nnz;
+    // (a pass over the indices and a wait for its answer, for those who ask)
+    if (nnz > 0 && (tiles || blk_rows_pass(n, p, RP, nnz) || blk_cols_pass(n, p, RP, nnz)))
+        NMFCU_TRY(check_order(c, n, sv, s));
+    if (tiles && sv.strict) return build_csc_tiles(c, n, p, sv, s);
     int bits = 1;
     while (bits < 31 && ((int64_t)1 << bits) < p) bits++;
     size_t temp = 0;
@@ -1076,11 +1091,6 @@ nmfcu_status make_work(nmfcu_context *c, int64_t n, int64_t p, int RP, int64_t m
     return NMFCU_OK;
 }
 
-// Entries of an average segment from which the blocked passes run: a segment
-// costs a warp its line's pointers, factor row and sum (about as much as 16
-// entries), which a few entries do not pay for.
-constexpr int64_t kBlkEntries = 16;
-
 // Segments and line ranges of the blocked passes, for the passes that take
 // them (lines sorted, enough entries a segment).
 template <int RP>
@@ -1088,7 +1098,7 @@ nmfcu_status plan_blocked(nmfcu_context *c, int64_t n, int64_t p, SparseV &sv, c
     using C = BlkCfg<RP>;
     if (n <= 0 || p <= 0 || sv.nnz <= 0 || !sv.sorted) return NMFCU_OK;
     const int rb = (int)cdiv(p, C::ROWS), cb = (int)cdiv(n, C::ROWS);
-    const bool rows = sv.nnz >= kBlkEntries * n * rb, cols = sv.nnz >= kBlkEntries * p * cb;
+    const bool rows = blk_rows_pass(n, p, RP, sv.nnz), cols = blk_cols_pass(n, p, RP, sv.nnz);
     if (!rows && !cols) return NMFCU_OK;
     const int sms = nmfcu_internal::context_sms(c);
     std::vector<void *> b;
@@ -1214,7 +1224,7 @@ nmfcu_status run_csr(nmfcu_context *c, const nmfcu_options *o, int64_t n, int64_
                      cudaStream_t s, int64_t *n_dev, int64_t *n_iter) {
     const int RP = bucket_for(r);
     const bool stat = o->stop == NMFCU_STOP_STATIONARY;
-    NMFCU_TRY(build_csc(c, n, p, sv, s));
+    NMFCU_TRY(build_csc(c, n, p, RP, sv, s));
     Work w;
     NMFCU_TRY(make_work(c, n, p, RP, o->max_iter, w));
     NMFCU_TRY(put_factors(w, n, p, r, RP, W0, H0, in_kind, s));

@@ -9,6 +9,7 @@ import ctypes
 import numpy as np
 import pytest
 import scipy.sparse as sp
+import torch
 
 from conftest import rel_max
 
@@ -130,3 +131,31 @@ def test_repeated_entries():
         _native._ptr(W0), _native._ptr(H0), _native._ptr(W), _native._ptr(H), None, 0,
         ctypes.byref(nd), ctypes.byref(ni)))
     assert rel_max(W, want.W) <= TOL and rel_max(H, want.H) <= TOL
+
+
+def _launches(n, p, r, density):
+    """Kernels of a run of no iterations over a device CSR."""
+    V, W0, H0 = _inputs(n, p, r, density, 3)
+    M = sp.csr_matrix(V)
+    dev = [torch.from_numpy(x).cuda() for x in
+           (M.indptr.astype(np.int64), M.indices.astype(np.int32), M.data, W0, H0)]
+    o = _native.default_options()
+    o.method = _native.parse_method("lee")
+    o.max_iter = 0
+    ctx = _native.Context(0)
+    nd, ni = ctypes.c_int64(0), ctypes.c_int64(0)
+    at = [ctypes.c_void_p(x.data_ptr()) for x in dev]
+    before = ctx.launch_count()
+    _native.check(_native.load().nmfcu_run_csr_device(
+        ctx.handle, ctypes.byref(o), n, p, r, M.nnz, *at, None, ctypes.byref(nd),
+        ctypes.byref(ni), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    count = ctx.launch_count() - before
+    ctx.close()
+    return count
+
+
+def test_order_is_read_where_it_counts():
+    """The rows' order matters to the copy by tiles and to the blocked passes
+    alone: entries too few for both cost no pass over the indices.  The blocked
+    passes' plan is four launches."""
+    assert _launches(700, 1500, 20, 0.2) == _launches(700, 1500, 20, 0.004) + 1 + 4
