@@ -512,6 +512,11 @@ constexpr int kTileRows = 16;      // rows of W a tile (few tiles)
 constexpr int kGramGroup = 16;     // blocks of a group
 enum : int { GRAM_NONE = 0, GRAM_SUMS = 1, GRAM_FULL = 2 };
 
+// Tiles of `len` rows or columns, up to 2^31 - 1 of them.
+__host__ __device__ inline int tile_count(int len, int tile) {
+    return (int)(((unsigned)len + (unsigned)tile - 1u) / (unsigned)tile);
+}
+
 // How an epilogue or Gram launch over `len` rows of W / columns of H runs: a
 // block a tile up to two blocks a multiprocessor, beyond that a warp a tile.
 // At 296 tiles the first still fits the chip at once; the second has every
@@ -812,7 +817,7 @@ __global__ void __launch_bounds__(THREADS)
         const int i0 = blockIdx.x * kTileRows;
         if (warp < kTileRows / 4) steps(i0, min(kTileRows, n - i0), warp, warp + 1);
     } else {
-        const int tiles = (n + 31) / 32;
+        const int tiles = tile_count(n, 32);
         for (int t = blockIdx.x + gridDim.x * warp; t < tiles; t += gridDim.x * GA::WARPS)
             steps(t * 32, min(32, n - t * 32), 0, 8);
     }
@@ -840,7 +845,7 @@ __global__ void __launch_bounds__(THREADS)
     if (FEW) {
         if (warp < kTileCols / 4) steps(blockIdx.x * kTileCols, warp, warp + 1);
     } else {
-        const int tiles = (p + kTileCols - 1) / kTileCols;
+        const int tiles = tile_count(p, kTileCols);
         for (int t = blockIdx.x + gridDim.x * warp; t < tiles; t += gridDim.x * GA::WARPS)
             steps(t * kTileCols, 0, kTileCols / 4);
     }
@@ -1045,11 +1050,11 @@ __global__ void h_transpose(const double *__restrict__ H, TH *__restrict__ Ht, i
 static __global__ void __launch_bounds__(kThreads)
     convert_f64_f32(const double *__restrict__ src, int64_t lds, float *__restrict__ dst,
                     int64_t ldd, int n, int p, bool aligned) {
-    const int j = (blockIdx.x * kThreads + threadIdx.x) * 4;
+    const int64_t j = ((int64_t)blockIdx.x * kThreads + threadIdx.x) * 4;
     if (j >= p) return;
-    for (int i = blockIdx.y; i < n; i += gridDim.y) {
-        const double *a = src + (int64_t)i * lds + j;
-        float *d = dst + (int64_t)i * ldd + j;
+    for (int64_t i = blockIdx.y; i < n; i += gridDim.y) {
+        const double *a = src + i * lds + j;
+        float *d = dst + i * ldd + j;
         if (aligned && j + 3 < p) {
             const double2 x = __ldcs(reinterpret_cast<const double2 *>(a));
             const double2 y = __ldcs(reinterpret_cast<const double2 *>(a) + 1);

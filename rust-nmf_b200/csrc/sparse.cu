@@ -819,7 +819,7 @@ nmfcu_status build_csc(nmfcu_context *c, int64_t n, int64_t p, int RP, SparseV &
     sv.cidx = static_cast<int32_t *>(cb[1]);
     sv.cval = static_cast<double *>(cb[2]);
     const int64_t tile_rows = (n + kCscRows - 1) / kCscRows;
-    const bool tiles = nnz >= kCscTileEntries && p < INT32_MAX && tile_rows <= 65535 &&
+    const bool tiles = nnz >= kCscTileEntries && p <= INT32_MAX - kCscCols && tile_rows <= 65535 &&
                        tile_rows * p <= nnz;
     // (a pass over the indices and a wait for its answer, for those who ask)
     if (nnz > 0 && (tiles || blk_rows_pass(n, p, RP, nnz) || blk_cols_pass(n, p, RP, nnz)))

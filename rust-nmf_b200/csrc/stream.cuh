@@ -1799,7 +1799,7 @@ __global__ void __launch_bounds__(THREADS, EpiSmem<RP, THREADS>::BLOCKS)
             for (int x = threadIdx.x; x < RP * RP; x += THREADS) sG[x] = e.G[x];
         __syncthreads();
         if (stopped) return;
-        const int tiles = (p + TC - 1) / TC;
+        const int tiles = tile_count(p, TC);
         for (int t = blockIdx.x + gridDim.x * warp; t < tiles; t += gridDim.x * WARPS) {
             const int j0 = t * TC, j = j0 + lane;
             const int ct = j0 / tcols, c = j0 - ct * tcols + lane;
@@ -1958,7 +1958,7 @@ __global__ void __launch_bounds__(THREADS, EpiSmem<RP, THREADS>::BLOCKS)
             for (int x = threadIdx.x; x < RP * RP; x += THREADS) sG[x] = e.G[x];
         __syncthreads();
         if (stopped) return;
-        const int tiles = (n + 31) / 32;
+        const int tiles = tile_count(n, 32);
         for (int t = blockIdx.x + gridDim.x * warp; t < tiles; t += gridDim.x * WARPS) {
             const int i0 = t * 32, i = i0 + lane;
             const int rt = i0 / trows, rl = i0 - rt * trows;
