@@ -350,6 +350,12 @@ constexpr int min_blocks_for() {
     return BShapes<T>::min_blocks[SHAPE];
 }
 
+// The same by bucket, for f32 (any shape).
+template <typename T>
+constexpr int kBucketBlocks[kBuckets + 1] = {min_blocks_for<T, 0, 0>(), min_blocks_for<T, 1, 0>(),
+                                             min_blocks_for<T, 2, 0>(),
+                                             min_blocks_for<T, kBuckets, 0>()};
+
 template <typename T, int B, int SHAPE, bool kComponentFast>
 __global__ void __launch_bounds__(kThreads, (min_blocks_for<T, B, SHAPE>()))
     batch_mu(MuArgs<T> a, const int *__restrict__ off, const BItem *__restrict__ items) {
@@ -587,7 +593,15 @@ struct BatchPlan {
 // 5000: H step 1260 us with four columns (17 warps a multiprocessor, buckets
 // in turn), 678 with two; W step 927 (7 warps), 765 with two.  The same
 // columns, one by one, in either.
+//
+// Where all ranks are of one bucket, two columns save no launch, and a step has
+// twice the blocks: only as long as those take no more waves than the blocks of
+// four columns, and up to rank 14 (the kernel of all ranks spills above).  20
+// iterations, both steps with four / with two columns: 60 solves of rank 5 at
+// 3000 x 12000 68.0 / 106.7 ms; at 2000 x 5000 30 of rank 16 39.7 / 50.1, 20 of
+// rank 8 (one wave either way) 29.7 / 19.8.
 constexpr int kNarrowWarps = 32;
+constexpr int kNarrowRank = 14;
 
 // Solves of one rank form a class; a class is cut into groups of NS solves;
 // every (group, tile) pair is one CTA of its bucket's launch.
@@ -615,11 +629,21 @@ BatchPlan plan_batch(int n, int p, int nsolves, const int32_t *ranks, int comp, 
                 bp.group_off.push_back(g + i < members.size() ? offsets[members[g + i]] : -1);
         }
     }
+    const bool one_bucket =
+        !groups.empty() && bucket_of(groups.front().R) == bucket_of(groups.back().R);
     const auto plan_step = [&](int cols, StepPlan &sp) {
         const int wide = (cols + kTile<T> - 1) / kTile<T>;
+        const int thin = (cols + kNarrowTile<T> - 1) / kNarrowTile<T>;
+        const int64_t ng = (int64_t)groups.size();
         sp.narrow = BTraits<T>::NARROW != BTraits<T>::CPT &&
-                    (int64_t)groups.size() * wide * (kThreads / 32) < (int64_t)kNarrowWarps * sms;
-        const int tiles = sp.narrow ? (cols + kNarrowTile<T> - 1) / kNarrowTile<T> : wide;
+                    ng * wide * (kThreads / 32) < (int64_t)kNarrowWarps * sms;
+        if (sp.narrow && one_bucket) {
+            const int64_t places = (int64_t)sms * kBucketBlocks<T>[bucket_of(groups[0].R)];
+            const int64_t thin_places = (int64_t)sms * kBucketBlocks<T>[kBuckets];
+            sp.narrow = groups[0].R <= kNarrowRank && (ng * thin + thin_places - 1) / thin_places <=
+                                                          (ng * wide + places - 1) / places;
+        }
+        const int tiles = sp.narrow ? thin : wide;
         for (int b = 0; b < (sp.narrow ? 1 : kBuckets); b++)
             for (const Group &g : groups) {
                 if (!sp.narrow && bucket_of(g.R) != b) continue;
