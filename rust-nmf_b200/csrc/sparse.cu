@@ -371,8 +371,8 @@ constexpr int blk_rows(int RP) { return kBlkBytes / (RP * 8) / 32 * 32; }  // ro
 template <int RP>
 struct BlkCfg {
     static constexpr int PAIRS = RP / 2;
-    static constexpr int GL = PAIRS >= 4 ? 4 : PAIRS >= 2 ? 2 : 1;  // lanes of an entry
-    static constexpr int UPL = (PAIRS + GL - 1) / GL;               // pairs of a lane
+    static constexpr int GL = 4;                       // lanes of an entry
+    static constexpr int UPL = (PAIRS + GL - 1) / GL;  // pairs of a lane
     // Warps: as many as the registers of GL rows' pairs leave room for.
     static constexpr int WARPS = UPL >= 4 ? 12 : 16;
     static constexpr int ROWS = blk_rows(RP);
@@ -745,15 +745,33 @@ nmfcu_status carve(nmfcu_context *c, int slot, const std::vector<size_t> &sizes,
     return NMFCU_OK;
 }
 
-// Entries of an average segment from which the blocked passes run: a segment
-// costs a warp its line's pointers, factor row and sum (about as much as 16
-// entries), which a few entries do not pay for.
-constexpr int64_t kBlkEntries = 16;
-inline bool blk_rows_pass(int64_t n, int64_t p, int RP, int64_t nnz) {
-    return nnz >= kBlkEntries * n * cdiv(p, blk_rows(RP));
+// Entries of an average segment from which the blocked passes run (0: never): a
+// segment costs a warp its line's pointers, factor row and sum, which a few
+// entries do not pay for, and the gathering passes lose by the length of a
+// factor row: up to rank 6, and at ranks 9 and 10 without the ratio, which leave
+// three eighths of a group's lanes idle, the blocked ones never win.  The lines
+// are where both are about equally fast at 10000 x 50000 and at 8000 x 16000
+// (10000 x 50000 with the ratio, gathering / blocked, us an iteration: rank 20 at
+// 16 entries 724 / 735, at 24 987 / 782; rank 10 at 32 339 / 447, at 96 828 /
+// 812; rank 4 at 128 257 / 337).
+constexpr int64_t blk_entries(int RP, bool ratio) {
+    switch (RP) {
+        case 8: return ratio ? 192 : 80;
+        case 10: return ratio ? 90 : 0;
+        case 12: return ratio ? 56 : 80;
+        case 14: return ratio ? 54 : 72;
+        case 16: return ratio ? 28 : 20;
+        case 20: return ratio ? 18 : 36;
+        case 24: return ratio ? 15 : 18;
+        case 28: return ratio ? 19 : 24;
+        case 32: return 15;
+        default: return 0;
+    }
 }
-inline bool blk_cols_pass(int64_t n, int64_t p, int RP, int64_t nnz) {
-    return nnz >= kBlkEntries * p * cdiv(n, blk_rows(RP));
+// Whether the pass over `lines` against `len` factor rows runs blocked.
+inline bool blk_pass(int64_t lines, int64_t len, int RP, bool ratio, int64_t nnz) {
+    const int64_t least = blk_entries(RP, ratio);
+    return least > 0 && nnz >= least * lines * (int64_t)cdiv(len, blk_rows(RP));
 }
 
 // Whether the rows of the CSR are in (strict) column order.
@@ -807,7 +825,7 @@ nmfcu_status build_csc_tiles(nmfcu_context *c, int64_t n, int64_t p, SparseV &sv
 // stable radix sort of the column indices.  10^8 entries, 20000 x 50000: 5.2
 // ms by the sort, 1.8 by tiles; 1.5 10^6, 5000 x 10000: 0.08 and 0.11.
 constexpr int64_t kCscTileEntries = 1 << 22;
-nmfcu_status build_csc(nmfcu_context *c, int64_t n, int64_t p, int RP, SparseV &sv,
+nmfcu_status build_csc(nmfcu_context *c, int64_t n, int64_t p, int RP, bool ratio, SparseV &sv,
                        cudaStream_t s) {
     const int64_t nnz = sv.nnz;
     std::vector<void *> cb;
@@ -822,7 +840,7 @@ nmfcu_status build_csc(nmfcu_context *c, int64_t n, int64_t p, int RP, SparseV &
     const bool tiles = nnz >= kCscTileEntries && p <= INT32_MAX - kCscCols && tile_rows <= 65535 &&
                        tile_rows * p <= nnz;
     // (a pass over the indices and a wait for its answer, for those who ask)
-    if (nnz > 0 && (tiles || blk_rows_pass(n, p, RP, nnz) || blk_cols_pass(n, p, RP, nnz)))
+    if (nnz > 0 && (tiles || blk_pass(n, p, RP, ratio, nnz) || blk_pass(p, n, RP, ratio, nnz)))
         NMFCU_TRY(check_order(c, n, sv, s));
     if (tiles && sv.strict) return build_csc_tiles(c, n, p, sv, s);
     int bits = 1;
@@ -875,10 +893,12 @@ struct Loop {
     void blocked(const int64_t *ptr, const int32_t *idx, const double *val, const int32_t *seg,
                  const int *bound, int lines, const double *G, const double *F, int frows,
                  double *acc, double *out) {
-        auto *k = sparse_pass_blocked<RP, RATIO, OUT_KM>;
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, BlkCfg<RP>::SMEM);
-        k<<<sms, 32 * BlkCfg<RP>::WARPS, BlkCfg<RP>::SMEM, s>>>(ptr, idx, val, seg, bound, lines, lines, G, F,
-                                                     frows, acc, out, w.st);
+        if constexpr (blk_entries(RP, RATIO) > 0) {
+            auto *k = sparse_pass_blocked<RP, RATIO, OUT_KM>;
+            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, BlkCfg<RP>::SMEM);
+            k<<<sms, 32 * BlkCfg<RP>::WARPS, BlkCfg<RP>::SMEM, s>>>(
+                ptr, idx, val, seg, bound, lines, lines, G, F, frows, acc, out, w.st);
+        }
     }
     // H^T of an H the last epilogue did not write.
     void transpose_h() {
@@ -935,13 +955,13 @@ struct Loop {
                     blocked<false, true>(sv.cptr, sv.cidx, sv.cval, sv.cseg, sv.cbound, p, nullptr,
                                          w.W, n, w.accH, w.numH);
             } else {
-            const unsigned grid = line_grid(p, sms);
-            if (ratio)
-                sparse_pass<RP, true, true><<<grid, kT, 0, s>>>(sv.cptr, sv.cidx, sv.cval, p, p, w.Ht,
-                                                             w.W, w.numH, w.st);
-            else
-                sparse_pass<RP, false, true><<<grid, kT, 0, s>>>(sv.cptr, sv.cidx, sv.cval, p, p,
-                                                              nullptr, w.W, w.numH, w.st);
+                const unsigned grid = line_grid(p, sms);
+                if (ratio)
+                    sparse_pass<RP, true, true><<<grid, kT, 0, s>>>(sv.cptr, sv.cidx, sv.cval, p, p,
+                                                                    w.Ht, w.W, w.numH, w.st);
+                else
+                    sparse_pass<RP, false, true><<<grid, kT, 0, s>>>(
+                        sv.cptr, sv.cidx, sv.cval, p, p, nullptr, w.W, w.numH, w.st);
             }
         }
         nmfcu_internal::TimedScope sc(c, s, NMFCU_KCLASS_OTHER);
@@ -959,13 +979,13 @@ struct Loop {
                     blocked<false, false>(sv.rptr, sv.ridx, sv.rval, sv.rseg, sv.rbound, n,
                                           nullptr, w.Ht, p, w.numW, nullptr);
             } else {
-            const unsigned grid = line_grid(n, sms);
-            if (ratio)
-                sparse_pass<RP, true, false><<<grid, kT, 0, s>>>(sv.rptr, sv.ridx, sv.rval, n, 0, w.W,
-                                                              w.Ht, w.numW, w.st);
-            else
-                sparse_pass<RP, false, false><<<grid, kT, 0, s>>>(sv.rptr, sv.ridx, sv.rval, n, 0,
-                                                               nullptr, w.Ht, w.numW, w.st);
+                const unsigned grid = line_grid(n, sms);
+                if (ratio)
+                    sparse_pass<RP, true, false><<<grid, kT, 0, s>>>(
+                        sv.rptr, sv.ridx, sv.rval, n, 0, w.W, w.Ht, w.numW, w.st);
+                else
+                    sparse_pass<RP, false, false><<<grid, kT, 0, s>>>(
+                        sv.rptr, sv.ridx, sv.rval, n, 0, nullptr, w.Ht, w.numW, w.st);
             }
         }
         nmfcu_internal::TimedScope sc(c, s, NMFCU_KCLASS_OTHER);
@@ -1094,11 +1114,11 @@ nmfcu_status make_work(nmfcu_context *c, int64_t n, int64_t p, int RP, int64_t m
 // Segments and line ranges of the blocked passes, for the passes that take
 // them (lines sorted, enough entries a segment).
 template <int RP>
-nmfcu_status plan_blocked(nmfcu_context *c, int64_t n, int64_t p, SparseV &sv, cudaStream_t s) {
-    using C = BlkCfg<RP>;
+nmfcu_status plan_blocked(nmfcu_context *c, int64_t n, int64_t p, bool ratio, SparseV &sv,
+                          cudaStream_t s) {
     if (n <= 0 || p <= 0 || sv.nnz <= 0 || !sv.sorted) return NMFCU_OK;
-    const int rb = (int)cdiv(p, C::ROWS), cb = (int)cdiv(n, C::ROWS);
-    const bool rows = blk_rows_pass(n, p, RP, sv.nnz), cols = blk_cols_pass(n, p, RP, sv.nnz);
+    const int rb = (int)cdiv(p, blk_rows(RP)), cb = (int)cdiv(n, blk_rows(RP));
+    const bool rows = blk_pass(n, p, RP, ratio, sv.nnz), cols = blk_pass(p, n, RP, ratio, sv.nnz);
     if (!rows && !cols) return NMFCU_OK;
     const int sms = nmfcu_internal::context_sms(c);
     std::vector<void *> b;
@@ -1111,7 +1131,7 @@ nmfcu_status plan_blocked(nmfcu_context *c, int64_t n, int64_t p, SparseV &sv, c
     const auto plan = [&](const int64_t *ptr, const int32_t *idx, int64_t lines, int blocks,
                           int32_t *seg, int *bound) {
         line_segments<<<std::min<unsigned>(cdiv(lines * (blocks + 1), kT), (unsigned)sms * 32), kT,
-                        0, s>>>(ptr, idx, (int)lines, C::ROWS, blocks, seg);
+                        0, s>>>(ptr, idx, (int)lines, blk_rows(RP), blocks, seg);
         line_bounds<<<cdiv(sms + 1, kT), kT, 0, s>>>(ptr, (int)lines, sv.nnz, sms, bound);
     };
     if (rows) {
@@ -1132,7 +1152,7 @@ template <int RP>
 nmfcu_status run_loop_t(nmfcu_context *c, const nmfcu_options *o, int64_t n, int64_t p, int64_t r,
                         SparseV sv, Work w, cudaStream_t s, bool stat, int64_t *n_dev,
                         int64_t *n_iter) {
-    NMFCU_TRY(plan_blocked<RP>(c, n, p, sv, s));
+    NMFCU_TRY(plan_blocked<RP>(c, n, p, o->method == NMFCU_BRUNET, sv, s));
     Loop<RP> L{c, o, (int)n, (int)p, (int)r, sv, w, s, nmfcu_internal::context_sms(c)};
     NMFCU_CUDA_TRY(cudaMemsetAsync(w.st, 0, sizeof(RunState), s));
     L.transpose_h();
@@ -1224,7 +1244,7 @@ nmfcu_status run_csr(nmfcu_context *c, const nmfcu_options *o, int64_t n, int64_
                      cudaStream_t s, int64_t *n_dev, int64_t *n_iter) {
     const int RP = bucket_for(r);
     const bool stat = o->stop == NMFCU_STOP_STATIONARY;
-    NMFCU_TRY(build_csc(c, n, p, RP, sv, s));
+    NMFCU_TRY(build_csc(c, n, p, RP, o->method == NMFCU_BRUNET, sv, s));
     Work w;
     NMFCU_TRY(make_work(c, n, p, RP, o->max_iter, w));
     NMFCU_TRY(put_factors(w, n, p, r, RP, W0, H0, in_kind, s));

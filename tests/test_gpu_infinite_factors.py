@@ -92,8 +92,8 @@ def _stored_brunet(M, W, H):
         return W * num / H.sum(1)[None, :], H
 
 
-# Lines with enough entries for the blocked passes at every number of lanes an
-# entry (rank 1-2 one, 3-6 two, above four), and sparser ones, which gather.
+# Lines that gather (the lower ranks, the sparser ones) and lines with enough
+# entries for the blocked passes.
 @pytest.mark.parametrize("side", ["w", "h"])
 @pytest.mark.parametrize("n,p,r,density", [(150, 170, 2, 0.5), (301, 500, 4, 0.6),
                                            (300, 500, 6, 0.6), (1100, 2200, 20, 0.2),

@@ -133,14 +133,14 @@ def test_repeated_entries():
     assert rel_max(W, want.W) <= TOL and rel_max(H, want.H) <= TOL
 
 
-def _launches(n, p, r, density):
+def _launches(n, p, r, density, method="lee"):
     """Kernels of a run of no iterations over a device CSR."""
     V, W0, H0 = _inputs(n, p, r, density, 3)
     M = sp.csr_matrix(V)
     dev = [torch.from_numpy(x).cuda() for x in
            (M.indptr.astype(np.int64), M.indices.astype(np.int32), M.data, W0, H0)]
     o = _native.default_options()
-    o.method = _native.parse_method("lee")
+    o.method = _native.parse_method(method)
     o.max_iter = 0
     ctx = _native.Context(0)
     nd, ni = ctypes.c_int64(0), ctypes.c_int64(0)
@@ -159,3 +159,16 @@ def test_order_is_read_where_it_counts():
     alone: entries too few for both cost no pass over the indices.  The blocked
     passes' plan is four launches."""
     assert _launches(700, 1500, 20, 0.2) == _launches(700, 1500, 20, 0.004) + 1 + 4
+
+
+# Small factor rows are gathered as fast as they are read from shared memory;
+# a line's entries in a block have to pay for the segment.
+@pytest.mark.parametrize("n,p,r,density,method,blocked", [
+    (300, 500, 2, 0.9, "brunet", False), (300, 500, 4, 0.9, "lee", False),
+    (300, 500, 6, 0.9, "brunet", False), (300, 500, 10, 0.9, "lee", False),
+    (300, 500, 10, 0.9, "brunet", True), (300, 300, 8, 0.53, "brunet", False),
+    (300, 300, 8, 0.53, "lee", True), (700, 1000, 20, 0.03, "lee", False),
+    (700, 1000, 20, 0.03, "brunet", True), (700, 700, 32, 0.02, "lee", False),
+    (700, 700, 32, 0.03, "lee", True)])
+def test_which_passes(n, p, r, density, method, blocked):
+    assert _launches(n, p, r, density, method) == _launches(n, p, r, 0.001, method) + 5 * blocked
