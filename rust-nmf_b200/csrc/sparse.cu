@@ -792,7 +792,7 @@ nmfcu_status check_order(nmfcu_context *c, int64_t n, SparseV &sv, cudaStream_t 
     return NMFCU_OK;
 }
 
-// The CSC copy by tiles (rows in strict order, a table no longer than nnz).
+// The CSC copy by tiles (rows in strict order).
 nmfcu_status build_csc_tiles(nmfcu_context *c, int64_t n, int64_t p, SparseV &sv, cudaStream_t s) {
     const int rows = (int)cdiv(n, kCscRows), cols = (int)cdiv(p, kCscCols);
     const int sms = nmfcu_internal::context_sms(c);
@@ -820,11 +820,15 @@ nmfcu_status build_csc_tiles(nmfcu_context *c, int64_t n, int64_t p, SparseV &sv
     return NMFCU_OK;
 }
 
-// The CSC copy of the CSR: by tiles, or (few entries, rows out of order or with
-// repeats, or so sparse that the tiles' table would outgrow the entries) by a
-// stable radix sort of the column indices.  10^8 entries, 20000 x 50000: 5.2
-// ms by the sort, 1.8 by tiles; 1.5 10^6, 5000 x 10000: 0.08 and 0.11.
-constexpr int64_t kCscTileEntries = 1 << 22;
+// The CSC copy of the CSR: by tiles, or (few entries, fewer than four a column
+// of a tile, rows out of order or with repeats) by a stable radix sort of the
+// column indices.  The tiles cost their table and a pass over the order first.
+// A run of no iterations at rank 2, sort / tiles, us: 20000 x 50000, 94 10^6
+// entries (12 a tile's column) 5161 / 2009, 31 10^6 (4) 1570 / 1459, 24 10^6 (3)
+// 1159 / 1380; 10000 x 20000, 12.6 10^6 545 / 496, 6.3 10^6 376 / 454; 5000 x
+// 4000, 5.1 10^6 332 / 456.
+constexpr int64_t kCscTileEntries = 1 << 23;
+constexpr int64_t kCscColumnEntries = 4;
 nmfcu_status build_csc(nmfcu_context *c, int64_t n, int64_t p, int RP, bool ratio, SparseV &sv,
                        cudaStream_t s) {
     const int64_t nnz = sv.nnz;
@@ -838,7 +842,7 @@ nmfcu_status build_csc(nmfcu_context *c, int64_t n, int64_t p, int RP, bool rati
     sv.cval = static_cast<double *>(cb[2]);
     const int64_t tile_rows = (n + kCscRows - 1) / kCscRows;
     const bool tiles = nnz >= kCscTileEntries && p <= INT32_MAX - kCscCols && tile_rows <= 65535 &&
-                       tile_rows * p <= nnz;
+                       kCscColumnEntries * tile_rows * p <= nnz;
     // (a pass over the indices and a wait for its answer, for those who ask)
     if (nnz > 0 && (tiles || blk_pass(n, p, RP, ratio, nnz) || blk_pass(p, n, RP, ratio, nnz)))
         NMFCU_TRY(check_order(c, n, sv, s));

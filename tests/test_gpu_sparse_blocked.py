@@ -135,8 +135,12 @@ def test_repeated_entries():
 
 def _launches(n, p, r, density, method="lee"):
     """Kernels of a run of no iterations over a device CSR."""
-    V, W0, H0 = _inputs(n, p, r, density, 3)
-    M = sp.csr_matrix(V)
+    return _launches_of(sp.csr_matrix(_inputs(n, p, r, density, 3)[0]), r, method)
+
+
+def _launches_of(M, r, method):
+    n, p = M.shape
+    W0, H0 = np.ones((n, r)), np.ones((r, p))
     dev = [torch.from_numpy(x).cuda() for x in
            (M.indptr.astype(np.int64), M.indices.astype(np.int32), M.data, W0, H0)]
     o = _native.default_options()
@@ -172,3 +176,24 @@ def test_order_is_read_where_it_counts():
     (700, 700, 32, 0.03, "lee", True)])
 def test_which_passes(n, p, r, density, method, blocked):
     assert _launches(n, p, r, density, method) == _launches(n, p, r, 0.001, method) + 5 * blocked
+
+
+# The copy by tiles takes 2^23 entries and four a column of a tile: one row and
+# a few columns past whole tiles; nearly full ones; rows of one tile; one tile
+# of columns.
+@pytest.mark.parametrize("n,p,density", [(2177, 8195, 0.5), (3000, 3300, 0.9), (100, 100001, 0.9),
+                                         (70001, 300, 0.41)])
+def test_csc_by_tiles(oracle, n, p, density):
+    V, W0, H0 = _inputs(n, p, 3, density, n + p)
+    assert np.count_nonzero(V) > 1 << 23
+    _check(oracle, "lee", V, W0, H0, iters=2)
+
+
+@pytest.mark.parametrize("n,p,density,tiles", [
+    (2177, 8195, 0.5, True), (2177, 7000, 0.5, False),  # 8.9 and 7.6 10^6 entries
+    (12800, 30000, 0.035, True), (12800, 30000, 0.028, False)])  # 4.5 and 3.6 a tile's column
+def test_csc_rule(n, p, density, tiles):
+    """By tiles, and after the order, five launches and one; by the sort five."""
+    gen = np.random.default_rng(1)
+    M = sp.random(n, p, density, "csr", rng=gen)
+    assert _launches_of(M, 2, "lee") == _launches(300, 200, 2, 0.5) + tiles
