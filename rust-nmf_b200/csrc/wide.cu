@@ -183,7 +183,7 @@ __global__ void wide_transpose(const double *__restrict__ H, int r, int64_t p,
 __device__ __forceinline__ double quotient(double v, double w) {
     const double q = nmfcu::ratio_div(v, w);
     const double a = fabs(w);
-    if (!(a > 0x1p-500 && a < 0x1p500 && q < 0x1p500)) return q;
+    if (!(a > 0x1p-500 && a < 0x1p500 && fabs(q) < 0x1p500)) return q;
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(w));
     return fma(fma(-q, w, v), r, q);

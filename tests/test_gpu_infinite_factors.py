@@ -74,6 +74,20 @@ def test_wide_objective_is_infinite(oracle, method, side, n, p):
     assert got.n_iter == ref["n_iter"] == 1
 
 
+@pytest.mark.parametrize("r", [20, 34])
+@pytest.mark.parametrize("v", [np.inf, -np.inf])
+def test_infinite_entry(oracle, r, v):
+    """The ratio of an infinite entry of V keeps its sign (py_nmf_run, like the
+    reference's, takes a V of any sign; nmf() itself refuses a negative one)."""
+    V, W, H = _inputs(50, 70, r)
+    V[3, 5] = v
+    ref = oracle.nmf_method("brunet", V, W, H, 1)
+    got = _native.py_nmf_run("brunet", V, W, H, 1)
+    assert np.all(ref["H"][:, 5] == v)
+    np.testing.assert_array_equal(np.isfinite(got["H"]), np.isfinite(ref["H"]))
+    np.testing.assert_array_equal(got["H"][:, 5], ref["H"][:, 5])
+
+
 def _stored_brunet(M, W, H):
     """One brunet iteration over the stored entries of M alone."""
     c = M.tocoo()
