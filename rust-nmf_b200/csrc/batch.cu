@@ -592,7 +592,11 @@ struct BatchPlan {
 // to cover the latency of their chains.  72 solves of ranks 2..10 at 2000 x
 // 5000: H step 1260 us with four columns (17 warps a multiprocessor, buckets
 // in turn), 678 with two; W step 927 (7 warps), 765 with two.  The same
-// columns, one by one, in either.
+// columns, one by one, in either.  20 iterations over several buckets, steps
+// below the line with four / with two: 30 solves of ranks 8, 9 at 2000 x 5000
+// 47.0 / 23.2 ms, 60 at 3000 x 12000 (W step alone) 146 / 122; 60 of ranks 7..9
+// there 138 / 124; 110 of ranks 2..12 at 2000 x 5000 67.7 / 50.0; 96 of ranks
+// 2..9 at 3000 x 6000 80.3 / 67.0; 72 of ranks 2..10 at 500 x 20000 118 / 66.
 //
 // Where all ranks are of one bucket, two columns save no launch, and a step has
 // twice the blocks: only as long as those take no more waves than the blocks of

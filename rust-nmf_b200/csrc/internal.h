@@ -41,9 +41,10 @@ nmfcu_status context_prepare(nmfcu_context *c, int64_t n, int64_t p);
 nmfcu_status default_context(int device, nmfcu_context **out);
 
 // A scratch buffer of the context that grows to at least `bytes` (slot
-// 0..25, one owner per slot; the contents survive between calls).  Owners:
-// 0..12, 16, 17 batch.cu; 13..15 linkage.cu; 18..23 sparse.cu (serve.cu
-// uses the slots of its own contexts).
+// 0..26; the contents survive between calls).  Owners: 0..12, 16, 17
+// batch.cu; 13..15 linkage.cu; 18..23, 26 sparse.cu; 24, 25 wide.cu.  A batch
+// with ranks above 16 borrows 20..22 within its call; serve.cu uses 12..16 of
+// its own contexts, which run single solves alone (24, 25 above rank 32).
 constexpr int kContextSlots = 27;
 nmfcu_status context_buffer(nmfcu_context *c, int slot, size_t bytes, void **out);
 

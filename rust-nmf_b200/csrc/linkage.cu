@@ -137,9 +137,10 @@ __global__ void __launch_bounds__(kR) finish_sums(const double *__restrict__ par
 // kCl blocks by st.async, which counts it in on the receiver's mbarrier; when
 // all kCl * kTc / 32 are there, every warp reduces them and knows the step's
 // outcome.  All blocks decide from the same candidates, so they take the same
-// steps.  Eight blocks a cluster: sixteen such clusters are resident at once,
-// clusters of 16 are only eight.  Blocks of 128 / 512 threads took 28.0 /
-// 26.5 ms.
+// steps.  Eight blocks a cluster: at one block a multiprocessor sixteen such
+// clusters are resident at once, of clusters of 16 only eight; sizes and chain
+// of up to p = 13000 or so leave shared memory for a second block.  Blocks of
+// 128 / 512 threads took 28.0 / 26.5 ms.
 //
 // Two candidate buffers in turn: a warp sends step t + 2 after it has all of
 // step t + 1, which holds every warp's candidate, sent after that warp had

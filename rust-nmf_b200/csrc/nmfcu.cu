@@ -507,9 +507,9 @@ struct PassSet {
     CUtensorMap tmVrH, tmVrW, tmXwU, tmXhU;  // tcr: V (f32), W / H unit layouts
 };
 
-// The split-bf16 form runs lee / offset / hals / dnmf on the tensor cores;
-// brunet's and nsNMF's ratio is formed per element, so they keep the FP32
-// CUDA-core passes.
+// The split-bf16 form runs lee / offset / hals / dnmf on split planes of V
+// (tc_pass); brunet's and nsNMF's ratio is formed per element from the f32 V,
+// between two tensor-core products (tcr_pass).
 bool tc_form(const nmfcu_options *o) {
     return o->precision == NMFCU_PREC_BF16X3 && o->method != NMFCU_BRUNET &&
            o->method != NMFCU_NSNMF;

@@ -364,8 +364,11 @@ __global__ void __launch_bounds__(kT)
 // through its GL entries, each lane with every GL-th pair of the entry's row;
 // W H comes together so that each lane ends with its own entry's, and divides
 // it once.  A fixed butterfly adds the groups at the segment's end.  Bound:
-// shared-memory reads of factor rows at random bank phases, about 2.6 cycles
-// an entry, and at the ratio the latency of its FP64 chain.
+// latency.  The shared-memory reads of factor rows, at random bank phases about
+// 2.6 cycles an entry, are half of a pass (0.93 of 1.83 ms with the ratio, of
+// 1.54 without, at 10^8 entries and rank 20); a warp has one chunk of 32
+// entries in flight, whose shuffles (and FP64 chain at the ratio) follow one
+// another, and a segment ends in a butterfly and a sum in global memory.
 constexpr int kBlkBytes = 200 * 1024;  // of F in shared memory
 constexpr int blk_rows(int RP) { return kBlkBytes / (RP * 8) / 32 * 32; }  // rows of F a block
 template <int RP>

@@ -1447,8 +1447,11 @@ __global__ void __launch_bounds__(DWRCfg<RP>::kWarps * 32, 1)
 // c the middle of m's 1/128 (its seven leading fraction bits), r = m / c - 1,
 //   ln x = k ln 2 + ln c + (r - r^2/2 + ... - r^6/6),  |r| <= 1/256,
 // the term left out below 3e-18.  Above sqrt 2 the table holds ln c - ln 2 and
-// k goes up by one, so that nothing cancels near x = 1.  The error is that of
-// the final additions.  Ten FP64 operations and one 16-byte load.
+// k goes up by one, so that k ln 2 cancels nothing near x = 1.  There ln c and
+// the polynomial cancel, both up to 1/256: the error is absolute, about 1e-18
+// however small ln x is, and relative to ln x grows as x nears 1 (2e-12 at
+// 1 + 1e-6).  KL adds v ln q to v's own size, whose rounding, 1e-16 v, is far
+// above 1e-18 v.  Ten FP64 operations and one 16-byte load.
 constexpr int kLogEntries = 128;
 __device__ __forceinline__ void log_table_init(double2 *t) {
     const int j = threadIdx.x;
