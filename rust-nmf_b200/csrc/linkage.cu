@@ -205,6 +205,10 @@ __device__ __forceinline__ void bar_expect(unsigned bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                  : "memory");
 }
+// A warp's lanes leave a wait together, with one answer: what follows votes and
+// reduces over all of them.  (A lane that has seen the phase end goes on seeing
+// it: the next one of that barrier needs this warp.  The vote in the loop costs
+// 0.3 % of a step; behind it, 7 %.)
 __device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity) {
     for (unsigned i = 0; i < kWaitLimit; i++) {
         unsigned ok;
@@ -215,7 +219,7 @@ __device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity) {
             : "=r"(ok)
             : "r"(bar), "r"(parity)
             : "memory");
-        if (ok) return true;
+        if (__all_sync(0xffffffffu, ok)) return true;
     }
     return false;
 }

@@ -86,3 +86,11 @@ def test_tree_leaves_by_one_barrier():
         assert "late = true;" in given_up and "break;" in given_up
     assert "bar_wait(" in after[after.index("cl.sync("):]
     assert "atomicExch(gave_up" in after
+
+
+def test_tree_warp_gives_up_as_one():
+    """The lanes of a warp leave a wait with one answer: one that went on alone
+    would reduce over lanes that have left the steps."""
+    body = _kernel(CSRC / "linkage.cu", "bool bar_wait")
+    assert re.findall(r"(if \([^\n]*\) )?return (\w+);", body) == [
+        ("if (__all_sync(0xffffffffu, ok)) ", "true"), ("", "false")]
