@@ -1655,15 +1655,16 @@ def run_sparse(args, world, rank, local):
     avg = tot / max(nl, 1)
     csr_bytes = nnz * 12
     achieved = csr_bytes / (avg / 1000.0) / 1e9
-    roof = {"bound": "hbm", "kernel": ("sparse_pass<H> (CSC columns)" if dom == "hstep"
-                                        else "sparse_pass<W> (CSR rows)"),
+    roof = {"bound": "hbm", "kernel": ("sparse H pass (CSC columns)" if dom == "hstep"
+                                        else "sparse W pass (CSR rows)"),
             "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "peak_kind": peak_kind, "launches": nl, "avg_launch_ms": avg, "traffic": None,
             "algorithmic_bytes_per_launch": csr_bytes,
             "gathered_factor_bytes_per_launch": nnz * (r + r % 2) * 8,
             "class_ms": {c: classes[c][1] for c in classes},
             "note": ("algorithmic bytes = the CSR a pass streams (12 B a stored entry); each "
-                     "stored entry also gathers an f64 factor row from L2")}
+                     "stored entry also reads an f64 factor row, from shared memory "
+                     "where lines have enough entries a block of rows, else from L2")}
     # End to end: host CSR arrays through nmfcu_run_csr.
     e2e = None
     if not args.no_e2e:
